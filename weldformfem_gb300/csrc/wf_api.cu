@@ -2074,6 +2074,7 @@ WF_API wf_status wf_init(wf_domain *d) {
     t.sy0 = m.sy0;
     t.H = m.H;
     t.cs0 = std::sqrt(t.K / m.rho);
+    t.i3GH = 1.0 / (3.0 * t.G + t.H);
     t.model = m.model;
     t.hol_K = m.hol_K;
     t.hol_m = m.hol_m;
@@ -2217,6 +2218,7 @@ WF_API wf_status wf_init(wf_domain *d) {
     }
     CUDA_TRY(dalloc(d, &S.sr, 6 * ne));
     CUDA_TRY(dalloc(d, &S.rr, 6 * ne));
+    CUDA_TRY(dalloc_raw(d, &S.adj, (size_t)ne * (d->npe == 8 ? 9 : 10)));
     CUDA_TRY(dalloc(d, &S.fe, (size_t)ne * d->npe * 3));
     if (P.hg_on) CUDA_TRY(dalloc(d, &S.fhg, (size_t)ne * d->npe * 3));
   }
@@ -2842,7 +2844,7 @@ WF_API wf_status wf_get_halo_forces(wf_domain *d, int64_t e0, int64_t e1, double
   if (s) return s;
   if (!out || e0 < 0 || e1 > d->ne || e0 > e1) return WF_ERR_ARG;
   CUDA_TRY(cudaSetDevice(d->device));
-  const size_t k = (size_t)(e1 - e0) * d->npe * 3, at = (size_t)e0 * d->npe * 3;
+  const size_t k = (size_t)(e1 - e0) * d->npe * 3;
   if (d->precision == WF_MIXED) {
     // FP32 forces (element force minus hourglass force) [npe * 3][ne]: the
     // element range of every (corner, component) row, widened exactly; the
@@ -2858,14 +2860,24 @@ WF_API wf_status wf_get_halo_forces(wf_domain *d, int64_t e0, int64_t e1, double
     d->d2h_bytes += (int64_t)(sizeof(float) * rows * m);
     return WF_OK;
   }
-  CUDA_TRY(cudaMemcpyAsync(out, d->S.fe + at, sizeof(double) * k, cudaMemcpyDeviceToHost,
-                           d->stream));
-  if (d->S.fhg)
-    CUDA_TRY(cudaMemcpyAsync(out + k, d->S.fhg + at, sizeof(double) * k, cudaMemcpyDeviceToHost,
-                             d->stream));
-  else
-    std::fill(out + k, out + 2 * k, 0.0);
-  CUDA_TRY(cudaStreamSynchronize(d->stream));
+  // FP64 forces [npe * 3][ne] on the device: the element range of every row,
+  // put into the caller's per-element order
+  const size_t m = (size_t)(e1 - e0), rows = (size_t)d->npe * 3;
+  std::vector<double> h(k);
+  for (int part = 0; part < 2; part++) {
+    const double *src = part ? d->S.fhg : d->S.fe;
+    double *dst = out + part * k;
+    if (!src) {
+      std::fill(dst, dst + k, 0.0);
+      continue;
+    }
+    if (k == 0) continue;
+    CUDA_TRY(cudaMemcpy2DAsync(h.data(), sizeof(double) * m, src + e0, sizeof(double) * d->ne,
+                               sizeof(double) * m, rows, cudaMemcpyDeviceToHost, d->stream));
+    CUDA_TRY(cudaStreamSynchronize(d->stream));
+    for (size_t r = 0; r < rows; r++)
+      for (size_t e = 0; e < m; e++) dst[e * rows + r] = h[r * m + e];
+  }
   d->d2h_bytes += (int64_t)(sizeof(double) * 2 * k);
   return WF_OK;
 }
@@ -2875,7 +2887,7 @@ WF_API wf_status wf_set_halo_forces(wf_domain *d, int64_t e0, int64_t e1, const 
   if (s) return s;
   if (!in || e0 < 0 || e1 > d->ne || e0 > e1) return WF_ERR_ARG;
   CUDA_TRY(cudaSetDevice(d->device));
-  const size_t k = (size_t)(e1 - e0) * d->npe * 3, at = (size_t)e0 * d->npe * 3;
+  const size_t k = (size_t)(e1 - e0) * d->npe * 3;
   if (d->precision == WF_MIXED) {
     const size_t m = (size_t)(e1 - e0), rows = (size_t)d->npe * 3;
     std::vector<float> h(rows * m);
@@ -2886,12 +2898,18 @@ WF_API wf_status wf_set_halo_forces(wf_domain *d, int64_t e0, int64_t e1, const 
     d->h2d_bytes += (int64_t)(sizeof(float) * rows * m);
     return WF_OK;
   }
-  CUDA_TRY(cudaMemcpyAsync(d->S.fe + at, in, sizeof(double) * k, cudaMemcpyHostToDevice,
-                           d->stream));
-  if (d->S.fhg)
-    CUDA_TRY(cudaMemcpyAsync(d->S.fhg + at, in + k, sizeof(double) * k, cudaMemcpyHostToDevice,
-                             d->stream));
-  CUDA_TRY(cudaStreamSynchronize(d->stream));
+  const size_t m = (size_t)(e1 - e0), rows = (size_t)d->npe * 3;
+  std::vector<double> h(k);
+  for (int part = 0; part < 2; part++) {
+    double *dst = part ? d->S.fhg : d->S.fe;
+    const double *src = in + part * k;
+    if (!dst || k == 0) continue;
+    for (size_t r = 0; r < rows; r++)
+      for (size_t e = 0; e < m; e++) h[r * m + e] = src[e * rows + r];
+    CUDA_TRY(cudaMemcpy2DAsync(dst + e0, sizeof(double) * d->ne, h.data(), sizeof(double) * m,
+                               sizeof(double) * m, rows, cudaMemcpyHostToDevice, d->stream));
+    CUDA_TRY(cudaStreamSynchronize(d->stream));
+  }
   d->h2d_bytes += (int64_t)(sizeof(double) * 2 * k);
   return WF_OK;
 }

@@ -1,9 +1,11 @@
-// FP64 step kernels: the reference's arithmetic, operation for operation.
+// FP64 step kernels.
 //
-// This translation unit is compiled with --fmad=false so that every
-// expression rounds exactly as the reference CPU code does with FMA
-// contraction off (the reference build passes --fmad=false to nvcc,
-// src/common/CMakeLists.txt:16). One step is four launches:
+// This translation unit is compiled with --fmad=false: tetrahedra run the
+// reference's arithmetic operation for operation and round exactly as the
+// reference CPU code does with FMA contraction off (the reference build passes
+// --fmad=false to nvcc, src/common/CMakeLists.txt:16). Hexahedra compute the
+// same quantities in fewer operations (k_fp64_hexes), with explicit FMA, and
+// stay within 1e-9 of the reference. One step is four launches:
 //   geometry  (element): J, detJ, volume             -> vol
 //   nodal     (node)   : volume sums, lumped mass, J ratio
 //   elements  (element): dN, D/W, pressure, Jaumann + radial return,
@@ -21,16 +23,6 @@ namespace {
 constexpr int kElemThreads = 128;
 constexpr int kNodeThreads = 256;
 
-// Flanagan-Belytschko hourglass base vectors of the 8-node hexahedron
-// (test_1el_3D.cpp:166-169), as compile-time signs.
-__device__ __forceinline__ constexpr int hg_sig(int j, int a) {
-  constexpr signed char t[4][8] = {{1, 1, -1, -1, -1, -1, 1, 1},
-                                   {1, -1, -1, 1, -1, 1, 1, -1},
-                                   {1, -1, 1, -1, 1, -1, 1, -1},
-                                   {-1, 1, -1, 1, 1, -1, 1, -1}};
-  return t[j][a];
-}
-
 __device__ __forceinline__ double det3(const double J[3][3]) {
   // Matrix::calcDet (include/common/Matrix.h:593-620)
   return J[0][0] * J[1][1] * J[2][2] - J[0][0] * J[1][2] * J[2][1] -
@@ -38,35 +30,18 @@ __device__ __forceinline__ double det3(const double J[3][3]) {
          J[0][2] * J[1][0] * J[2][1] - J[0][2] * J[1][1] * J[2][0];
 }
 
-// Jacobian of the element from its node coordinates
-// (Domain_d.C:1822-1830 hexahedron, :1866-1870 tetrahedron).
-template <int NPE>
-__device__ __forceinline__ void jacobian(const double (&x2)[NPE][3], double J[3][3]) {
-  if constexpr (NPE == 8) {
+// Jacobian of a tetrahedron from its node coordinates (Domain_d.C:1866-1870).
+__device__ __forceinline__ void jacobian(const double (&x2)[4][3], double J[3][3]) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      J[0][k] = 0.125 * (-x2[0][k] + x2[1][k] + x2[2][k] - x2[3][k] - x2[4][k] + x2[5][k] +
-                         x2[6][k] - x2[7][k]);
-      J[1][k] = 0.125 * (-x2[0][k] - x2[1][k] + x2[2][k] + x2[3][k] - x2[4][k] - x2[5][k] +
-                         x2[6][k] + x2[7][k]);
-      J[2][k] = 0.125 * (-x2[0][k] - x2[1][k] - x2[2][k] - x2[3][k] + x2[4][k] + x2[5][k] +
-                         x2[6][k] + x2[7][k]);
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      J[0][k] = x2[1][k] - x2[0][k];
-      J[1][k] = x2[2][k] - x2[0][k];
-      J[2][k] = x2[3][k] - x2[0][k];
-    }
+  for (int k = 0; k < 3; k++) {
+    J[0][k] = x2[1][k] - x2[0][k];
+    J[1][k] = x2[2][k] - x2[0][k];
+    J[2][k] = x2[3][k] - x2[0][k];
   }
 }
 
-// dN/dx * detJ from the adjugate of J (AdjMat, Matrix.h:694-727;
-// Domain_d.C:1842-1851 hexahedron, :1881-1887 tetrahedron).
-template <int NPE>
-__device__ __forceinline__ void shape_derivs(const double J[3][3], double dH[3][NPE]) {
-  double inv[3][3];
+// Adjugate of J (AdjMat, Matrix.h:694-727), inv[k][m].
+__device__ __forceinline__ void adjugate(const double J[3][3], double inv[3][3]) {
   inv[0][0] = (J[1][1] * J[2][2] - J[1][2] * J[2][1]);
   inv[1][0] = -(J[1][0] * J[2][2] - J[1][2] * J[2][0]);
   inv[2][0] = (J[1][0] * J[2][1] - J[1][1] * J[2][0]);
@@ -76,30 +51,99 @@ __device__ __forceinline__ void shape_derivs(const double J[3][3], double dH[3][
   inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]);
   inv[1][2] = -(J[0][0] * J[1][2] - J[0][2] * J[1][0]);
   inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]);
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const double a0 = inv[k][0], a1 = inv[k][1], a2 = inv[k][2];
-    if constexpr (NPE == 8) {
-      dH[k][0] = 0.125 * (-a0 - a1 - a2);
-      dH[k][1] = 0.125 * (a0 - a1 - a2);
-      dH[k][2] = 0.125 * (a0 + a1 - a2);
-      dH[k][3] = 0.125 * (-a0 + a1 - a2);
-      dH[k][4] = 0.125 * (-a0 - a1 + a2);
-      dH[k][5] = 0.125 * (a0 - a1 + a2);
-      dH[k][6] = 0.125 * (a0 + a1 + a2);
-      dH[k][7] = 0.125 * (-a0 + a1 + a2);
-    } else {
-      dH[k][0] = -a0 - a1 - a2;
-      dH[k][1] = a0;
-      dH[k][2] = a1;
-      dH[k][3] = a2;
-    }
-  }
 }
 
 template <int NPE>
 __device__ __forceinline__ double weight() {
   return NPE == 8 ? 8.0 : 1.0 / 6.0;
+}
+
+// Walsh sums of the eight nodal values of a hexahedron, weighted by the corner
+// signs {-, xi, eta, zeta, eta zeta, xi zeta, xi eta, xi eta zeta} (index 0 is
+// not formed): 1..3 are the derivative directions of the trilinear shape
+// functions at the centre (8 J for coordinates), 4..7 the hourglass base
+// vectors. 23 additions; unused outputs cost nothing.
+__device__ __forceinline__ void walsh8d(const double (&v)[8], double (&o)[8]) {
+  const double a0 = v[1] + v[0], b0 = v[1] - v[0];
+  const double a1 = v[2] + v[3], b1 = v[2] - v[3];
+  const double a2 = v[5] + v[4], b2 = v[5] - v[4];
+  const double a3 = v[6] + v[7], b3 = v[6] - v[7];
+  const double c0 = a1 + a0, d0 = a1 - a0, e0 = b1 + b0, f0 = b1 - b0;
+  const double c1 = a3 + a2, d1 = a3 - a2, e1 = b3 + b2, f1 = b3 - b2;
+  o[1] = e1 + e0;
+  o[2] = d1 + d0;
+  o[3] = c1 - c0;
+  o[4] = d1 - d0;
+  o[5] = e1 - e0;
+  o[6] = f1 + f0;
+  o[7] = f1 - f0;
+}
+
+// Nodal values of o1 xi + o2 eta + o3 zeta: opposite corners differ in sign,
+// so 6 additions give all eight.
+__device__ __forceinline__ void synth_linear(double o1, double o2, double o3, double (&v)[8]) {
+  const double p = o3 + o2, m = o3 - o2;
+  v[6] = p + o1;
+  v[7] = p - o1;
+  v[5] = m + o1;
+  v[4] = m - o1;
+  v[0] = -v[6];
+  v[1] = -v[7];
+  v[2] = -v[4];
+  v[3] = -v[5];
+}
+
+// Nodal values of o4 eta zeta + o5 xi zeta + o6 xi eta + o7 xi eta zeta: the
+// part even under the inversion of the corner (o4, o5, o6) and the odd one.
+__device__ __forceinline__ void synth_hourglass(double o4, double o5, double o6, double o7,
+                                                double (&v)[8]) {
+  const double s = o4 + o5, d = o4 - o5;
+  const double e06 = s + o6, e17 = d - o6;   // corners 0, 6 and 1, 7
+  const double e24 = o6 - s, e35 = -d - o6;  // corners 2, 4 and 3, 5
+  v[6] = e06 + o7;
+  v[0] = e06 - o7;
+  v[1] = e17 + o7;
+  v[7] = e17 - o7;
+  v[4] = e24 + o7;
+  v[2] = e24 - o7;
+  v[3] = e35 + o7;
+  v[5] = e35 - o7;
+}
+
+// adj(X) and det(X) of X = 8 J (rows xi, eta, zeta): A[k][m] = cofactor [m][k].
+__device__ __forceinline__ double adjugate8(const double X[3][3], double A[3][3]) {
+  A[0][0] = fma(X[1][1], X[2][2], -(X[1][2] * X[2][1]));
+  A[1][0] = fma(X[1][2], X[2][0], -(X[1][0] * X[2][2]));
+  A[2][0] = fma(X[1][0], X[2][1], -(X[1][1] * X[2][0]));
+  A[0][1] = fma(X[0][2], X[2][1], -(X[0][1] * X[2][2]));
+  A[1][1] = fma(X[0][0], X[2][2], -(X[0][2] * X[2][0]));
+  A[2][1] = fma(X[0][1], X[2][0], -(X[0][0] * X[2][1]));
+  A[0][2] = fma(X[0][1], X[1][2], -(X[0][2] * X[1][1]));
+  A[1][2] = fma(X[0][2], X[1][0], -(X[0][0] * X[1][2]));
+  A[2][2] = fma(X[0][0], X[1][1], -(X[0][1] * X[1][0]));
+  return fma(X[0][2], A[2][0], fma(X[0][1], A[1][0], X[0][0] * A[0][0]));
+}
+
+// v^0.6666666 (the hourglass coefficient's exponent, test_1el_3D.cpp:185) for
+// v > 0: the inverse cube root from its FP32 value by one third-order
+// correction, y (1 + e / 3 + 2 e^2 / 9) with e = 1 - v y^3 of about 1e-7, then
+// v^(2/3) = v y, and v^(0.6666666 - 2/3) = exp(z) with |z| < 5e-6 as
+// 1 + z + z^2 / 2; in z the logarithm of the mantissa is FP32 (3e-8 absolute,
+// 2e-15 in the result). About 15 FP64 instructions; values out of the FP32
+// range take pow.
+__device__ __forceinline__ double pow_two_thirds(double v) {
+  if (!(v > 1e-30 && v < 1e30)) return pow(v, 0.6666666);
+  const double y0 = (double)rcbrtf((float)v);
+  const double e = fma(-(v * y0), y0 * y0, 1.0);
+  const double y = fma(y0 * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), y0);
+  // v = m 2^q with m in [1, 2): ln m from its FP32 rounding and the rest
+  const int hi = __double2hiint(v);
+  const double md = __hiloint2double(0x3ff00000 | (hi & 0xfffff), __double2loint(v));
+  const float m = (float)md;
+  const double ln = fma((double)((hi >> 20) - 1023), 0.693147180559945309,
+                        (double)logf(m) + (double)((float)(md - (double)m) / m));
+  const double z = (0.6666666 - 2.0 / 3.0) * ln;
+  return (v * y) * fma(z, fma(z, 0.5, 1.0), 1.0);
 }
 
 template <int NPE>
@@ -115,8 +159,32 @@ __device__ __forceinline__ void gather_x(const StepParams &P, const double *x, i
   }
 }
 
+// X[m][k] = sum of the corners' coordinates k weighted by the sign of
+// direction m (8 J), from differences along the edges (21 additions a
+// component; the velocity sums take 17). The pressure is the bulk modulus
+// times a change of volume of 1e-3 and less, and differences of sums of
+// absolute coordinates left the step's largest rounding error (against 64-bit
+// sums of coordinates relative to a corner, 1.05 M hexahedra, 20 steps:
+// displacement 2e-13 from edge differences, 8e-13 without, as the reference's
+// alternating sums).
+__device__ __forceinline__ void corner_sums(const double (&x2)[8][3], double (&X)[3][3]) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    double v[8];
+#pragma unroll
+    for (int a = 0; a < 8; a++) v[a] = x2[a][k];
+    X[0][k] = ((v[1] - v[0]) + (v[2] - v[3])) + ((v[5] - v[4]) + (v[6] - v[7]));
+    X[1][k] = ((v[2] - v[1]) + (v[3] - v[0])) + ((v[6] - v[5]) + (v[7] - v[4]));
+    X[2][k] = ((v[4] - v[0]) + (v[6] - v[2])) + ((v[5] - v[1]) + (v[7] - v[3]));
+  }
+}
+
 // ---------------------------------------------------------------------------
-// geometry: vol = 0.0 + detJ * w * 1.0 (Mechanical.C:264-293)
+// geometry: vol = 0.0 + detJ * w * 1.0 (Mechanical.C:264-293), and the adjugate
+// of the Jacobian (of 8 J for hexahedra) for the element kernel of the step:
+// 72 bytes written and read once cost less than the 70 FP64 instructions that
+// form it again (1.05 M hexahedra: element kernel 805 -> 662 us, this one
+// 150 -> 152 us).
 template <int NPE>
 __global__ void __launch_bounds__(kElemThreads) k_fp64_geometry(StepParams P, Fp64State S,
                                                            int store_detj) {
@@ -125,13 +193,26 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_geometry(StepParams P, Fp
   double x2[NPE][3];
   int32_t nid[NPE];
   gather_x<NPE>(P, S.x, e, x2, nid);
-  double J[3][3];
-  jacobian<NPE>(x2, J);
-  double detJ = det3(J);
-  double v = 0.0;
-  v += detJ * weight<NPE>() * 1.0;
+  double J[3][3], A[3][3], detJ, v;
+  if constexpr (NPE == 8) {
+    corner_sums(x2, J);
+    detJ = adjugate8(J, A) * (1.0 / 512.0);
+    v = detJ * 8.0;
+  } else {
+    jacobian(x2, J);
+    adjugate(J, A);
+    detJ = det3(J);
+    v = 0.0;
+    v += detJ * weight<NPE>() * 1.0;
+  }
   S.vol[e] = v;
   if (store_detj) S.detJ[e] = detJ;
+  if (!S.adj) return;   // the preamble of a mixed domain, or its detJ readback
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+#pragma unroll
+    for (int m = 0; m < 3; m++) S.adj[(3 * k + m) * P.ne + e] = A[k][m];
+  if constexpr (NPE == 4) S.adj[9 * P.ne + e] = detJ;
 }
 
 // ---------------------------------------------------------------------------
@@ -175,11 +256,31 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodal(StepParams P, Fp64S
   voln /= NPE;
   S.voln[n] = voln;
   if (P.mass_mode == 0 || init_mode) {
-    double mass = 0.0;
-    const double f = 1.0;
-    for (int32_t k = 0; k < c; k++) {
-      int32_t e = elem(k);
-      mass += f * __ldg(&S.rho[e]) * voln / c;
+    // rho_e voln / c per element, added in list order; the quotient is formed
+    // anew only where the density changes (an FP64 division is about ten
+    // FP64 instructions, and most meshes have one density; the densities are
+    // compared as bit patterns, off the FP64 pipe). Hexahedra around a node
+    // of one density share voln rho outright.
+    double mass = 0.0, share = 0.0;
+    long long rho = 0;
+    bool same = true;
+    if (NPE == 8)
+      for (int32_t k = 0; k < c; k++) {
+        const long long r = __double_as_longlong(__ldg(&S.rho[elem(k)]));
+        same &= k == 0 || r == rho;
+        rho = r;
+      }
+    if (NPE == 8 && same && c > 0) {
+      mass = __longlong_as_double(rho) * voln;
+    } else {
+      for (int32_t k = 0; k < c; k++) {
+        const double r = __ldg(&S.rho[elem(k)]);
+        if (k == 0 || __double_as_longlong(r) != rho) {
+          rho = __double_as_longlong(r);
+          share = r * voln / c;
+        }
+        mass += share;
+      }
     }
     S.mass[n] = mass;
   }
@@ -217,42 +318,220 @@ __device__ __forceinline__ double hollomon_et(double strain, const MatDev &m) {
   return 0.;
 }
 
+// Element pressure: calcElemPressure (Mechanical.C:691-819) from the mean of
+// the nodes' J ratios, or calcElemPressureANP (:1220-1250). div_v is the
+// divergence of the predicted velocity times detJ (stabilisation only).
+template <int NPE>
+__device__ __forceinline__ double element_pressure(const StepParams &P, const Fp64State &S,
+                                                   const MatDev &m, int64_t e,
+                                                   const int32_t (&nid)[NPE], double vol,
+                                                   double div_v) {
+  double p;
+  if (P.press_alg == 1) {
+    p = S.p[e];
+    for (int a = 0; a < NPE; a++) p += P.k0 * (1.0 - __ldg(&S.jr[nid[a]]));
+    p *= 0.25 * NPE;
+    return p;
+  }
+  const double K = m.K;
+  double J_avg = 0.0;
+#pragma unroll
+  for (int a = 0; a < NPE; a++) J_avg += __ldg(&S.jr[nid[a]]);
+  J_avg /= NPE;
+  if (!P.stab_on) {
+    // All stabilisation parameters zero: J_bar = 0 * J_local + 1 * J_avg
+    // = J_avg and the 0 * log(J_bar) term adds only a signed zero.
+    double J_bar = J_avg;
+    if (J_bar < 0.0) J_bar = 0.2;
+    return -K * (J_bar - 1.0);
+  }
+  const double J_local = vol / __ldg(&S.vol0[e]);
+  const double *st = P.stab;
+  const double rho_e = S.rho[e];
+  const double h = pow(vol, 1.0 / 3.0);
+  bool is_contact = false;
+  if (P.contact) {
+    for (int a = 0; a < NPE; a++) {
+      double c0 = S.cf[nid[a]], c1 = S.cf[P.np + nid[a]], c2 = S.cf[2 * P.np + nid[a]];
+      if (c0 * c0 + c1 * c1 + c2 * c2 > 0) { is_contact = true; break; }
+    }
+  }
+  double alpha = is_contact ? st[1] : st[0];
+  double J_bar = alpha * J_local + (1 - alpha) * J_avg;
+  if (J_bar < st[9]) J_bar = 0.2;
+  double p_physical = -K * (st[6] * log(J_bar) + (1.0 - st[6]) * (J_bar - 1.0));
+  double c = sqrt(K / rho_e);
+  double tau = h / (2.0 * c);
+  double p_pspg = 0.0;
+  double p_hg = (is_contact ? st[3] : st[2]) * K * fabs(J_local - J_avg);
+  double p_q = 0.0;
+  if (div_v < 0.0) {
+    double t1 = st[7] * tau * div_v * K, t2 = st[8] * K;
+    p_pspg = (t2 < t1) ? t2 : t1;
+    double q1 = st[4] * rho_e * h * c * (-div_v);
+    double delta_J = 1.0 - J_local;
+    double q2 = st[5] * K * delta_J;
+    p_q = is_contact ? 0.5 * (q1 + q2) : ((q1 < q2) ? q2 : q1);
+  }
+  p = p_physical + p_pspg + p_hg + p_q;
+  return p;
+}
+
+// Yield stress and tangent modulus of the element's law. eff, jTh and temp
+// carry what the rate-dependent laws share between the two.
+struct LawState {
+  double eff, jTh, temp;
+};
+template <int NPE, bool TH>
+__device__ __forceinline__ double yield_stress(const StepParams &P, const Fp64State &S,
+                                               const MatDev &m, int32_t mat_id,
+                                               const int32_t (&nid)[NPE], double pls, double s00,
+                                               double s11, double s22, double s01, double s12,
+                                               double s02, LawState &w) {
+  w.eff = 0.0;
+  w.jTh = m.jc_Th;
+  w.temp = m.g_T;  // GMT element temperature
+  if (m.model == WF_MAT_JOHNSON_COOK || m.model == WF_MAT_GMT) {
+    // effective strain rate (Mechanical.C:1701-1705)
+    w.eff = sqrt(0.5 * ((s00 - s11) * (s00 - s11) + (s11 - s22) * (s11 - s22) +
+                        (s22 - s00) * (s22 - s00)) +
+                 3.0 * (s01 * s01 + s12 * s12 + s02 * s02));
+    if constexpr (TH) {
+      // element temperature: mean of its node temperatures (the reference
+      // reads T[e], a node array indexed by element)
+      double ts = 0.0;
+#pragma unroll
+      for (int a = 0; a < NPE; a++) ts += S.T[nid[a]];
+      w.temp = ts / NPE;
+      if (m.model == WF_MAT_JOHNSON_COOK)
+        w.jTh = 1.0 - pow((w.temp - m.jc_Tt) / (m.jc_Tm - m.jc_Tt), m.jc_m);
+    }
+    if (m.model == WF_MAT_JOHNSON_COOK) {
+      // CalcJohnsonCookYieldStress (Material.cuh:377-392)
+      const double sr = (w.eff == 0.0) ? 1.e-5 : w.eff;
+      return (m.sy0 + m.jc_B * pow(pls, m.jc_n)) * (1.0 + m.jc_C * log(sr / m.jc_eps0)) * w.jTh;
+    }
+    return gmt_sy(pls, w.eff, w.temp, P.mats + mat_id);
+  }
+  if (m.model == WF_MAT_HOLLOMON) return hollomon_sy(pls, m);
+  return m.sy0 + m.H * pls;
+}
+__device__ __forceinline__ double tangent_modulus(const StepParams &P, const MatDev &m,
+                                                  int32_t mat_id, double pls,
+                                                  const LawState &w) {
+  if (m.model == WF_MAT_JOHNSON_COOK) {
+    // CalcJohnsonCookTangentModulus (Material.cuh:397-410) at min(edot, m_max_edot)
+    const double er = (P.max_edot < w.eff) ? P.max_edot : w.eff;
+    return (pls > 0.) ? m.jc_n * m.jc_B * pow(pls, m.jc_n - 1.) *
+                            (1.0 + m.jc_C * log(er / m.jc_eps0)) * w.jTh
+                      : m.E * 0.1;
+  }
+  if (m.model == WF_MAT_GMT)
+    return gmt_et(pls, (P.max_edot < w.eff) ? P.max_edot : w.eff, w.temp, P.mats + mat_id);
+  return (m.model == WF_MAT_HOLLOMON) ? hollomon_et(pls, m) : m.H;
+}
+
+// Plastic heat (Mechanical.C:1783-1810): m_plheatfraction sigma : (d eps_p / dt),
+// the plastic strain increment along the returned stress, shear terms doubled.
+__device__ __forceinline__ double plastic_heat(const StepParams &P, const double (&SG)[6],
+                                               double dep, double sy, double dt) {
+  const double f = dep / sy;
+  const double idt = 1. / dt;
+  const double ixx = f * (SG[0] - 0.5 * (SG[1] + SG[2]));
+  const double iyy = f * (SG[1] - 0.5 * (SG[0] + SG[2]));
+  const double izz = f * (SG[2] - 0.5 * (SG[0] + SG[1]));
+  const double ixy = 1.5 * f * (SG[3]), ixz = 1.5 * f * (SG[5]), iyz = 1.5 * f * (SG[4]);
+  return P.plheat_frac * (SG[0] * (ixx * idt) + 2.0 * SG[3] * (ixy * idt) +
+                          2.0 * SG[5] * (ixz * idt) + SG[1] * (iyy * idt) +
+                          2.0 * SG[4] * (iyz * idt) + SG[2] * (izz * idt));
+}
+
+// Artificial viscosity (calcArtificialViscosity, Mechanical.C:1948-1977; serial
+// in the reference, per element here).
+__device__ __forceinline__ void add_viscosity(const StepParams &P, const Fp64State &S,
+                                              const MatDev &m, int64_t e, double eps_v, double vol,
+                                              double (&SG)[6]) {
+  const double c = sqrt(m.K / S.rho[e]);
+  if (fabs(eps_v) > 1e-12) {
+    const double l = pow(vol, 1.0 / 3.0);
+    double q = P.av[0] * c * fabs(eps_v) * l + P.av[1] * pow(eps_v * l, 2);
+    q = (1e9 < q) ? 1e9 : q;
+    const double qs = (eps_v > 0) ? -q : q;
+    SG[0] += qs;
+    SG[1] += qs;
+    SG[2] += qs;
+  }
+}
+
+// calcThermalExpansion (Thermal.C:163-178): exp_T times the mean of the
+// previous step's element-node temperature rates, read at the element's node
+// ids as the reference indexes them.
+template <int NPE>
+__device__ __forceinline__ double thermal_strain_rate(const StepParams &P, const Fp64State &S,
+                                                      const MatDev &m, const int32_t (&nid)[NPE],
+                                                      long long step) {
+  const double *prev = S.dte + ((step + 1) & 1) * P.ne * NPE;
+  double g = 0.0;
+#pragma unroll
+  for (int a = 0; a < NPE; a++) g += 1.0 / NPE * prev[nid[a]];
+  return m.exp_T * g;
+}
+
+// Element-node temperature rates (Domain_d::ThermalCalcs, Thermal.C:27-106):
+// -(K T)_a / m_a plus the plastic heat 0.9 q vol split evenly over the nodes
+// over m_a cp; KT = (K T)_a. One division per node.
+template <int NPE>
+__device__ __forceinline__ void store_temperature_rates(const StepParams &P, const Fp64State &S,
+                                                        const MatDev &m, int64_t e,
+                                                        const int32_t (&nid)[NPE], long long step,
+                                                        const double (&KT)[NPE], double q_pl,
+                                                        double vol) {
+  double *cur = S.dte + (step & 1) * P.ne * NPE + e * NPE;
+  const double heat = 0.9 * q_pl * vol / NPE / m.cp_T;
+#pragma unroll
+  for (int a = 0; a < NPE; a++) cur[a] = (heat - KT[a]) / S.mass[nid[a]];
+}
+
 // ---------------------------------------------------------------------------
 // elements: calcElemJAndDerivatives, calcElemStrainRates (Mechanical.C:41-126),
 // calcElemPressure (:691-819) or calcElemPressureANP (:1220-1250),
 // CalcStressStrain (:1664-1839), calcArtificialViscosity (:1948-1977),
 // calcElemForces (:375-481) and the 3-D viscous hourglass forces.
 // TH: thermal coupling (a separate instantiation keeps the common case's
-// register allocation).
-template <int NPE, bool TH>
-__global__ void __launch_bounds__(kElemThreads) k_fp64_elements(StepParams P, Fp64State S) {
+// register allocation). Element forces go to fe[(a * 3 + k) * ne + e] (and the
+// hourglass forces to fhg likewise): neighbouring threads store neighbouring
+// values, and the node gather reads them so.
+//
+// Tetrahedra: the reference's operations in its order (FMA contraction off),
+// bit for bit the reference's forces.
+template <bool TH>
+__global__ void __launch_bounds__(kElemThreads) k_fp64_tets(StepParams P, Fp64State S) {
+  constexpr int NPE = 4;
   int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= P.ne) return;
   const int64_t ne = P.ne;
   int32_t nid[NPE];
+#pragma unroll
+  for (int a = 0; a < NPE; a++) nid[a] = __ldg(&P.elnod[a * ne + e]);
+  // dN/dx detJ (Domain_d.C:1881-1887) from the step's adjugate
   double dH[3][NPE];
-  double detJ;
-  {
-    double x2[NPE][3];
-    gather_x<NPE>(P, S.x, e, x2, nid);
-    double J[3][3];
-    jacobian<NPE>(x2, J);
-    shape_derivs<NPE>(J, dH);
-    detJ = det3(J);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const double a0 = __ldg(&S.adj[(3 * k) * ne + e]), a1 = __ldg(&S.adj[(3 * k + 1) * ne + e]),
+                 a2 = __ldg(&S.adj[(3 * k + 2) * ne + e]);
+    dH[k][0] = -a0 - a1 - a2;
+    dH[k][1] = a0;
+    dH[k][2] = a1;
+    dH[k][3] = a2;
   }
-  double vol = 0.0;
-  vol += detJ * weight<NPE>() * 1.0;
+  const double detJ = __ldg(&S.adj[9 * ne + e]);
+  const double vol = __ldg(&S.vol[e]);
   const int32_t mat_id = P.emat ? __ldg(&P.emat[e]) : 0;
   const MatDev m = P.mats[mat_id];
 
   // strain rate and spin (str_rate / rot_rate, upper triangle)
   double s00 = 0.0, s11 = 0.0, s22 = 0.0, s01 = 0.0, s12 = 0.0, s02 = 0.0;
   double w01 = 0.0, w12 = 0.0, w02 = 0.0;
-  double hm[3][4];
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) hm[k][j] = 0.0;
   double div_v = 0.0;
   const double f = 1.0 / detJ;
 #pragma unroll
@@ -271,87 +550,17 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_elements(StepParams P, Fp
     w12 = w12 + f * (d2 * v1 - d1 * v2);
     w02 = w02 + f * (d2 * v0 - d0 * v2);
     if (P.stab_on) div_v += d0 * v0 + d1 * v1 + d2 * v2;
-    if constexpr (NPE == 8) {
-      if (P.hg_on) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          // v * Gamma with Gamma = +-1 is exact: add or subtract
-          if (hg_sig(j, a) > 0) {
-            hm[0][j] += v0; hm[1][j] += v1; hm[2][j] += v2;
-          } else {
-            hm[0][j] -= v0; hm[1][j] -= v1; hm[2][j] -= v2;
-          }
-        }
-      }
-    }
   }
   s01 = s01 * 0.5; s02 = s02 * 0.5; s12 = s12 * 0.5;
   w01 = w01 * 0.5; w02 = w02 * 0.5; w12 = w12 * 0.5;
   const long long step = TH ? P.st->step : 0;
   if constexpr (TH) {
-    // calcThermalExpansion (Thermal.C:163-178): the previous step's
-    // element-node temperature rates read at the element's node ids, as the
-    // reference indexes them
-    const double *prev = S.dte + ((step + 1) & 1) * ne * NPE;
-    double g = 0.0;
-#pragma unroll
-    for (int a = 0; a < NPE; a++) g += 1.0 / NPE * prev[nid[a]];
-    const double c = m.exp_T * g;
+    const double c = thermal_strain_rate(P, S, m, nid, step);
     s00 = s00 - c;
     s11 = s11 - c;
     s22 = s22 - c;
   }
-
-  // pressure
-  double p;
-  if (P.press_alg == 1) {
-    p = S.p[e];
-    for (int a = 0; a < NPE; a++) p += P.k0 * (1.0 - __ldg(&S.jr[nid[a]]));
-    p *= 0.25 * NPE;
-  } else {
-    const double K = m.K;
-    const double J_local = vol / __ldg(&S.vol0[e]);
-    double J_avg = 0.0;
-#pragma unroll
-    for (int a = 0; a < NPE; a++) J_avg += __ldg(&S.jr[nid[a]]);
-    J_avg /= NPE;
-    if (!P.stab_on) {
-      // All stabilisation parameters zero: J_bar = 0 * J_local + 1 * J_avg
-      // = J_avg and the 0 * log(J_bar) term adds only a signed zero.
-      double J_bar = J_avg;
-      if (J_bar < 0.0) J_bar = 0.2;
-      p = -K * (J_bar - 1.0);
-    } else {
-      const double *st = P.stab;
-      const double rho_e = S.rho[e];
-      const double h = pow(vol, 1.0 / 3.0);
-      bool is_contact = false;
-      if (P.contact) {
-        for (int a = 0; a < NPE; a++) {
-          double c0 = S.cf[nid[a]], c1 = S.cf[P.np + nid[a]], c2 = S.cf[2 * P.np + nid[a]];
-          if (c0 * c0 + c1 * c1 + c2 * c2 > 0) { is_contact = true; break; }
-        }
-      }
-      double alpha = is_contact ? st[1] : st[0];
-      double J_bar = alpha * J_local + (1 - alpha) * J_avg;
-      if (J_bar < st[9]) J_bar = 0.2;
-      double p_physical = -K * (st[6] * log(J_bar) + (1.0 - st[6]) * (J_bar - 1.0));
-      double c = sqrt(K / rho_e);
-      double tau = h / (2.0 * c);
-      double p_pspg = 0.0;
-      double p_hg = (is_contact ? st[3] : st[2]) * K * fabs(J_local - J_avg);
-      double p_q = 0.0;
-      if (div_v < 0.0) {
-        double t1 = st[7] * tau * div_v * K, t2 = st[8] * K;
-        p_pspg = (t2 < t1) ? t2 : t1;
-        double q1 = st[4] * rho_e * h * c * (-div_v);
-        double delta_J = 1.0 - J_local;
-        double q2 = st[5] * K * delta_J;
-        p_q = is_contact ? 0.5 * (q1 + q2) : ((q1 < q2) ? q2 : q1);
-      }
-      p = p_physical + p_pspg + p_hg + p_q;
-    }
-  }
+  const double p = element_pressure(P, S, m, e, nid, vol, div_v);
 
   // Jaumann rate + radial return (CalcStressStrain). The tensor3 algebra of
   // the reference (Tensor3.C) written out on the six stored components: the
@@ -392,50 +601,12 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_elements(StepParams P, Fp
                            2.0 * t4 * t4 + d2s * d2s);
   const double sig_trial = sqrt(3.0 * J2);
   double pls = S.pls[e];
-  double sy;
-  double eff = 0.0;
-  double jTh = m.jc_Th;
-  double temp = m.g_T;  // GMT element temperature
-  if (m.model == WF_MAT_JOHNSON_COOK || m.model == WF_MAT_GMT) {
-    // effective strain rate (Mechanical.C:1701-1705)
-    eff = sqrt(0.5 * ((s00 - s11) * (s00 - s11) + (s11 - s22) * (s11 - s22) +
-                      (s22 - s00) * (s22 - s00)) +
-               3.0 * (s01 * s01 + s12 * s12 + s02 * s02));
-    if constexpr (TH) {
-      // element temperature: mean of its node temperatures (the reference
-      // reads T[e], a node array indexed by element)
-      double ts = 0.0;
-#pragma unroll
-      for (int a = 0; a < NPE; a++) ts += S.T[nid[a]];
-      temp = ts / NPE;
-      if (m.model == WF_MAT_JOHNSON_COOK) jTh = 1.0 - pow((temp - m.jc_Tt) / (m.jc_Tm - m.jc_Tt), m.jc_m);
-    }
-    if (m.model == WF_MAT_JOHNSON_COOK) {
-      // CalcJohnsonCookYieldStress (Material.cuh:377-392)
-      const double sr = (eff == 0.0) ? 1.e-5 : eff;
-      sy = (m.sy0 + m.jc_B * pow(pls, m.jc_n)) * (1.0 + m.jc_C * log(sr / m.jc_eps0)) * jTh;
-    } else {
-      sy = gmt_sy(pls, eff, temp, P.mats + mat_id);
-    }
-  } else if (m.model == WF_MAT_HOLLOMON) {
-    sy = hollomon_sy(pls, m);
-  } else {
-    sy = m.sy0 + m.H * pls;
-  }
+  LawState law;
+  const double sy = yield_stress<NPE, TH>(P, S, m, mat_id, nid, pls, s00, s11, s22, s01, s12, s02,
+                                          law);
   double dep = 0.0;
   if (sy < sig_trial) {
-    double H;
-    if (m.model == WF_MAT_JOHNSON_COOK) {
-      // CalcJohnsonCookTangentModulus (Material.cuh:397-410) at min(edot, m_max_edot)
-      const double er = (P.max_edot < eff) ? P.max_edot : eff;
-      H = (pls > 0.) ? m.jc_n * m.jc_B * pow(pls, m.jc_n - 1.) *
-                           (1.0 + m.jc_C * log(er / m.jc_eps0)) * jTh
-                     : m.E * 0.1;
-    } else if (m.model == WF_MAT_GMT) {
-      H = gmt_et(pls, (P.max_edot < eff) ? P.max_edot : eff, temp, P.mats + mat_id);
-    } else {
-      H = (m.model == WF_MAT_HOLLOMON) ? hollomon_et(pls, m) : m.H;
-    }
+    const double H = tangent_modulus(P, m, mat_id, pls, law);
     const double G = m.G;
     const double dgamma = (sig_trial - sy) / (3.0 * G + H);
     const double factor = 1.0 - (3.0 * G * dgamma) / sig_trial;
@@ -445,20 +616,8 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_elements(StepParams P, Fp
     dep = dgamma;
   }
   double SG[6] = {t0 - p, t1 - p, t2 - p, t3, t4, t5};
-  // plastic heat (Mechanical.C:1783-1810): m_plheatfraction sigma : (d eps_p / dt), the
-  // plastic strain increment along the returned stress, shear terms doubled
   double q_pl = 0.0;
-  if (TH && dep > 0.0) {
-    const double f = dep / sy;
-    const double idt = 1. / dt;
-    const double ixx = f * (SG[0] - 0.5 * (SG[1] + SG[2]));
-    const double iyy = f * (SG[1] - 0.5 * (SG[0] + SG[2]));
-    const double izz = f * (SG[2] - 0.5 * (SG[0] + SG[1]));
-    const double ixy = 1.5 * f * (SG[3]), ixz = 1.5 * f * (SG[5]), iyz = 1.5 * f * (SG[4]);
-    q_pl = P.plheat_frac * (SG[0] * (ixx * idt) + 2.0 * SG[3] * (ixy * idt) +
-                            2.0 * SG[5] * (ixz * idt) + SG[1] * (iyy * idt) +
-                            2.0 * SG[4] * (iyz * idt) + SG[2] * (izz * idt));
-  }
+  if (TH && dep > 0.0) q_pl = plastic_heat(P, SG, dep, sy, dt);
   // total strain: eps = eps + dt * D
   {
     double e0 = S.eps[e], e1 = S.eps[ne + e], e2 = S.eps[2 * ne + e];
@@ -470,20 +629,7 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_elements(StepParams P, Fp
     S.eps[4 * ne + e] = e4 + s12 * dt;
     S.eps[5 * ne + e] = e5 + s02 * dt;
   }
-  // artificial viscosity (serial in the reference; per element here)
-  if (P.av_on) {
-    const double c = sqrt(m.K / S.rho[e]);
-    const double eps_v = (s00 + s11 + s22);
-    if (fabs(eps_v) > 1e-12) {
-      const double l = pow(vol, 1.0 / 3.0);
-      double q = P.av[0] * c * fabs(eps_v) * l + P.av[1] * pow(eps_v * l, 2);
-      q = (1e9 < q) ? 1e9 : q;
-      const double qs = (eps_v > 0) ? -q : q;
-      SG[0] += qs;
-      SG[1] += qs;
-      SG[2] += qs;
-    }
-  }
+  if (P.av_on) add_viscosity(P, S, m, e, s00 + s11 + s22, vol, SG);
   S.p[e] = p;
   S.pls[e] = pls;
   S.sy[e] = sy;
@@ -494,11 +640,10 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_elements(StepParams P, Fp
   S.tau[3 * ne + e] = t3; S.tau[4 * ne + e] = t4; S.tau[5 * ne + e] = t5;
   S.sr[e] = s00; S.sr[ne + e] = s11; S.sr[2 * ne + e] = s22;
   S.sr[3 * ne + e] = s01; S.sr[4 * ne + e] = s12; S.sr[5 * ne + e] = s02;
-  S.rr[e] = 0.0; S.rr[ne + e] = 0.0; S.rr[2 * ne + e] = 0.0;
+  // the spin's diagonal stays zero (rows 0..2 are never written)
   S.rr[3 * ne + e] = w01; S.rr[4 * ne + e] = w12; S.rr[5 * ne + e] = w02;
 
   // element forces f = w * B^T sigma (3-D branch of calcElemForces)
-  double *fe = &S.fe[e * NPE * 3];
   const double w = weight<NPE>();
 #pragma unroll
   for (int a = 0; a < NPE; a++) {
@@ -508,69 +653,214 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_elements(StepParams P, Fp
     f0 += d1 * sg3 + d2 * sg5;
     f1 += d0 * sg3 + d2 * sg4;
     f2 += d1 * sg4 + d0 * sg5;
-    fe[3 * a] = f0 * w;
-    fe[3 * a + 1] = f1 * w;
-    fe[3 * a + 2] = f2 * w;
-  }
-  if constexpr (NPE == 8) {
-    if (P.hg_on) {
-      const double ch = P.hg_coef * pow(vol, 0.6666666) * S.rho[e] * 0.25 * m.cs0;
-      double chm[3][4];
-#pragma unroll
-      for (int k = 0; k < 3; k++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) chm[k][j] = ch * hm[k][j];
-      double *fh = &S.fhg[e * 24];
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          // acc -= ch * h * Gamma with Gamma = +-1: exact sign flips
-          double acc = 0.0;
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            if (hg_sig(j, i) > 0) acc -= chm[k][j];
-            else acc += chm[k][j];
-          }
-          fh[3 * i + k] = acc;
-        }
-      }
-    }
+    S.fe[(3 * a) * ne + e] = f0 * w;
+    S.fe[(3 * a + 1) * ne + e] = f1 * w;
+    S.fe[(3 * a + 2) * ne + e] = f2 * w;
   }
   if constexpr (TH) {
-    // Domain_d::ThermalCalcs (Thermal.C:27-106), element part: conduction
-    // K_ij = (sum_d dN_i detJ dN_j detJ) k_T / detJ w against the node
-    // temperatures, and the plastic heat 0.9 q vol split evenly over the nodes
-    double Te[NPE];
+    // conduction (K T)_i = (sum_d dN_i detJ sum_k dN_k detJ T_k) k_T / detJ w:
+    // through the temperature gradient, 24 products instead of a 4 x 4 matrix
+    double gT[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int a = 0; a < NPE; a++) Te[a] = S.T[nid[a]];
-    const double heat = 0.9 * q_pl;
-    const double elem_pow = heat * vol;
-    const double pow_per_node = elem_pow / NPE;
-    double *cur = S.dte + (step & 1) * ne * NPE + e * NPE;
-    const double wt = weight<NPE>();
-    for (int i = 0; i < NPE; i++) {
-      double dT = 0.0;
-      for (int k = 0; k < NPE; k++) {
-        double kk = 0.0;
+    for (int a = 0; a < NPE; a++) {
+      const double Ta = S.T[nid[a]];
 #pragma unroll
-        for (int dd = 0; dd < 3; dd++) kk += dH[dd][i] * dH[dd][k];
-        dT += kk * m.k_T / detJ * wt * Te[k];
-      }
-      const double mi = S.mass[nid[i]];
-      const double m_inv = 1.0 / mi;
-      double r = -m_inv * dT;
-      r += pow_per_node / (mi * m.cp_T);
-      cur[i] = r;
+      for (int dd = 0; dd < 3; dd++) gT[dd] = fma(dH[dd][a], Ta, gT[dd]);
     }
+    const double kf = m.k_T * f * w;
+    double KT[NPE];
+#pragma unroll
+    for (int a = 0; a < NPE; a++)
+      KT[a] = kf * fma(dH[0][a], gT[0], fma(dH[1][a], gT[1], dH[2][a] * gT[2]));
+    store_temperature_rates(P, S, m, e, nid, step, KT, q_pl, vol);
+  }
+}
+
+// Hexahedra: the same quantities through the Walsh sums of the nodal values,
+// with FMA. GB300 issues 2 FP64 instructions per SM and clock, so the FP64
+// instruction count is the time: written out as the reference's loops over
+// nodes and derivatives the element took 957 FP64 instructions. With
+// X = 8 J the three derivative sums of the coordinates, A = adj(X) and
+// D = det(X): volume D / 64, velocity gradient A G / D with G the velocity's
+// derivative sums, nodal forces the synthesis of A^T sigma / 64, and the
+// powers of two are exact. The reference's yy and zz Jaumann terms are
+// (a - b) + (b - a), exactly zero.
+template <bool TH>
+__global__ void __launch_bounds__(kElemThreads) k_fp64_hexes(StepParams P, Fp64State S) {
+  constexpr int NPE = 8;
+  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= P.ne) return;
+  const int64_t ne = P.ne;
+  int32_t nid[NPE];
+#pragma unroll
+  for (int a = 0; a < NPE; a++) nid[a] = __ldg(&P.elnod[a * ne + e]);
+  double A[3][3];
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+#pragma unroll
+    for (int mm = 0; mm < 3; mm++) A[k][mm] = __ldg(&S.adj[(3 * k + mm) * ne + e]);
+  const double vol = __ldg(&S.vol[e]), D = vol * 64.0;
+  const int32_t mat_id = P.emat ? __ldg(&P.emat[e]) : 0;
+  const MatDev &m = P.mats[mat_id];
+  double G[3][3];
+  {
+    // velocity sums; the hourglass forces depend on nothing else
+    double ch = 0.0;
+    if (P.hg_on) ch = P.hg_coef * pow_two_thirds(vol) * S.rho[e] * 0.25 * m.cs0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      double v[8], o[8];
+#pragma unroll
+      for (int a = 0; a < 8; a++) v[a] = __ldg(&S.vp[k * P.np + nid[a]]);
+      walsh8d(v, o);
+      G[0][k] = o[1];
+      G[1][k] = o[2];
+      G[2][k] = o[3];
+      if (P.hg_on) {
+        double h[8];
+        synth_hourglass(-(ch * o[4]), -(ch * o[5]), -(ch * o[6]), -(ch * o[7]), h);
+#pragma unroll
+        for (int a = 0; a < 8; a++) S.fhg[(3 * a + k) * ne + e] = h[a];
+      }
+    }
+  }
+  // strain rate and spin from L[i][k] = d v_k / d x_i = (A G)[i][k] / D
+  const double f = 1.0 / D, fh = 0.5 * f;
+  auto AG = [&](int i, int k) {
+    return fma(A[i][2], G[2][k], fma(A[i][1], G[1][k], A[i][0] * G[0][k]));
+  };
+  double s00 = AG(0, 0) * f, s11 = AG(1, 1) * f, s22 = AG(2, 2) * f;
+  const double l10 = AG(1, 0), l01 = AG(0, 1), l21 = AG(2, 1), l12 = AG(1, 2), l20 = AG(2, 0),
+               l02 = AG(0, 2);
+  const double s01 = fh * (l10 + l01), w01 = fh * (l10 - l01);
+  const double s12 = fh * (l21 + l12), w12 = fh * (l21 - l12);
+  const double s02 = fh * (l20 + l02), w02 = fh * (l20 - l02);
+  // the divergence times detJ = D / 512
+  const double div_v = P.stab_on ? (s00 + s11 + s22) * (D * (1.0 / 512.0)) : 0.0;
+  const long long step = TH ? P.st->step : 0;
+  if constexpr (TH) {
+    const double c = thermal_strain_rate(P, S, m, nid, step);
+    s00 = s00 - c;
+    s11 = s11 - c;
+    s22 = s22 - c;
+  }
+  const double p = element_pressure(P, S, m, e, nid, vol, div_v);
+
+  // Jaumann rate with the reference's product, then the radial return; the
+  // pressure drops out of the trial stress's deviator
+  const double dt = P.espec ? P.spec_dt[P.espec[e]] : P.dt;
+  double t0 = S.tau[e], t1 = S.tau[ne + e], t2 = S.tau[2 * ne + e];
+  double t3 = S.tau[3 * ne + e], t4 = S.tau[4 * ne + e], t5 = S.tau[5 * ne + e];
+  {
+    const double g2 = 2.0 * m.G * dt;
+    const double c = (1.0 / 3.0) * (s00 + s11 + s22);
+    const double q0 = 2.0 * fma(t3, w01, t5 * w02);
+    const double q3 = fma(w01, t0 + t1, fma(w02, t4, -(t5 * w12)));
+    const double q4 = fma(w12, t1 + t2, fma(w02, t3, -(t5 * w01)));
+    const double q5 = fma(w02, t0 + t2, fma(w12, t3, w01 * t4));
+    t0 = fma(q0, dt, fma(s00 - c, g2, t0));
+    t1 = fma(s11 - c, g2, t1);
+    t2 = fma(s22 - c, g2, t2);
+    t3 = fma(q3, dt, fma(s01, g2, t3));
+    t4 = fma(q4, dt, fma(s12, g2, t4));
+    t5 = fma(q5, dt, fma(s02, g2, t5));
+  }
+  const double tm = (1.0 / 3.0) * (t0 + t1 + t2);
+  const double d0s = t0 - tm, d1s = t1 - tm, d2s = t2 - tm;
+  // sig_trial^2 = 3 J2
+  const double q2 = 1.5 * fma(d0s, d0s, fma(d1s, d1s, fma(d2s, d2s,
+                          2.0 * fma(t3, t3, fma(t4, t4, t5 * t5)))));
+  double pls = S.pls[e];
+  LawState law;
+  const double sy = yield_stress<NPE, TH>(P, S, m, mat_id, nid, pls, s00, s11, s22, s01, s12, s02,
+                                          law);
+  double dep = 0.0;
+  // sy < sig_trial, without the square root for elements well inside the
+  // yield surface (a NaN enters and fails the exact test, as sy < NaN does)
+  if (sy < 0.0 || !(q2 < sy * sy)) {
+    // (0 and infinity keep the square root's value)
+    const double rs = rsqrt(q2), sig_trial = (q2 > 0.0 && !isinf(q2)) ? q2 * rs : q2;
+    if (sy < sig_trial) {
+      const double G3 = 3.0 * m.G;
+      const double dgamma = (m.model == WF_MAT_BILINEAR)
+                                ? (sig_trial - sy) * m.i3GH
+                                : (sig_trial - sy) / (G3 + tangent_modulus(P, m, mat_id, pls, law));
+      const double factor = 1.0 - (G3 * dgamma) * rs;
+      t0 = d0s * factor; t1 = d1s * factor; t2 = d2s * factor;
+      t3 = t3 * factor; t4 = t4 * factor; t5 = t5 * factor;
+      pls += dgamma;
+      dep = dgamma;
+    }
+  }
+  double SG[6] = {t0 - p, t1 - p, t2 - p, t3, t4, t5};
+  double q_pl = 0.0;
+  if (TH && dep > 0.0) q_pl = plastic_heat(P, SG, dep, sy, dt);
+  S.eps[e] = fma(s00, dt, S.eps[e]);
+  S.eps[ne + e] = fma(s11, dt, S.eps[ne + e]);
+  S.eps[2 * ne + e] = fma(s22, dt, S.eps[2 * ne + e]);
+  S.eps[3 * ne + e] = fma(s01, dt, S.eps[3 * ne + e]);
+  S.eps[4 * ne + e] = fma(s12, dt, S.eps[4 * ne + e]);
+  S.eps[5 * ne + e] = fma(s02, dt, S.eps[5 * ne + e]);
+  if (P.av_on) add_viscosity(P, S, m, e, s00 + s11 + s22, vol, SG);
+  S.p[e] = p;
+  S.pls[e] = pls;
+  S.sy[e] = sy;
+#pragma unroll
+  for (int c = 0; c < 6; c++) S.sig[c * ne + e] = SG[c];
+  S.tau[e] = t0; S.tau[ne + e] = t1; S.tau[2 * ne + e] = t2;
+  S.tau[3 * ne + e] = t3; S.tau[4 * ne + e] = t4; S.tau[5 * ne + e] = t5;
+  S.sr[e] = s00; S.sr[ne + e] = s11; S.sr[2 * ne + e] = s22;
+  S.sr[3 * ne + e] = s01; S.sr[4 * ne + e] = s12; S.sr[5 * ne + e] = s02;
+  // the spin's diagonal stays zero (rows 0..2 are never written)
+  S.rr[3 * ne + e] = w01; S.rr[4 * ne + e] = w12; S.rr[5 * ne + e] = w02;
+
+  // forces: synthesis of A^T sigma / 64
+  const double c64 = 1.0 / 64.0;
+  const double sxx = SG[0] * c64, syy = SG[1] * c64, szz = SG[2] * c64, sxy = SG[3] * c64,
+               syz = SG[4] * c64, sxz = SG[5] * c64;
+  const double Sk[3][3] = {{sxx, sxy, sxz}, {sxy, syy, syz}, {sxz, syz, szz}};
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    double o[3], v[8];
+#pragma unroll
+    for (int mm = 0; mm < 3; mm++)
+      o[mm] = fma(A[2][mm], Sk[2][k], fma(A[1][mm], Sk[1][k], A[0][mm] * Sk[0][k]));
+    synth_linear(o[0], o[1], o[2], v);
+#pragma unroll
+    for (int a = 0; a < 8; a++) S.fe[(3 * a + k) * ne + e] = v[a];
+  }
+  if constexpr (TH) {
+    // conduction in the same form: detJ grad T = A (sums of T) / 512,
+    // (K T)_a = synthesis of A^T (detJ grad T) / 64 times k_T / detJ
+    double tv[8], o[8], gT[3], KT[8];
+#pragma unroll
+    for (int a = 0; a < 8; a++) tv[a] = S.T[nid[a]];
+    walsh8d(tv, o);
+#pragma unroll
+    for (int i = 0; i < 3; i++) gT[i] = fma(A[i][2], o[3], fma(A[i][1], o[2], A[i][0] * o[1]));
+    const double kf = m.k_T * f * c64;
+    double u[3];
+#pragma unroll
+    for (int mm = 0; mm < 3; mm++)
+      u[mm] = kf * fma(A[2][mm], gT[2], fma(A[1][mm], gT[1], A[0][mm] * gT[0]));
+    synth_linear(u[0], u[1], u[2], KT);
+    store_temperature_rates(P, S, m, e, nid, step, KT, q_pl, vol);
   }
 }
 
 // ---------------------------------------------------------------------------
-// deterministic block sum (fixed shuffle tree, warps combined in order)
+// Infinity or NaN, from the bits (no FP64 instruction).
+__device__ __forceinline__ bool not_finite(double v) {
+  return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
+}
+
+// deterministic block sum (fixed shuffle tree, warps combined in order); a warp
+// of zeros adds nothing and skips its five FP64 additions
 __device__ __forceinline__ double block_sum(double v, double *sh) {
+  if (__any_sync(0xffffffffu, __double_as_longlong(v) << 1 != 0)) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) sh[wid] = v;
   __syncthreads();
@@ -693,24 +983,45 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64S
   if (n < P.nn) {
     const int64_t np = P.np;
     const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
-    double fi[3] = {0.0, 0.0, 0.0};
-    for (int32_t k = 0; k < c; k++) {
-      const int64_t base = (int64_t)__ldg(&P.slot[b + k]) * 3;
-      fi[0] += __ldg(&S.fe[base]);
-      fi[1] += __ldg(&S.fe[base + 1]);
-      fi[2] += __ldg(&S.fe[base + 2]);
+    // the element forces, then the hourglass forces, each summed in list
+    // order; eight entries at a time, so that a chunk's loads are in flight
+    // together
+    double fi[3] = {0.0, 0.0, 0.0}, fh[3] = {0.0, 0.0, 0.0};
+    for (int32_t k0 = 0; k0 < c; k0 += 8) {
+      int64_t base[8];
+      double g[8][3];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int32_t sl = (k0 + j < c) ? __ldg(&P.slot[b + k0 + j]) : -1;
+        base[j] = (sl >= 0) ? (int64_t)(sl % NPE) * 3 * P.ne + sl / NPE : -1;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int q = 0; q < 3; q++) g[j][q] = (base[j] >= 0) ? __ldg(&S.fe[base[j] + q * P.ne]) : 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int q = 0; q < 3; q++) fi[q] += g[j][q];
+      if (P.hg_on) {
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+#pragma unroll
+          for (int q = 0; q < 3; q++)
+            g[j][q] = (base[j] >= 0) ? __ldg(&S.fhg[base[j] + q * P.ne]) : 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+#pragma unroll
+          for (int q = 0; q < 3; q++) fh[q] += g[j][q];
+      }
     }
     if (P.hg_on) {
-      for (int32_t k = 0; k < c; k++) {
-        const int64_t base = (int64_t)__ldg(&P.slot[b + k]) * 3;
-        fi[0] -= __ldg(&S.fhg[base]);
-        fi[1] -= __ldg(&S.fhg[base + 1]);
-        fi[2] -= __ldg(&S.fhg[base + 2]);
-      }
+#pragma unroll
+      for (int q = 0; q < 3; q++) fi[q] -= fh[q];
     }
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      if (!isfinite(fi[k])) {
+      if (not_finite(fi[k])) {
         fi[k] = 0.0;
         atomicOr(&P.st->status, 1u);
         atomicMin(&P.st->first_bad_node, (long long)n);
@@ -772,33 +1083,59 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64S
       S.cf[2 * np + n] = cf[2];
     }
     if (!P.contact && (fl & NF_REACTION)) {
+      const double fr = P.react_dim == 0 ? fi[0] : (P.react_dim == 1 ? fi[1] : fi[2]);
       if (P.rnode)
-        P.rnode[n] = fi[P.react_dim];  // summed per specimen by the reaction kernel
+        P.rnode[n] = fr;  // summed per specimen by the reaction kernel
       else
-        r = fi[P.react_dim];
+        r = fr;
     }
     const uint32_t code = P.bc[n];
     const double *bv = &P.bcval[3 * (code >> 3)];
     const double dt = P.nspec_of ? P.spec_dt[P.nspec_of[n]] : P.dt;
+    if constexpr (NPE == 8) {
+      // one reciprocal of the mass and the step's products formed once
+      const double inv_m = 1.0 / mass;
+      const double gdt = P.gamma * dt, pdt = (0.5 - P.beta) * dt, bdt2 = P.beta * dt * dt,
+                   rdt = (1.0 - P.gamma) * dt;
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      double a = (0.0 - fi[k]) / mass;
-      if (P.contact) a += cf[k] / mass;
-      if (code & (1u << k)) a = 0.0;
-      a = P.fcorr * (a - P.alpha * pa[k]);
-      double v = vp[k] + P.gamma * dt * a;
-      if (code & (1u << k)) v = bv[k];
-      double udt = dt * (vold[k] + (0.5 - P.beta) * dt * pa[k]);
-      udt += P.beta * dt * dt * a;
-      x[k] += udt;
-      u[k] += udt;
-      double vnext = v + (1.0 - P.gamma) * dt * a;
-      if (code & (1u << k)) vnext = bv[k];
-      S.x[k * np + n] = x[k];
-      S.u[k * np + n] = u[k];
-      S.v[k * np + n] = v;
-      S.pa[k * np + n] = a;
-      S.vp[k * np + n] = vnext;
+      for (int k = 0; k < 3; k++) {
+        const bool fixed = code & (1u << k);
+        double a = (cf[k] - fi[k]) * inv_m;
+        if (fixed) a = 0.0;
+        a = P.fcorr * fma(-P.alpha, pa[k], a);
+        double v = fma(gdt, a, vp[k]);
+        if (fixed) v = bv[k];
+        const double udt = fma(bdt2, a, dt * fma(pdt, pa[k], vold[k]));
+        double vnext = fma(rdt, a, v);
+        if (fixed) vnext = bv[k];
+        S.x[k * np + n] = x[k] + udt;
+        S.u[k * np + n] = u[k] + udt;
+        S.v[k * np + n] = v;
+        S.pa[k * np + n] = a;
+        S.vp[k * np + n] = vnext;
+      }
+    } else {
+      // the reference's operations in its order
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        double a = (0.0 - fi[k]) / mass;
+        if (P.contact) a += cf[k] / mass;
+        if (code & (1u << k)) a = 0.0;
+        a = P.fcorr * (a - P.alpha * pa[k]);
+        double v = vp[k] + P.gamma * dt * a;
+        if (code & (1u << k)) v = bv[k];
+        double udt = dt * (vold[k] + (0.5 - P.beta) * dt * pa[k]);
+        udt += P.beta * dt * dt * a;
+        x[k] += udt;
+        u[k] += udt;
+        double vnext = v + (1.0 - P.gamma) * dt * a;
+        if (code & (1u << k)) vnext = bv[k];
+        S.x[k * np + n] = x[k];
+        S.u[k * np + n] = u[k];
+        S.v[k * np + n] = v;
+        S.pa[k * np + n] = a;
+        S.vp[k * np + n] = vnext;
+      }
     }
     if (P.thermal) {
       // ThermalCalcs node part (Thermal.C:108-126): element-node rates of the
@@ -844,7 +1181,9 @@ __global__ void k_fp64_predict(StepParams P, Fp64State S) {
   const double *bv = &P.bcval[3 * (code >> 3)];
   for (int k = 0; k < 3; k++) {
     const double dt = P.nspec_of ? P.spec_dt[P.nspec_of[n]] : P.dt;
-    double v = S.v[k * P.np + n] + (1.0 - P.gamma) * dt * S.pa[k * P.np + n];
+    // rounded as the node kernel's predictor of the next step
+    const double v0 = S.v[k * P.np + n], a0 = S.pa[k * P.np + n], c = (1.0 - P.gamma) * dt;
+    double v = (P.npe == 8) ? fma(c, a0, v0) : v0 + c * a0;
     if (code & (1u << k)) v = bv[k];
     S.vp[k * P.np + n] = v;
   }
@@ -898,16 +1237,14 @@ void fp64_nodal(const StepParams &P, const Fp64State &S, cudaStream_t st, int in
 void fp64_elements(const StepParams &P, const Fp64State &S, cudaStream_t st) {
   const int t = spread(P.ne, kElemThreads, P.sms);
   const unsigned g = (unsigned)grid_for(P.ne, t);
-  if (P.npe == 8)
-    if (P.thermal)
-      k_fp64_elements<8, true><<<g, t, 0, st>>>(P, S);
-    else
-      k_fp64_elements<8, false><<<g, t, 0, st>>>(P, S);
+  if (P.npe == 8 && P.thermal)
+    k_fp64_hexes<true><<<g, t, 0, st>>>(P, S);
+  else if (P.npe == 8)
+    k_fp64_hexes<false><<<g, t, 0, st>>>(P, S);
+  else if (P.thermal)
+    k_fp64_tets<true><<<g, t, 0, st>>>(P, S);
   else
-    if (P.thermal)
-      k_fp64_elements<4, true><<<g, t, 0, st>>>(P, S);
-    else
-      k_fp64_elements<4, false><<<g, t, 0, st>>>(P, S);
+    k_fp64_tets<false><<<g, t, 0, st>>>(P, S);
 }
 
 void fp64_nodes(const StepParams &P, const Fp64State &S, cudaStream_t st, int node_grid) {

@@ -15,6 +15,7 @@ namespace wf {
 // Per-material constants on the device (Elastic_ / Material_, Material.cuh).
 struct MatDev {
   double K, G, sy0, H, cs0, hol_K, hol_m, eps0, eps1, E;
+  double i3GH;                               // 1 / (3 G + H), bilinear return
   double jc_B, jc_n, jc_C, jc_eps0, jc_Th;  // Johnson-Cook; jc_Th = 1 - T_h^m (host-computed)
   double jc_m, jc_Tm, jc_Tt;                 // its temperature terms (thermal coupling)
   double k_T, cp_T, exp_T;                   // conductivity, heat capacity, expansion
@@ -196,7 +197,10 @@ struct Fp64State {
   double *mass, *voln, *jr, *s0;                 // [np]
   double *vol, *vol0, *rho, *p, *pls, *sy, *detJ;  // [ne]
   double *tau, *sig, *eps, *sr, *rr;             // [6][ne]
-  double *fe, *fhg;                              // [ne][npe][3]
+  double *fe, *fhg;                              // [npe * 3][ne]
+  // adjugate of the step's Jacobian [9][ne] (hexahedra: of 8 J), tetrahedra
+  // with detJ as a tenth row
+  double *adj;
   // thermal coupling: nodal temperature, die heat per node (kept after the
   // contact ends), and the element-node temperature rates of the step in two
   // buffers [2][ne][npe] chosen by step parity (the thermal expansion of a
