@@ -2158,7 +2158,7 @@ WF_API wf_status wf_init(wf_domain *d) {
     CUDA_TRY(dalloc(d, &P.rnode, np));
   }
   // reaction history and step state
-  d->node_grid = (d->precision == WF_MIXED) ? mix_node_grid(nn) : fp64_node_grid(nn, P.sms);
+  d->node_grid = (d->precision == WF_MIXED) ? mix_node_grid(nn) : fp64_node_grid(nn, P.sms, P.tri_on);
   CUDA_TRY(dalloc(d, &P.partials, std::max(d->node_grid, 32)));
   d->hist_cap = 1 << 16;
   CUDA_TRY(dalloc(d, &P.hist, d->hist_cap));

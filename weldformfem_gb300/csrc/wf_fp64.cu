@@ -256,30 +256,28 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodal(StepParams P, Fp64S
   voln /= NPE;
   S.voln[n] = voln;
   if (P.mass_mode == 0 || init_mode) {
-    // rho_e voln / c per element, added in list order; the quotient is formed
-    // anew only where the density changes (an FP64 division is about ten
-    // FP64 instructions, and most meshes have one density; the densities are
-    // compared as bit patterns, off the FP64 pipe). Hexahedra around a node
-    // of one density share voln rho outright.
-    double mass = 0.0, share = 0.0;
-    long long rho = 0;
-    bool same = true;
-    if (NPE == 8)
-      for (int32_t k = 0; k < c; k++) {
-        const long long r = __double_as_longlong(__ldg(&S.rho[elem(k)]));
-        same &= k == 0 || r == rho;
-        rho = r;
-      }
-    if (NPE == 8 && same && c > 0) {
-      mass = __longlong_as_double(rho) * voln;
+    // sum of rho_e voln / c over the node's elements. The densities of a mesh
+    // of one material differ in their last bits (rho_0 vol_0 / vol_0), so
+    // every entry needs its own quotient: FP64 divisions at about ten FP64
+    // instructions each.
+    double mass = 0.0;
+    if constexpr (NPE == 8) {
+      // the densities' sum times voln / c; the division is exact, a
+      // multiplication, for the 1, 2, 4 or 8 elements of a box mesh's nodes
+      double rs = 0.0;
+      for (int32_t k = 0; k < c; k++) rs += __ldg(&S.rho[elem(k)]);
+      mass = rs * voln;
+      if (c & (c - 1)) mass /= c;
+      else mass *= (c == 8 ? 0.125 : c == 4 ? 0.25 : c == 2 ? 0.5 : 1.0 / c);
     } else {
+      // the reference's sum in list order, bit for bit: x / c as q = x (1 / c)
+      // corrected by its remainder, correctly rounded when 1 / c is (Markstein's
+      // theorem; x / c for c up to 4096 checked on random x)
+      const double dc = c, rc = 1.0 / dc;
       for (int32_t k = 0; k < c; k++) {
-        const double r = __ldg(&S.rho[elem(k)]);
-        if (k == 0 || __double_as_longlong(r) != rho) {
-          rho = __double_as_longlong(r);
-          share = r * voln / c;
-        }
-        mass += share;
+        const double x = __ldg(&S.rho[elem(k)]) * voln;
+        const double q = x * rc;
+        mass += fma(fma(-q, dc, x), rc, q);
       }
     }
     S.mass[n] = mass;
@@ -435,15 +433,11 @@ __device__ __forceinline__ double tangent_modulus(const StepParams &P, const Mat
 // the plastic strain increment along the returned stress, shear terms doubled.
 __device__ __forceinline__ double plastic_heat(const StepParams &P, const double (&SG)[6],
                                                double dep, double sy, double dt) {
-  const double f = dep / sy;
-  const double idt = 1. / dt;
-  const double ixx = f * (SG[0] - 0.5 * (SG[1] + SG[2]));
-  const double iyy = f * (SG[1] - 0.5 * (SG[0] + SG[2]));
-  const double izz = f * (SG[2] - 0.5 * (SG[0] + SG[1]));
-  const double ixy = 1.5 * f * (SG[3]), ixz = 1.5 * f * (SG[5]), iyz = 1.5 * f * (SG[4]);
-  return P.plheat_frac * (SG[0] * (ixx * idt) + 2.0 * SG[3] * (ixy * idt) +
-                          2.0 * SG[5] * (ixz * idt) + SG[1] * (iyy * idt) +
-                          2.0 * SG[4] * (iyz * idt) + SG[2] * (izz * idt));
+  // sigma : increment with the increment (3/2) dep / sy dev(sigma) written out
+  const double a = SG[0] - SG[1], b = SG[1] - SG[2], c = SG[2] - SG[0];
+  const double nn = 0.5 * fma(a, a, fma(b, b, c * c));
+  const double ss = fma(SG[3], SG[3], fma(SG[4], SG[4], SG[5] * SG[5]));
+  return P.plheat_frac * (nn + 3.0 * ss) * dep / (sy * dt);
 }
 
 // Artificial viscosity (calcArtificialViscosity, Mechanical.C:1948-1977; serial
@@ -492,6 +486,89 @@ __device__ __forceinline__ void store_temperature_rates(const StepParams &P, con
   for (int a = 0; a < NPE; a++) cur[a] = (heat - KT[a]) / S.mass[nid[a]];
 }
 
+// The stress part of an element in FMA form (hexahedra, and tetrahedra with
+// thermal coupling): Jaumann rate, radial return, artificial viscosity; writes
+// the element's fields and returns sigma in SG and the plastic heat. In: the
+// strain rate, the spin and the pressure. The reference's yy and zz Jaumann
+// terms are (a - b) + (b - a), exactly zero.
+template <int NPE, bool TH>
+__device__ __forceinline__ void stress_step(const StepParams &P, const Fp64State &S,
+                                            const MatDev &m, int32_t mat_id, int64_t e,
+                                            const int32_t (&nid)[NPE], double s00, double s11,
+                                            double s22, double s01, double s12, double s02,
+                                            double w01, double w12, double w02, double p,
+                                            double vol, double (&SG)[6], double &q_pl) {
+  const int64_t ne = P.ne;
+  // Jaumann rate with the reference's product, then the radial return; the
+  // pressure drops out of the trial stress's deviator
+  const double dt = P.espec ? P.spec_dt[P.espec[e]] : P.dt;
+  double t0 = S.tau[e], t1 = S.tau[ne + e], t2 = S.tau[2 * ne + e];
+  double t3 = S.tau[3 * ne + e], t4 = S.tau[4 * ne + e], t5 = S.tau[5 * ne + e];
+  {
+    const double g2 = 2.0 * m.G * dt;
+    const double c = (1.0 / 3.0) * (s00 + s11 + s22);
+    const double q0 = 2.0 * fma(t3, w01, t5 * w02);
+    const double q3 = fma(w01, t0 + t1, fma(w02, t4, -(t5 * w12)));
+    const double q4 = fma(w12, t1 + t2, fma(w02, t3, -(t5 * w01)));
+    const double q5 = fma(w02, t0 + t2, fma(w12, t3, w01 * t4));
+    t0 = fma(q0, dt, fma(s00 - c, g2, t0));
+    t1 = fma(s11 - c, g2, t1);
+    t2 = fma(s22 - c, g2, t2);
+    t3 = fma(q3, dt, fma(s01, g2, t3));
+    t4 = fma(q4, dt, fma(s12, g2, t4));
+    t5 = fma(q5, dt, fma(s02, g2, t5));
+  }
+  const double tm = (1.0 / 3.0) * (t0 + t1 + t2);
+  const double d0s = t0 - tm, d1s = t1 - tm, d2s = t2 - tm;
+  // sig_trial^2 = 3 J2
+  const double q2 = 1.5 * fma(d0s, d0s, fma(d1s, d1s, fma(d2s, d2s,
+                          2.0 * fma(t3, t3, fma(t4, t4, t5 * t5)))));
+  double pls = S.pls[e];
+  LawState law;
+  const double sy = yield_stress<NPE, TH>(P, S, m, mat_id, nid, pls, s00, s11, s22, s01, s12, s02,
+                                          law);
+  double dep = 0.0;
+  // sy < sig_trial, without the square root for elements well inside the
+  // yield surface (a NaN enters and fails the exact test, as sy < NaN does)
+  if (sy < 0.0 || !(q2 < sy * sy)) {
+    // (0 and infinity keep the square root's value)
+    const double rs = rsqrt(q2), sig_trial = (q2 > 0.0 && !isinf(q2)) ? q2 * rs : q2;
+    if (sy < sig_trial) {
+      const double G3 = 3.0 * m.G;
+      const double dgamma = (m.model == WF_MAT_BILINEAR)
+                                ? (sig_trial - sy) * m.i3GH
+                                : (sig_trial - sy) / (G3 + tangent_modulus(P, m, mat_id, pls, law));
+      const double factor = 1.0 - (G3 * dgamma) * rs;
+      t0 = d0s * factor; t1 = d1s * factor; t2 = d2s * factor;
+      t3 = t3 * factor; t4 = t4 * factor; t5 = t5 * factor;
+      pls += dgamma;
+      dep = dgamma;
+    }
+  }
+  SG[0] = t0 - p; SG[1] = t1 - p; SG[2] = t2 - p;
+  SG[3] = t3; SG[4] = t4; SG[5] = t5;
+  q_pl = 0.0;
+  if (TH && dep > 0.0) q_pl = plastic_heat(P, SG, dep, sy, dt);
+  S.eps[e] = fma(s00, dt, S.eps[e]);
+  S.eps[ne + e] = fma(s11, dt, S.eps[ne + e]);
+  S.eps[2 * ne + e] = fma(s22, dt, S.eps[2 * ne + e]);
+  S.eps[3 * ne + e] = fma(s01, dt, S.eps[3 * ne + e]);
+  S.eps[4 * ne + e] = fma(s12, dt, S.eps[4 * ne + e]);
+  S.eps[5 * ne + e] = fma(s02, dt, S.eps[5 * ne + e]);
+  if (P.av_on) add_viscosity(P, S, m, e, s00 + s11 + s22, vol, SG);
+  S.p[e] = p;
+  S.pls[e] = pls;
+  S.sy[e] = sy;
+#pragma unroll
+  for (int c = 0; c < 6; c++) S.sig[c * ne + e] = SG[c];
+  S.tau[e] = t0; S.tau[ne + e] = t1; S.tau[2 * ne + e] = t2;
+  S.tau[3 * ne + e] = t3; S.tau[4 * ne + e] = t4; S.tau[5 * ne + e] = t5;
+  S.sr[e] = s00; S.sr[ne + e] = s11; S.sr[2 * ne + e] = s22;
+  S.sr[3 * ne + e] = s01; S.sr[4 * ne + e] = s12; S.sr[5 * ne + e] = s02;
+  // the spin's diagonal stays zero (rows 0..2 are never written)
+  S.rr[3 * ne + e] = w01; S.rr[4 * ne + e] = w12; S.rr[5 * ne + e] = w02;
+}
+
 // ---------------------------------------------------------------------------
 // elements: calcElemJAndDerivatives, calcElemStrainRates (Mechanical.C:41-126),
 // calcElemPressure (:691-819) or calcElemPressureANP (:1220-1250),
@@ -504,7 +581,6 @@ __device__ __forceinline__ void store_temperature_rates(const StepParams &P, con
 //
 // Tetrahedra: the reference's operations in its order (FMA contraction off),
 // bit for bit the reference's forces.
-template <bool TH>
 __global__ void __launch_bounds__(kElemThreads) k_fp64_tets(StepParams P, Fp64State S) {
   constexpr int NPE = 4;
   int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -553,13 +629,6 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_tets(StepParams P, Fp64St
   }
   s01 = s01 * 0.5; s02 = s02 * 0.5; s12 = s12 * 0.5;
   w01 = w01 * 0.5; w02 = w02 * 0.5; w12 = w12 * 0.5;
-  const long long step = TH ? P.st->step : 0;
-  if constexpr (TH) {
-    const double c = thermal_strain_rate(P, S, m, nid, step);
-    s00 = s00 - c;
-    s11 = s11 - c;
-    s22 = s22 - c;
-  }
   const double p = element_pressure(P, S, m, e, nid, vol, div_v);
 
   // Jaumann rate + radial return (CalcStressStrain). The tensor3 algebra of
@@ -602,9 +671,8 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_tets(StepParams P, Fp64St
   const double sig_trial = sqrt(3.0 * J2);
   double pls = S.pls[e];
   LawState law;
-  const double sy = yield_stress<NPE, TH>(P, S, m, mat_id, nid, pls, s00, s11, s22, s01, s12, s02,
+  const double sy = yield_stress<NPE, false>(P, S, m, mat_id, nid, pls, s00, s11, s22, s01, s12, s02,
                                           law);
-  double dep = 0.0;
   if (sy < sig_trial) {
     const double H = tangent_modulus(P, m, mat_id, pls, law);
     const double G = m.G;
@@ -613,11 +681,8 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_tets(StepParams P, Fp64St
     t0 = d0s * factor; t1 = d1s * factor; t2 = d2s * factor;
     t3 = t3 * factor; t4 = t4 * factor; t5 = t5 * factor;
     pls += dgamma;
-    dep = dgamma;
   }
   double SG[6] = {t0 - p, t1 - p, t2 - p, t3, t4, t5};
-  double q_pl = 0.0;
-  if (TH && dep > 0.0) q_pl = plastic_heat(P, SG, dep, sy, dt);
   // total strain: eps = eps + dt * D
   {
     double e0 = S.eps[e], e1 = S.eps[ne + e], e2 = S.eps[2 * ne + e];
@@ -657,23 +722,85 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_tets(StepParams P, Fp64St
     S.fe[(3 * a + 1) * ne + e] = f1 * w;
     S.fe[(3 * a + 2) * ne + e] = f2 * w;
   }
-  if constexpr (TH) {
-    // conduction (K T)_i = (sum_d dN_i detJ sum_k dN_k detJ T_k) k_T / detJ w:
-    // through the temperature gradient, 24 products instead of a 4 x 4 matrix
-    double gT[3] = {0.0, 0.0, 0.0};
+}
+
+// Tetrahedra with thermal coupling: the same quantities from the velocity
+// gradient, (dN detJ) v / detJ with the velocities relative to node 0 (dN_0 is
+// minus the sum of the others), in FMA form. The reference's node loop takes
+// 156 FP64 instructions for the strain rate and spin, this 57, and its 4 x 4
+// conduction matrix 16 divisions.
+__global__ void __launch_bounds__(kElemThreads) k_fp64_tets_thermal(StepParams P, Fp64State S) {
+  constexpr int NPE = 4;
+  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= P.ne) return;
+  const int64_t ne = P.ne;
+  int32_t nid[NPE];
 #pragma unroll
-    for (int a = 0; a < NPE; a++) {
-      const double Ta = S.T[nid[a]];
+  for (int a = 0; a < NPE; a++) nid[a] = __ldg(&P.elnod[a * ne + e]);
+  // A[k][m]: dN_(m+1)/dx_k detJ; node 0 has minus the row sums
+  double A[3][3];
 #pragma unroll
-      for (int dd = 0; dd < 3; dd++) gT[dd] = fma(dH[dd][a], Ta, gT[dd]);
-    }
-    const double kf = m.k_T * f * w;
-    double KT[NPE];
+  for (int k = 0; k < 3; k++)
 #pragma unroll
-    for (int a = 0; a < NPE; a++)
-      KT[a] = kf * fma(dH[0][a], gT[0], fma(dH[1][a], gT[1], dH[2][a] * gT[2]));
-    store_temperature_rates(P, S, m, e, nid, step, KT, q_pl, vol);
+    for (int mm = 0; mm < 3; mm++) A[k][mm] = __ldg(&S.adj[(3 * k + mm) * ne + e]);
+  const double detJ = __ldg(&S.adj[9 * ne + e]), vol = __ldg(&S.vol[e]);
+  const int32_t mat_id = P.emat ? __ldg(&P.emat[e]) : 0;
+  const MatDev &m = P.mats[mat_id];
+  const double f = 1.0 / detJ, fh = 0.5 * f;
+  double G[3][3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const double v0 = __ldg(&S.vp[k * P.np + nid[0]]);
+#pragma unroll
+    for (int mm = 0; mm < 3; mm++) G[mm][k] = __ldg(&S.vp[k * P.np + nid[mm + 1]]) - v0;
   }
+  auto AG = [&](int i, int k) {
+    return fma(A[i][2], G[2][k], fma(A[i][1], G[1][k], A[i][0] * G[0][k]));
+  };
+  const double l10 = AG(1, 0), l01 = AG(0, 1), l21 = AG(2, 1), l12 = AG(1, 2), l20 = AG(2, 0),
+               l02 = AG(0, 2);
+  const double a00 = AG(0, 0), a11 = AG(1, 1), a22 = AG(2, 2);
+  const double s01 = fh * (l10 + l01), w01 = fh * (l10 - l01);
+  const double s12 = fh * (l21 + l12), w12 = fh * (l21 - l12);
+  const double s02 = fh * (l20 + l02), w02 = fh * (l20 - l02);
+  const long long step = P.st->step;
+  const double c = thermal_strain_rate(P, S, m, nid, step);
+  const double s00 = fma(a00, f, -c), s11 = fma(a11, f, -c), s22 = fma(a22, f, -c);
+  const double p = element_pressure(P, S, m, e, nid, vol, P.stab_on ? a00 + a11 + a22 : 0.0);
+  double SG[6], q_pl;
+  stress_step<NPE, true>(P, S, m, mat_id, e, nid, s00, s11, s22, s01, s12, s02, w01, w12, w02, p,
+                         vol, SG, q_pl);
+  // forces f = w B^T sigma; node 0 balances the others
+  const double w = weight<NPE>();
+  const double Sk[3][3] = {{SG[0] * w, SG[3] * w, SG[5] * w},
+                           {SG[3] * w, SG[1] * w, SG[4] * w},
+                           {SG[5] * w, SG[4] * w, SG[2] * w}};
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    double sum = 0.0;
+#pragma unroll
+    for (int mm = 0; mm < 3; mm++) {
+      const double v = fma(A[2][mm], Sk[2][k], fma(A[1][mm], Sk[1][k], A[0][mm] * Sk[0][k]));
+      S.fe[(3 * (mm + 1) + k) * ne + e] = v;
+      sum += v;
+    }
+    S.fe[k * ne + e] = -sum;
+  }
+  // conduction (K T)_i = (sum_d dN_i detJ sum_k dN_k detJ T_k) k_T / detJ w
+  // through the temperature gradient, the temperatures relative to node 0
+  const double T0 = S.T[nid[0]];
+  double dT[3], gT[3], KT[NPE];
+#pragma unroll
+  for (int mm = 0; mm < 3; mm++) dT[mm] = S.T[nid[mm + 1]] - T0;
+  const double kf = m.k_T * f * w;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+    gT[i] = kf * fma(A[i][2], dT[2], fma(A[i][1], dT[1], A[i][0] * dT[0]));
+#pragma unroll
+  for (int mm = 0; mm < 3; mm++)
+    KT[mm + 1] = fma(A[2][mm], gT[2], fma(A[1][mm], gT[1], A[0][mm] * gT[0]));
+  KT[0] = -(KT[1] + KT[2] + KT[3]);
+  store_temperature_rates(P, S, m, e, nid, step, KT, q_pl, vol);
 }
 
 // Hexahedra: the same quantities through the Walsh sums of the nodal values,
@@ -683,8 +810,7 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_tets(StepParams P, Fp64St
 // X = 8 J the three derivative sums of the coordinates, A = adj(X) and
 // D = det(X): volume D / 64, velocity gradient A G / D with G the velocity's
 // derivative sums, nodal forces the synthesis of A^T sigma / 64, and the
-// powers of two are exact. The reference's yy and zz Jaumann terms are
-// (a - b) + (b - a), exactly zero.
+// powers of two are exact.
 template <bool TH>
 __global__ void __launch_bounds__(kElemThreads) k_fp64_hexes(StepParams P, Fp64State S) {
   constexpr int NPE = 8;
@@ -746,73 +872,9 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_hexes(StepParams P, Fp64S
   }
   const double p = element_pressure(P, S, m, e, nid, vol, div_v);
 
-  // Jaumann rate with the reference's product, then the radial return; the
-  // pressure drops out of the trial stress's deviator
-  const double dt = P.espec ? P.spec_dt[P.espec[e]] : P.dt;
-  double t0 = S.tau[e], t1 = S.tau[ne + e], t2 = S.tau[2 * ne + e];
-  double t3 = S.tau[3 * ne + e], t4 = S.tau[4 * ne + e], t5 = S.tau[5 * ne + e];
-  {
-    const double g2 = 2.0 * m.G * dt;
-    const double c = (1.0 / 3.0) * (s00 + s11 + s22);
-    const double q0 = 2.0 * fma(t3, w01, t5 * w02);
-    const double q3 = fma(w01, t0 + t1, fma(w02, t4, -(t5 * w12)));
-    const double q4 = fma(w12, t1 + t2, fma(w02, t3, -(t5 * w01)));
-    const double q5 = fma(w02, t0 + t2, fma(w12, t3, w01 * t4));
-    t0 = fma(q0, dt, fma(s00 - c, g2, t0));
-    t1 = fma(s11 - c, g2, t1);
-    t2 = fma(s22 - c, g2, t2);
-    t3 = fma(q3, dt, fma(s01, g2, t3));
-    t4 = fma(q4, dt, fma(s12, g2, t4));
-    t5 = fma(q5, dt, fma(s02, g2, t5));
-  }
-  const double tm = (1.0 / 3.0) * (t0 + t1 + t2);
-  const double d0s = t0 - tm, d1s = t1 - tm, d2s = t2 - tm;
-  // sig_trial^2 = 3 J2
-  const double q2 = 1.5 * fma(d0s, d0s, fma(d1s, d1s, fma(d2s, d2s,
-                          2.0 * fma(t3, t3, fma(t4, t4, t5 * t5)))));
-  double pls = S.pls[e];
-  LawState law;
-  const double sy = yield_stress<NPE, TH>(P, S, m, mat_id, nid, pls, s00, s11, s22, s01, s12, s02,
-                                          law);
-  double dep = 0.0;
-  // sy < sig_trial, without the square root for elements well inside the
-  // yield surface (a NaN enters and fails the exact test, as sy < NaN does)
-  if (sy < 0.0 || !(q2 < sy * sy)) {
-    // (0 and infinity keep the square root's value)
-    const double rs = rsqrt(q2), sig_trial = (q2 > 0.0 && !isinf(q2)) ? q2 * rs : q2;
-    if (sy < sig_trial) {
-      const double G3 = 3.0 * m.G;
-      const double dgamma = (m.model == WF_MAT_BILINEAR)
-                                ? (sig_trial - sy) * m.i3GH
-                                : (sig_trial - sy) / (G3 + tangent_modulus(P, m, mat_id, pls, law));
-      const double factor = 1.0 - (G3 * dgamma) * rs;
-      t0 = d0s * factor; t1 = d1s * factor; t2 = d2s * factor;
-      t3 = t3 * factor; t4 = t4 * factor; t5 = t5 * factor;
-      pls += dgamma;
-      dep = dgamma;
-    }
-  }
-  double SG[6] = {t0 - p, t1 - p, t2 - p, t3, t4, t5};
-  double q_pl = 0.0;
-  if (TH && dep > 0.0) q_pl = plastic_heat(P, SG, dep, sy, dt);
-  S.eps[e] = fma(s00, dt, S.eps[e]);
-  S.eps[ne + e] = fma(s11, dt, S.eps[ne + e]);
-  S.eps[2 * ne + e] = fma(s22, dt, S.eps[2 * ne + e]);
-  S.eps[3 * ne + e] = fma(s01, dt, S.eps[3 * ne + e]);
-  S.eps[4 * ne + e] = fma(s12, dt, S.eps[4 * ne + e]);
-  S.eps[5 * ne + e] = fma(s02, dt, S.eps[5 * ne + e]);
-  if (P.av_on) add_viscosity(P, S, m, e, s00 + s11 + s22, vol, SG);
-  S.p[e] = p;
-  S.pls[e] = pls;
-  S.sy[e] = sy;
-#pragma unroll
-  for (int c = 0; c < 6; c++) S.sig[c * ne + e] = SG[c];
-  S.tau[e] = t0; S.tau[ne + e] = t1; S.tau[2 * ne + e] = t2;
-  S.tau[3 * ne + e] = t3; S.tau[4 * ne + e] = t4; S.tau[5 * ne + e] = t5;
-  S.sr[e] = s00; S.sr[ne + e] = s11; S.sr[2 * ne + e] = s22;
-  S.sr[3 * ne + e] = s01; S.sr[4 * ne + e] = s12; S.sr[5 * ne + e] = s02;
-  // the spin's diagonal stays zero (rows 0..2 are never written)
-  S.rr[3 * ne + e] = w01; S.rr[4 * ne + e] = w12; S.rr[5 * ne + e] = w02;
+  double SG[6], q_pl;
+  stress_step<NPE, TH>(P, S, m, mat_id, e, nid, s00, s11, s22, s01, s12, s02, w01, w12, w02, p, vol,
+                       SG, q_pl);
 
   // forces: synthesis of A^T sigma / 64
   const double c64 = 1.0 / 64.0;
@@ -871,42 +933,131 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   return t;
 }
 
-// Rigid triangle-mesh contact of one external node (Domain_d::CalcContactForces,
-// Contact.C:31-334): the first triangle, in order, that the node penetrates
-// (d < 0 with its projection inside the triangle) gives the penalty normal
-// force pf * min(E A / l, 0.2 m / dt^2) * d plus damping, then Coulomb
+// Rigid triangle-mesh contact of the external nodes (Domain_d::CalcContactForces,
+// Contact.C:31-334). tri_search finds a node's triangle: the first one, in
+// order, that it penetrates (d < 0) with its projection inside. tri_contact
+// forms its contact force.
+//
+// Does node x's plane distance and projection hit triangle j (Contact.C:58-120)?
+__device__ __forceinline__ bool tri_hit(const StepParams &P, int32_t j, const double (&x)[3]) {
+  const double n0 = P.tri_nrm[3 * j], n1 = P.tri_nrm[3 * j + 1], n2 = P.tri_nrm[3 * j + 2];
+  const double dd = (n0 * x[0] + n1 * x[1] + n2 * x[2]) - P.tri_pp[j];
+  if (!(dd < 0)) return false;
+  const double Q[3] = {x[0] - n0 * dd, x[1] - n1 * dd, x[2] - n2 * dd};
+  for (int l = 0; l < 3; l++) {
+    const int nx = l + 1 > 2 ? 0 : l + 1;
+    const double *a = &P.tri_x[3 * P.tri_el[3 * j + l]];
+    const double *b = &P.tri_x[3 * P.tri_el[3 * j + nx]];
+    const double e1[3] = {b[0] - a[0], b[1] - a[1], b[2] - a[2]};
+    const double e2[3] = {Q[0] - a[0], Q[1] - a[1], Q[2] - a[2]};
+    const double c0 = e1[1] * e2[2] - e1[2] * e2[1];
+    const double c1 = e1[2] * e2[0] - e1[0] * e2[2];
+    const double c2 = e1[0] * e2[1] - e1[1] * e2[0];
+    const double crit = c0 * n0 + c1 * n1 + c2 * n2;
+    if (crit < 0.0) return false;
+  }
+  return true;
+}
+
+// The search of a block's nodes, all threads of the block taking part (act:
+// this thread has an external node). The FP64 test costs about 70 FP64
+// instructions a triangle, 16 cycles each on an SM of GB300, so the block
+// first stages the triangles as FP32 copies relative to the die's first node
+// (chunks of kTriChunk in shared memory) and rejects in FP32 what is certainly
+// missed; what is left, mostly one or two triangles a node, takes the FP64
+// test, in order, so the outcome is the FP64 search's. The margins: with R the
+// largest relative coordinate involved, every FP32 quantity of length is
+// within 2^-20 R and every product of two lengths within 2.4e-5 R^2 of its
+// exact value; a distance is rejected above 1e-5 R, an edge test below
+// -1e-4 R^2, and a comparison that involves an infinity or NaN rejects nothing.
+// 98 triangles over 13,671 nodes: node kernel 255 -> 24 us.
+constexpr int kTriChunk = 64;
+struct TriFilter {
+  float n[3], pp, v[3][3], r;
+};
+__device__ __forceinline__ int32_t tri_search(const StepParams &P, bool act,
+                                              const double (&x)[3], TriFilter *tf) {
+  int32_t hit = -1;
+  const double o0 = P.tri_x[0], o1 = P.tri_x[1], o2 = P.tri_x[2];
+  float xf[3] = {0.f, 0.f, 0.f};
+  if (act) {
+    xf[0] = (float)(x[0] - o0);
+    xf[1] = (float)(x[1] - o1);
+    xf[2] = (float)(x[2] - o2);
+  }
+  const float rx = fmaxf(fmaxf(fabsf(xf[0]), fabsf(xf[1])), fabsf(xf[2]));
+  for (int32_t j0 = 0; j0 < P.tri_ne; j0 += kTriChunk) {
+    // also the barrier before a chunk is overwritten
+    if (!__syncthreads_or(act && hit < 0)) break;
+    const int m = min(kTriChunk, P.tri_ne - j0);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+      const int32_t j = j0 + i;
+      TriFilter f;
+      const double n0 = P.tri_nrm[3 * j], n1 = P.tri_nrm[3 * j + 1], n2 = P.tri_nrm[3 * j + 2];
+      f.n[0] = (float)n0;
+      f.n[1] = (float)n1;
+      f.n[2] = (float)n2;
+      f.pp = (float)(P.tri_pp[j] - (n0 * o0 + n1 * o1 + n2 * o2));
+      f.r = 0.f;
+#pragma unroll
+      for (int l = 0; l < 3; l++) {
+        const double *a = &P.tri_x[3 * P.tri_el[3 * j + l]];
+        f.v[l][0] = (float)(a[0] - o0);
+        f.v[l][1] = (float)(a[1] - o1);
+        f.v[l][2] = (float)(a[2] - o2);
+#pragma unroll
+        for (int k = 0; k < 3; k++) f.r = fmaxf(f.r, fabsf(f.v[l][k]));
+      }
+      tf[i] = f;
+    }
+    __syncthreads();
+    if (act && hit < 0) {
+      for (int i = 0; i < m; i++) {
+        const TriFilter &f = tf[i];
+        const float R = rx + f.r;
+        const float d = f.n[0] * xf[0] + f.n[1] * xf[1] + f.n[2] * xf[2] - f.pp;
+        if (d > 1e-5f * R) continue;
+        const float q0 = xf[0] - f.n[0] * d, q1 = xf[1] - f.n[1] * d, q2 = xf[2] - f.n[2] * d;
+        const float lim = -1e-4f * R * R;
+        bool out = false;
+#pragma unroll
+        for (int l = 0; l < 3; l++) {
+          const int nx = l == 2 ? 0 : l + 1;
+          const float a0 = f.v[nx][0] - f.v[l][0], a1 = f.v[nx][1] - f.v[l][1],
+                      a2 = f.v[nx][2] - f.v[l][2];
+          const float b0 = q0 - f.v[l][0], b1 = q1 - f.v[l][1], b2 = q2 - f.v[l][2];
+          out |= (a1 * b2 - a2 * b1) * f.n[0] + (a2 * b0 - a0 * b2) * f.n[1] +
+                     (a0 * b1 - a1 * b0) * f.n[2] < lim;
+        }
+        if (out) continue;
+        if (tri_hit(P, j0 + i, x)) {
+          hit = j0 + i;
+          break;
+        }
+      }
+    }
+  }
+  return hit;
+}
+
+// The contact force of an external node on its triangle j (-1: none): penalty
+// normal force pf * min(E A / l, 0.2 m / dt^2) * d plus damping, then Coulomb
 // friction from the accumulated tangential slip (static cap, else dynamic
 // force along -v_t, slip reset). A node out of contact keeps its last contact
 // force, as in the reference. Returns the normal-force magnitude when the
 // triangle belongs to rigid body 0, the only body the reaction sums
 // (Contact.C:229, :326-329), else 0.
 __device__ __forceinline__ double tri_contact(const StepParams &P, const Fp64State &S, int64_t n,
-                                              const double (&x)[3], const double (&v)[3],
-                                              double m, double (&cf)[3]) {
+                                              int32_t j, const double (&x)[3],
+                                              const double (&v)[3], double m, double (&cf)[3]) {
   const int64_t np = P.np;
   cf[0] = S.cf[n];
   cf[1] = S.cf[np + n];
   cf[2] = S.cf[2 * np + n];
   double cfn = 0.0;
-  for (int32_t j = 0; j < P.tri_ne; j++) {
+  if (j >= 0) {
     const double n0 = P.tri_nrm[3 * j], n1 = P.tri_nrm[3 * j + 1], n2 = P.tri_nrm[3 * j + 2];
     const double dd = (n0 * x[0] + n1 * x[1] + n2 * x[2]) - P.tri_pp[j];
-    if (!(dd < 0)) continue;
-    const double Q[3] = {x[0] - n0 * dd, x[1] - n1 * dd, x[2] - n2 * dd};
-    bool inside = true;
-    for (int l = 0; l < 3 && inside; l++) {
-      const int nx = l + 1 > 2 ? 0 : l + 1;
-      const double *a = &P.tri_x[3 * P.tri_el[3 * j + l]];
-      const double *b = &P.tri_x[3 * P.tri_el[3 * j + nx]];
-      const double e1[3] = {b[0] - a[0], b[1] - a[1], b[2] - a[2]};
-      const double e2[3] = {Q[0] - a[0], Q[1] - a[1], Q[2] - a[2]};
-      const double c0 = e1[1] * e2[2] - e1[2] * e2[1];
-      const double c1 = e1[2] * e2[0] - e1[0] * e2[2];
-      const double c2 = e1[0] * e2[1] - e1[1] * e2[0];
-      const double crit = c0 * n0 + c1 * n1 + c2 * n2;
-      if (crit < 0.0) inside = false;
-    }
-    if (!inside) continue;
     const double dt = P.dt;
     const double v_reln = v[0] * n0 + v[1] * n1 + v[2] * n2;
     const double kgeo = P.tri_E0 * P.node_area[n] / P.nodlen[n];
@@ -959,7 +1110,6 @@ __device__ __forceinline__ double tri_contact(const StepParams &P, const Fp64Sta
     if (P.tri_mid[j] != 0) cfn = 0.0;
     // heat from the die (Contact.C:309), kept after the contact ends
     if (P.thermal) S.qc[n] = P.tri_hc * P.node_area[n] * (P.tri_Tdie - S.T[n]);
-    break;
   }
   S.cf[n] = cf[0];
   S.cf[np + n] = cf[1];
@@ -973,13 +1123,25 @@ __device__ __forceinline__ double tri_contact(const StepParams &P, const Fp64Sta
 // UpdateCorrectionAccVel (Domain_d.C:981-997), ImposeBCV,
 // UpdateCorrectionPos (:1005-1025) and the next step's UpdatePrediction
 // (:961-974) + ImposeBCV, which this kernel hands to the next step as vp.
-template <int NPE>
+// TRI: triangle-mesh dies.
+template <int NPE, bool TRI>
 __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64State S) {
   __shared__ double sh[kNodeThreads / 32];
   __shared__ bool am_last;
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const double time = P.st->time;
   double r = 0.0;
+  int32_t hit = -1;
+  if constexpr (TRI) {
+    __shared__ TriFilter tf[kTriChunk];
+    const bool ext = n < P.nn && (P.nflag[n] & NF_CONTACT);
+    double x[3] = {0.0, 0.0, 0.0};
+    if (ext) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) x[k] = S.x[k * P.np + n];
+    }
+    hit = tri_search(P, ext, x, tf);
+  }
   if (n < P.nn) {
     const int64_t np = P.np;
     const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
@@ -1040,8 +1202,8 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64S
       u[k] = S.u[k * np + n];
     }
     double cf[3] = {0.0, 0.0, 0.0};
-    if (P.tri_on) {
-      if (fl & NF_CONTACT) r = tri_contact(P, S, n, x, vp, mass, cf);
+    if constexpr (TRI) {
+      if (fl & NF_CONTACT) r = tri_contact(P, S, n, hit, x, vp, mass, cf);
     } else if (P.contact && (fl & NF_CONTACT)) {
       // rigid plane, outward normal (0, 0, -1), at z0 + vz * Time
       const double zd = P.c_z0 + P.c_vz * time;
@@ -1169,7 +1331,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64S
       P.st->time = time + P.dt;
       P.st->done_blocks = 0u;
     }
-    if (P.tri_on) tri_move<false>(P, time);
+    if constexpr (TRI) tri_move<false>(P, time);
   }
 }
 
@@ -1212,8 +1374,15 @@ static int spread(int64_t n, int max_threads, int sms) {
   return t;
 }
 
-int fp64_node_grid(int64_t nn, int sms) {
-  return (int)grid_for(nn, spread(nn, kNodeThreads, sms));
+// Node kernel: with a triangle-mesh die its blocks stage the triangles and its
+// last block moves the die, so they keep at least 128 threads.
+static int node_threads(int64_t nn, int sms, bool tri) {
+  const int t = spread(nn, kNodeThreads, sms);
+  return tri ? std::max(t, 128) : t;
+}
+
+int fp64_node_grid(int64_t nn, int sms, bool tri) {
+  return (int)grid_for(nn, node_threads(nn, sms, tri));
 }
 
 void fp64_geometry(const StepParams &P, const Fp64State &S, cudaStream_t st, bool store_detj) {
@@ -1242,18 +1411,22 @@ void fp64_elements(const StepParams &P, const Fp64State &S, cudaStream_t st) {
   else if (P.npe == 8)
     k_fp64_hexes<false><<<g, t, 0, st>>>(P, S);
   else if (P.thermal)
-    k_fp64_tets<true><<<g, t, 0, st>>>(P, S);
+    k_fp64_tets_thermal<<<g, t, 0, st>>>(P, S);
   else
-    k_fp64_tets<false><<<g, t, 0, st>>>(P, S);
+    k_fp64_tets<<<g, t, 0, st>>>(P, S);
 }
 
 void fp64_nodes(const StepParams &P, const Fp64State &S, cudaStream_t st, int node_grid) {
-  // node_grid = fp64_node_grid(P.nn, P.sms): blocks of the spread size
-  const int t = spread(P.nn, kNodeThreads, P.sms);
-  if (P.npe == 8)
-    k_fp64_nodes<8><<<node_grid, t, 0, st>>>(P, S);
+  // node_grid = fp64_node_grid(P.nn, P.sms, P.tri_on): blocks of that size
+  const int t = node_threads(P.nn, P.sms, P.tri_on);
+  if (P.npe == 8 && P.tri_on)
+    k_fp64_nodes<8, true><<<node_grid, t, 0, st>>>(P, S);
+  else if (P.npe == 8)
+    k_fp64_nodes<8, false><<<node_grid, t, 0, st>>>(P, S);
+  else if (P.tri_on)
+    k_fp64_nodes<4, true><<<node_grid, t, 0, st>>>(P, S);
   else
-    k_fp64_nodes<4><<<node_grid, t, 0, st>>>(P, S);
+    k_fp64_nodes<4, false><<<node_grid, t, 0, st>>>(P, S);
 }
 
 void fp64_predict(const StepParams &P, const Fp64State &S, cudaStream_t st) {

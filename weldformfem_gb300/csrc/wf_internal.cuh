@@ -336,7 +336,7 @@ void fp64_elements(const StepParams &P, const Fp64State &S, cudaStream_t st);
 void fp64_nodes(const StepParams &P, const Fp64State &S, cudaStream_t st, int node_grid);
 void fp64_predict(const StepParams &P, const Fp64State &S, cudaStream_t st);
 void fp64_density(const StepParams &P, const Fp64State &S, const double *rho0, cudaStream_t st);
-int fp64_node_grid(int64_t nn, int sms);
+int fp64_node_grid(int64_t nn, int sms, bool tri);
 
 // Launch shape of a tunable kernel: block size and items per thread
 // (grid-stride loop; grid = ceil(n / (bs * ept))).
