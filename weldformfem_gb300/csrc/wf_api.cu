@@ -217,6 +217,9 @@ struct wf_domain {
     cudaEvent_t ready = nullptr, done = nullptr;
     int state = 0;                // 0 free, 1 queued or copied, not yet written
   } snap[2];
+  // the FP64 contact kernel's branch beside the element kernel
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_ev[2] = {nullptr, nullptr};
   cudaStream_t out_stream = nullptr;
   int snap_next = 0;
   std::vector<uint8_t> surf_ext;  // external-surface flags and areas (contact), for the VTK
@@ -388,6 +391,7 @@ void free_device(wf_domain *d) {
   drop_graphs(d);
   // nothing of the domain's may still run when its memory goes back
   if (d->stream) cudaStreamSynchronize(d->stream);
+  if (d->side) cudaStreamSynchronize(d->side);
   if (d->out_stream) cudaStreamSynchronize(d->out_stream);
   for (void *p : d->allocs) cudaFreeAsync(p, d->stream);
   d->allocs.clear();
@@ -845,6 +849,9 @@ WF_API wf_status wf_domain_destroy(wf_domain *d) {
   free_mesh_dev(d);
   if (d->stream) cudaStreamDestroy(d->stream);
   if (d->out_stream) cudaStreamDestroy(d->out_stream);
+  for (cudaEvent_t ev : d->side_ev)
+    if (ev) cudaEventDestroy(ev);
+  if (d->side) cudaStreamDestroy(d->side);
   delete d;
   return WF_OK;
 }
@@ -2032,6 +2039,15 @@ WF_API wf_status wf_init(wf_domain *d) {
       CUDA_TRY(upload(d, &ed, en));
       or_flags(fl, ed, (uint8_t)NF_CONTACT, (int64_t)en.size(), d->stream);
       CUDA_TRY(cudaGetLastError());
+      // the search's nodes: the surface and the plane's candidates, if any
+      if (!d->cand.empty()) {
+        en.insert(en.end(), d->cand.begin(), d->cand.end());
+        std::sort(en.begin(), en.end());
+        en.erase(std::unique(en.begin(), en.end()), en.end());
+        CUDA_TRY(upload(d, &ed, en));
+      }
+      P.ext_list = ed;
+      P.n_ext = (int32_t)en.size();
     }
     tri_normals_planes(d->tri_x, d->tri_el, nrm, pp);
     double *tx = nullptr, *tvd = nullptr, *tn = nullptr, *tp = nullptr, *na = nullptr,
@@ -2158,7 +2174,7 @@ WF_API wf_status wf_init(wf_domain *d) {
     CUDA_TRY(dalloc(d, &P.rnode, np));
   }
   // reaction history and step state
-  d->node_grid = (d->precision == WF_MIXED) ? mix_node_grid(nn) : fp64_node_grid(nn, P.sms, P.tri_on);
+  d->node_grid = (d->precision == WF_MIXED) ? mix_node_grid(nn) : fp64_node_grid(nn, P.sms);
   CUDA_TRY(dalloc(d, &P.partials, std::max(d->node_grid, 32)));
   d->hist_cap = 1 << 16;
   CUDA_TRY(dalloc(d, &P.hist, d->hist_cap));
@@ -2212,6 +2228,14 @@ WF_API wf_status wf_init(wf_domain *d) {
   if (fp64) {
     CUDA_TRY(dalloc(d, &S.vp, 3 * np));
     CUDA_TRY(dalloc(d, &S.ut, 3 * np));
+    if (d->tri) {
+      CUDA_TRY(dalloc(d, &S.cfn, np));
+      if (!d->side) {
+        CUDA_TRY(cudaStreamCreateWithFlags(&d->side, cudaStreamNonBlocking));
+        for (cudaEvent_t &ev : d->side_ev)
+          CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+      }
+    }
     if (d->thermal) {
       CUDA_TRY(dalloc(d, &S.qc, np));
       CUDA_TRY(dalloc(d, &S.dte, 2 * ne * d->npe));
@@ -2486,7 +2510,19 @@ void launch_step(wf_domain *d) {
   if (d->precision == WF_FP64) {
     fp64_geometry(P, d->S, d->stream, false);
     fp64_nodal(P, d->S, d->stream, 0);
+    // triangle-mesh contact beside the element kernel, joined before the node
+    // update; after it where the stabilised pressure reads the last step's
+    // contact forces
+    const bool fork = P.tri_on && !P.stab_on;
+    if (fork) {
+      cudaEventRecord(d->side_ev[0], d->stream);
+      cudaStreamWaitEvent(d->side, d->side_ev[0], 0);
+      fp64_contact(P, d->S, d->side);
+      cudaEventRecord(d->side_ev[1], d->side);
+    }
     fp64_elements(P, d->S, d->stream);
+    if (fork) cudaStreamWaitEvent(d->stream, d->side_ev[1], 0);
+    else if (P.tri_on) fp64_contact(P, d->S, d->stream);
     fp64_nodes(P, d->S, d->stream, d->node_grid);
   } else if (tiled_mode(d)) {
     mix_geometry(P, d->M, d->mvol, d->stream, d->cfg[0]);
@@ -2525,6 +2561,7 @@ void launch_step_timed(wf_domain *d, cudaEvent_t *ev) {
     cudaEventRecord(ev[2], d->stream);
     fp64_elements(P, d->S, d->stream);
     cudaEventRecord(ev[3], d->stream);
+    if (P.tri_on) fp64_contact(P, d->S, d->stream);   // timed with the node phase
     fp64_nodes(P, d->S, d->stream, d->node_grid);
   } else if (flow_mode(d)) {
     // the dataflow step is one kernel: timed as the element phase
@@ -2722,7 +2759,9 @@ WF_API wf_status wf_run(wf_domain *d, int64_t nsteps) {
     }
   }
   // the split dataflow step launches the geometry and nodal kernels first
-  const int per_step = flow_mode(d) ? (d->F.split ? 3 : 1) : (sweep_mode(d) ? 3 : 4);
+  const int per_step = flow_mode(d) ? (d->F.split ? 3 : 1)
+                       : sweep_mode(d) ? 3
+                                       : 4 + (d->precision == WF_FP64 && d->P.tri_on ? 1 : 0);
   d->launches += (per_step + (d->nspec ? 1 : 0) + (d->P.energy_on ? 1 : 0)) * left;
   // graph replays: kGraphSteps at a time, then one graph of the remainder
   if (left >= kGraphSteps) {

@@ -244,11 +244,23 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodal(StepParams P, Fp64S
     else
       return __ldg(&P.slot[b + k]) / NPE;
   };
+  // sums in list order, eight entries at a time: a chunk's loads are in
+  // flight together
   double s = 0.0, s0 = 0.0;
-  for (int32_t k = 0; k < c; k++) {
-    int32_t e = elem(k);
-    s += __ldg(&S.vol[e]);
-    if (init_mode) s0 += __ldg(&S.vol0[e]);
+  for (int32_t k0 = 0; k0 < c; k0 += 8) {
+    double g[8], g0[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const int32_t e = (k0 + j < c) ? elem(k0 + j) : -1;
+      g[j] = (e >= 0) ? __ldg(&S.vol[e]) : 0.0;
+      g0[j] = (init_mode && e >= 0) ? __ldg(&S.vol0[e]) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) s += g[j];
+    if (init_mode) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) s0 += g0[j];
+    }
   }
   if (init_mode) S.s0[n] = s0;
   else s0 = S.s0[n];
@@ -260,26 +272,29 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodal(StepParams P, Fp64S
     // of one material differ in their last bits (rho_0 vol_0 / vol_0), so
     // every entry needs its own quotient: FP64 divisions at about ten FP64
     // instructions each.
-    double mass = 0.0;
-    if constexpr (NPE == 8) {
-      // the densities' sum times voln / c; the division is exact, a
-      // multiplication, for the 1, 2, 4 or 8 elements of a box mesh's nodes
-      double rs = 0.0;
-      for (int32_t k = 0; k < c; k++) rs += __ldg(&S.rho[elem(k)]);
-      mass = rs * voln;
-      if (c & (c - 1)) mass /= c;
-      else mass *= (c == 8 ? 0.125 : c == 4 ? 0.25 : c == 2 ? 0.5 : 1.0 / c);
-    } else {
-      // the reference's sum in list order, bit for bit: x / c as q = x (1 / c)
-      // corrected by its remainder, correctly rounded when 1 / c is (Markstein's
-      // theorem; x / c for c up to 4096 checked on random x)
-      const double dc = c, rc = 1.0 / dc;
-      for (int32_t k = 0; k < c; k++) {
-        const double x = __ldg(&S.rho[elem(k)]) * voln;
-        const double q = x * rc;
-        mass += fma(fma(-q, dc, x), rc, q);
+    double mass = 0.0, rs = 0.0;
+    const double dc = c, rc = 1.0 / dc;
+    for (int32_t k0 = 0; k0 < c; k0 += 8) {
+      double g[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) g[j] = (k0 + j < c) ? __ldg(&S.rho[elem(k0 + j)]) : 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        if constexpr (NPE == 8) {
+          rs += g[j];
+        } else {
+          // the reference's sum in list order, bit for bit: x / c as q = x (1 / c)
+          // corrected by its remainder, correctly rounded when 1 / c is
+          // (Markstein's theorem; x / c for c up to 4096 checked on random x)
+          const double x = g[j] * voln;
+          const double q = x * rc;
+          mass += fma(fma(-q, dc, x), rc, q);
+        }
       }
     }
+    // hexahedra: the densities' sum times voln / c, an exact division for the
+    // 1, 2, 4 or 8 elements of a box mesh's nodes
+    if constexpr (NPE == 8) mass = c > 0 ? rs * voln * rc : 0.0;
     S.mass[n] = mass;
   }
   S.jr[n] = s / s0;
@@ -970,11 +985,30 @@ __device__ __forceinline__ bool tri_hit(const StepParams &P, int32_t j, const do
 // within 2^-20 R and every product of two lengths within 2.4e-5 R^2 of its
 // exact value; a distance is rejected above 1e-5 R, an edge test below
 // -1e-4 R^2, and a comparison that involves an infinity or NaN rejects nothing.
-// 98 triangles over 13,671 nodes: node kernel 255 -> 24 us.
+// 98 triangles over 13,671 nodes: 255 -> 85 us a step, the contact force and
+// the die's motion included.
 constexpr int kTriChunk = 64;
 struct TriFilter {
   float n[3], pp, v[3][3], r;
 };
+__device__ __forceinline__ bool tri_miss(const TriFilter &f, const float (&xf)[3], float rx) {
+  const float R = rx + f.r;
+  const float d = f.n[0] * xf[0] + f.n[1] * xf[1] + f.n[2] * xf[2] - f.pp;
+  if (d > 1e-5f * R) return true;
+  const float q0 = xf[0] - f.n[0] * d, q1 = xf[1] - f.n[1] * d, q2 = xf[2] - f.n[2] * d;
+  const float lim = -1e-4f * R * R;
+  bool out = false;
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    const int nx = l == 2 ? 0 : l + 1;
+    const float a0 = f.v[nx][0] - f.v[l][0], a1 = f.v[nx][1] - f.v[l][1],
+                a2 = f.v[nx][2] - f.v[l][2];
+    const float b0 = q0 - f.v[l][0], b1 = q1 - f.v[l][1], b2 = q2 - f.v[l][2];
+    out |= (a1 * b2 - a2 * b1) * f.n[0] + (a2 * b0 - a0 * b2) * f.n[1] +
+               (a0 * b1 - a1 * b0) * f.n[2] < lim;
+  }
+  return out;
+}
 __device__ __forceinline__ int32_t tri_search(const StepParams &P, bool act,
                                               const double (&x)[3], TriFilter *tf) {
   int32_t hit = -1;
@@ -1011,29 +1045,23 @@ __device__ __forceinline__ int32_t tri_search(const StepParams &P, bool act,
       tf[i] = f;
     }
     __syncthreads();
-    if (act && hit < 0) {
-      for (int i = 0; i < m; i++) {
-        const TriFilter &f = tf[i];
-        const float R = rx + f.r;
-        const float d = f.n[0] * xf[0] + f.n[1] * xf[1] + f.n[2] * xf[2] - f.pp;
-        if (d > 1e-5f * R) continue;
-        const float q0 = xf[0] - f.n[0] * d, q1 = xf[1] - f.n[1] * d, q2 = xf[2] - f.n[2] * d;
-        const float lim = -1e-4f * R * R;
-        bool out = false;
-#pragma unroll
-        for (int l = 0; l < 3; l++) {
-          const int nx = l == 2 ? 0 : l + 1;
-          const float a0 = f.v[nx][0] - f.v[l][0], a1 = f.v[nx][1] - f.v[l][1],
-                      a2 = f.v[nx][2] - f.v[l][2];
-          const float b0 = q0 - f.v[l][0], b1 = q1 - f.v[l][1], b2 = q2 - f.v[l][2];
-          out |= (a1 * b2 - a2 * b1) * f.n[0] + (a2 * b0 - a0 * b2) * f.n[1] +
-                     (a0 * b1 - a1 * b0) * f.n[2] < lim;
-        }
-        if (out) continue;
+    // every lane advances to its next candidate, then all lanes test theirs
+    // together: tested where each lane meets it, the FP64 test ran once for
+    // every distinct triangle of a warp's nodes (contact kernel 75 us)
+    bool live = act && hit < 0;
+    int i = 0;
+    while (__any_sync(0xffffffffu, live)) {
+      if (live) {
+        while (i < m && tri_miss(tf[i], xf, rx)) i++;
+        live = i < m;
+      }
+      __syncwarp();
+      if (live) {
         if (tri_hit(P, j0 + i, x)) {
           hit = j0 + i;
-          break;
+          live = false;
         }
+        i++;
       }
     }
   }
@@ -1049,11 +1077,8 @@ __device__ __forceinline__ int32_t tri_search(const StepParams &P, bool act,
 // (Contact.C:229, :326-329), else 0.
 __device__ __forceinline__ double tri_contact(const StepParams &P, const Fp64State &S, int64_t n,
                                               int32_t j, const double (&x)[3],
-                                              const double (&v)[3], double m, double (&cf)[3]) {
+                                              const double (&v)[3], double m) {
   const int64_t np = P.np;
-  cf[0] = S.cf[n];
-  cf[1] = S.cf[np + n];
-  cf[2] = S.cf[2 * np + n];
   double cfn = 0.0;
   if (j >= 0) {
     const double n0 = P.tri_nrm[3 * j], n1 = P.tri_nrm[3 * j + 1], n2 = P.tri_nrm[3 * j + 2];
@@ -1068,9 +1093,7 @@ __device__ __forceinline__ double tri_contact(const StepParams &P, const Fp64Sta
     const double F_damp = 0.2 * ccrit * v_reln;
     const double F_normal = P.tri_pf * k * dd;
     const double sc = -(F_normal + F_damp);
-    cf[0] = n0 * sc;
-    cf[1] = n1 * sc;
-    cf[2] = n2 * sc;
+    double cf[3] = {n0 * sc, n1 * sc, n2 * sc};
     cfn = sqrt(cf[0] * cf[0] + cf[1] * cf[1] + cf[2] * cf[2]);
     // friction
     const double vn = v[0] * n0 + v[1] * n1 + v[2] * n2;
@@ -1110,11 +1133,48 @@ __device__ __forceinline__ double tri_contact(const StepParams &P, const Fp64Sta
     if (P.tri_mid[j] != 0) cfn = 0.0;
     // heat from the die (Contact.C:309), kept after the contact ends
     if (P.thermal) S.qc[n] = P.tri_hc * P.node_area[n] * (P.tri_Tdie - S.T[n]);
+    S.cf[n] = cf[0];
+    S.cf[np + n] = cf[1];
+    S.cf[2 * np + n] = cf[2];
   }
-  S.cf[n] = cf[0];
-  S.cf[np + n] = cf[1];
-  S.cf[2 * np + n] = cf[2];
   return cfn;
+}
+
+// Triangle-mesh contact of the nodes of P.ext_list (external surface) and, by
+// the last block, the die's motion to the next step. A kernel of its own that
+// runs beside the element kernel (it needs only the nodal phase), off the
+// step's chain of kernels; the node kernel picks up the forces (S.cf) and the
+// reaction shares (S.cfn). A warp's FP64 instruction takes 64 cycles however
+// many of its lanes are active, so the force of a node in contact (250 FP64
+// instructions) and the die's motion (100) are some 12 us of latency.
+constexpr int kContactThreads = 128;
+__global__ void __launch_bounds__(kContactThreads) k_fp64_contact(StepParams P, Fp64State S) {
+  __shared__ TriFilter tf[kTriChunk];
+  __shared__ bool am_last;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool act = i < P.n_ext;
+  const double time = P.st->time;
+  const int64_t n = act ? P.ext_list[i] : 0;
+  double x[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) x[k] = act ? S.x[k * P.np + n] : 0.0;
+  const int32_t hit = tri_search(P, act, x, tf);
+  if (act) {
+    const double v[3] = {S.vp[n], S.vp[P.np + n], S.vp[2 * P.np + n]};
+    S.cfn[n] = tri_contact(P, S, n, hit, x, v, S.mass[n]);
+  }
+  // every block has read the die: the last one moves it
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    am_last = atomicAdd(&P.st->contact_blocks, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (am_last) {
+    if (threadIdx.x == 0) P.st->contact_blocks = 0u;
+    __threadfence();
+    tri_move<false>(P, time);
+  }
 }
 
 // nodes: assemblyForces (Matrices.C:42-87) as a gather over the node's
@@ -1131,27 +1191,25 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64S
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const double time = P.st->time;
   double r = 0.0;
-  int32_t hit = -1;
-  if constexpr (TRI) {
-    __shared__ TriFilter tf[kTriChunk];
-    const bool ext = n < P.nn && (P.nflag[n] & NF_CONTACT);
-    double x[3] = {0.0, 0.0, 0.0};
-    if (ext) {
-#pragma unroll
-      for (int k = 0; k < 3; k++) x[k] = S.x[k * P.np + n];
-    }
-    hit = tri_search(P, ext, x, tf);
-  }
   if (n < P.nn) {
     const int64_t np = P.np;
     const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
     // the element forces, then the hourglass forces, each summed in list
     // order; eight entries at a time, so that a chunk's loads are in flight
     // together
-    double fi[3] = {0.0, 0.0, 0.0}, fh[3] = {0.0, 0.0, 0.0};
+    double fi[3] = {0.0, 0.0, 0.0}, fh[3] = {0.0, 0.0, 0.0}, sT = 0.0;
     for (int32_t k0 = 0; k0 < c; k0 += 8) {
       int64_t base[8];
       double g[8][3];
+      if (P.thermal) {
+        // the step's element-node temperature rates, in list order as well
+        const double *cur = S.dte + (P.st->step & 1) * P.ne * NPE;
+        double q[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) q[j] = (k0 + j < c) ? cur[__ldg(&P.slot[b + k0 + j])] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) sT += q[j];
+      }
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         const int32_t sl = (k0 + j < c) ? __ldg(&P.slot[b + k0 + j]) : -1;
@@ -1203,7 +1261,11 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64S
     }
     double cf[3] = {0.0, 0.0, 0.0};
     if constexpr (TRI) {
-      if (fl & NF_CONTACT) r = tri_contact(P, S, n, hit, x, vp, mass, cf);
+      if (fl & NF_CONTACT) {   // from the contact kernel
+#pragma unroll
+        for (int k = 0; k < 3; k++) cf[k] = S.cf[k * np + n];
+        r = S.cfn[n];
+      }
     } else if (P.contact && (fl & NF_CONTACT)) {
       // rigid plane, outward normal (0, 0, -1), at z0 + vz * Time
       const double zd = P.c_z0 + P.c_vz * time;
@@ -1254,7 +1316,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64S
     const uint32_t code = P.bc[n];
     const double *bv = &P.bcval[3 * (code >> 3)];
     const double dt = P.nspec_of ? P.spec_dt[P.nspec_of[n]] : P.dt;
-    if constexpr (NPE == 8) {
+    if constexpr (NPE == 8 || TRI) {
       // one reciprocal of the mass and the step's products formed once
       const double inv_m = 1.0 / mass;
       const double gdt = P.gamma * dt, pdt = (0.5 - P.beta) * dt, bdt2 = P.beta * dt * dt,
@@ -1300,11 +1362,8 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64S
       }
     }
     if (P.thermal) {
-      // ThermalCalcs node part (Thermal.C:108-126): element-node rates of the
-      // step gathered in list order, plus the die heat over m cp of material 0
-      const double *cur = S.dte + (P.st->step & 1) * P.ne * NPE;
-      double sT = 0.0;
-      for (int32_t k = 0; k < c; k++) sT += cur[__ldg(&P.slot[b + k])];
+      // ThermalCalcs node part (Thermal.C:108-126): the gathered rates plus
+      // the die heat over m cp of material 0
       S.T[n] = S.T[n] + (sT + S.qc[n] * 1.0 / (mass * P.cp0)) * P.dt;
     }
   }
@@ -1331,7 +1390,6 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodes(StepParams P, Fp64S
       P.st->time = time + P.dt;
       P.st->done_blocks = 0u;
     }
-    if constexpr (TRI) tri_move<false>(P, time);
   }
 }
 
@@ -1345,7 +1403,7 @@ __global__ void k_fp64_predict(StepParams P, Fp64State S) {
     const double dt = P.nspec_of ? P.spec_dt[P.nspec_of[n]] : P.dt;
     // rounded as the node kernel's predictor of the next step
     const double v0 = S.v[k * P.np + n], a0 = S.pa[k * P.np + n], c = (1.0 - P.gamma) * dt;
-    double v = (P.npe == 8) ? fma(c, a0, v0) : v0 + c * a0;
+    double v = (P.npe == 8 || P.tri_on) ? fma(c, a0, v0) : v0 + c * a0;
     if (code & (1u << k)) v = bv[k];
     S.vp[k * P.np + n] = v;
   }
@@ -1374,15 +1432,8 @@ static int spread(int64_t n, int max_threads, int sms) {
   return t;
 }
 
-// Node kernel: with a triangle-mesh die its blocks stage the triangles and its
-// last block moves the die, so they keep at least 128 threads.
-static int node_threads(int64_t nn, int sms, bool tri) {
-  const int t = spread(nn, kNodeThreads, sms);
-  return tri ? std::max(t, 128) : t;
-}
-
-int fp64_node_grid(int64_t nn, int sms, bool tri) {
-  return (int)grid_for(nn, node_threads(nn, sms, tri));
+int fp64_node_grid(int64_t nn, int sms) {
+  return (int)grid_for(nn, spread(nn, kNodeThreads, sms));
 }
 
 void fp64_geometry(const StepParams &P, const Fp64State &S, cudaStream_t st, bool store_detj) {
@@ -1417,8 +1468,8 @@ void fp64_elements(const StepParams &P, const Fp64State &S, cudaStream_t st) {
 }
 
 void fp64_nodes(const StepParams &P, const Fp64State &S, cudaStream_t st, int node_grid) {
-  // node_grid = fp64_node_grid(P.nn, P.sms, P.tri_on): blocks of that size
-  const int t = node_threads(P.nn, P.sms, P.tri_on);
+  // node_grid = fp64_node_grid(P.nn, P.sms): blocks of the spread size
+  const int t = spread(P.nn, kNodeThreads, P.sms);
   if (P.npe == 8 && P.tri_on)
     k_fp64_nodes<8, true><<<node_grid, t, 0, st>>>(P, S);
   else if (P.npe == 8)
@@ -1427,6 +1478,12 @@ void fp64_nodes(const StepParams &P, const Fp64State &S, cudaStream_t st, int no
     k_fp64_nodes<4, true><<<node_grid, t, 0, st>>>(P, S);
   else
     k_fp64_nodes<4, false><<<node_grid, t, 0, st>>>(P, S);
+}
+
+void fp64_contact(const StepParams &P, const Fp64State &S, cudaStream_t st) {
+  // at least one block: it moves the die
+  const unsigned g = std::max(1u, grid_for(P.n_ext, kContactThreads));
+  k_fp64_contact<<<g, kContactThreads, 0, st>>>(P, S);
 }
 
 void fp64_predict(const StepParams &P, const Fp64State &S, cudaStream_t st) {

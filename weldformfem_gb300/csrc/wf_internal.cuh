@@ -90,7 +90,7 @@ struct StepState {
   long long first_bad_node;  // smallest node id whose force was cleared (LLONG_MAX: none)
   double eint;               // accumulated internal energy (energy history)
   unsigned int energy_blocks;  // last-block-done counter of the energy kernel
-  unsigned int pad;
+  unsigned int contact_blocks;  // last-block-done counter of the FP64 contact kernel
 };
 
 // Node flags (uint8 per node).
@@ -166,6 +166,8 @@ struct StepParams {
   const int32_t *tri_mid;   // [tri_ne] rigid-body index; body 0 feeds the reaction
   const double *node_area;  // [nn] external-surface area share of each node
   const double *nodlen;     // [nn] mean element length at each node
+  const int32_t *ext_list;  // [n_ext] the nodes the search covers, ascending
+  int32_t n_ext;
   double tri_mu_s, tri_mu_d, tri_pf, tri_E0, end_t;
   // FP32 copies for the mixed-precision contact, relative to tri_ref
   float *tri_xf;            // [3 tri_nn]
@@ -206,6 +208,7 @@ struct Fp64State {
   // buffers [2][ne][npe] chosen by step parity (the thermal expansion of a
   // step reads the previous step's)
   double *T, *qc, *dte;
+  double *cfn;                                   // [np] reaction share (triangle-mesh contact)
 };
 
 // Mixed state. Positions are compensated float pairs (hi + lo, ~48-bit
@@ -336,7 +339,10 @@ void fp64_elements(const StepParams &P, const Fp64State &S, cudaStream_t st);
 void fp64_nodes(const StepParams &P, const Fp64State &S, cudaStream_t st, int node_grid);
 void fp64_predict(const StepParams &P, const Fp64State &S, cudaStream_t st);
 void fp64_density(const StepParams &P, const Fp64State &S, const double *rho0, cudaStream_t st);
-int fp64_node_grid(int64_t nn, int sms, bool tri);
+int fp64_node_grid(int64_t nn, int sms);
+// Triangle-mesh contact forces (S.cf, S.cfn) and the die's motion, between the
+// nodal phase and the node update of a step.
+void fp64_contact(const StepParams &P, const Fp64State &S, cudaStream_t st);
 
 // Launch shape of a tunable kernel: block size and items per thread
 // (grid-stride loop; grid = ceil(n / (bs * ept))).

@@ -16,7 +16,7 @@ template <bool F32>
 __device__ void tri_move(const StepParams &P, double time) {
   const double rf = 1.0e-2;
   double f = 1.0;
-  if (time < rf * P.end_t) f = pow(time / (rf * P.end_t), 0.5);
+  if (time < rf * P.end_t) f = sqrt(time / (rf * P.end_t));
   for (int32_t i = threadIdx.x; i < 3 * P.tri_nn; i += blockDim.x) {
     const double vk = f * P.tri_v[i];
     P.tri_x[i] = P.tri_x[i] + vk * P.dt;
