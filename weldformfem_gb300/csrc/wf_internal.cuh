@@ -393,6 +393,20 @@ int mix_cluster_fits(const StepParams &P, const MixState &M, float *vol, int blo
 // part: [nsteps][blocks] staging for the reaction's block partials.
 cudaError_t mix_cluster_run(const StepParams &P, const MixState &M, float *vol, double *part,
                             int64_t nsteps, int blocks, int bs, cudaStream_t st);
+// The cluster run with its state in shared memory. Per block, at most: nn nodes,
+// ne elements, nc copies of nodes its elements touch, nt copies of its nodes in
+// all blocks; mc entries of a node's list; words of a bitmap of the mesh's nodes;
+// chunk steps a launch.
+constexpr int kClusterSmemChunk = 1024;
+struct ClusterShape {
+  int32_t nn = 0, ne = 0, mc = 0, nc = 0, nt = 0, words = 0, chunk = 0;
+};
+// Whether it runs this domain (fills C from the blocks' largest counts).
+bool mix_cluster_smem_fits(const StepParams &P, const MixState &M, float *vol, int blocks, int bs,
+                           int64_t max_list, int64_t max_copies, int64_t max_targets,
+                           ClusterShape &C);
+cudaError_t mix_cluster_smem_run(const StepParams &P, const MixState &M, float *vol, int64_t nsteps,
+                                 int blocks, int bs, const ClusterShape &C, cudaStream_t st);
 // The mixed state's displacements (or positions) as AoS [nn][3] doubles, as
 // the export forms them, without exporting the other fields.
 void mix_node_aos(const StepParams &P, const MixState &M, bool displacement, double *out,
