@@ -267,6 +267,11 @@ struct wf_domain {
   double *cl_part = nullptr;      // [kClusterChunk][cl_blocks] reaction partials
   bool cl_smem = false;           // the cluster run keeps its state in shared memory
   ClusterShape cl_shape;
+  // tile runs (one cooperative launch per chunk of steps)
+  bool tile_run = false;
+  TileRunShape tr_shape;
+  double *tr_part = nullptr;      // [kTileRunChunk][tiles] reaction partials
+  unsigned *tr_bar = nullptr;     // the barrier's counter
   double *edge_min = nullptr;     // the shortest edge (wf_min_edge_length's device result)
   // batched ensemble
   int32_t nspec = 0;
@@ -1752,6 +1757,15 @@ void set_parity(wf_domain *d, int p) {
 }
 }  // namespace
 
+namespace {
+// Whether the automatic mode runs the per-phase arithmetic as tile runs
+// (reported as mode 1, whose arithmetic it is).
+bool tile_run_mode(const wf_domain *d) {
+  return d->precision == WF_MIXED && d->step_mode == 0 && d->tile_run && !d->P.energy_on &&
+         !d->phase_timing && !cluster_mode(d) && !tiled_mode(d) && !flow_mode(d) && !sweep_mode(d);
+}
+}  // namespace
+
 WF_API wf_status wf_set_step_mode(wf_domain *d, int32_t mode) {
   if (!d || mode < 0 || mode > 5) return WF_ERR_ARG;
   if (mode != d->step_mode) drop_graphs(d);   // the graphs hold the other kernels
@@ -2532,6 +2546,12 @@ WF_API wf_status wf_init(wf_domain *d) {
       }
     }
   }
+  d->tile_run = !fp64 && !d->nspec && !d->energy && mix_tile_run_shape(P, d->tr_shape);
+  if (d->tile_run) {
+    const TileRunShape &C = d->tr_shape;
+    CUDA_TRY(dalloc(d, &d->tr_part, (size_t)kTileRunChunk * C.ta * C.tb * C.tc));
+    CUDA_TRY(dalloc(d, &d->tr_bar, 1));
+  }
   CUDA_TRY(cudaStreamSynchronize(d->stream));
   if (d->init_stage) CUDA_TRY(cudaFreeAsync(d->init_stage, d->stream));
   d->init_stage = nullptr;
@@ -2815,6 +2835,15 @@ WF_API wf_status wf_run(wf_domain *d, int64_t nsteps) {
       left -= chunk;
     }
   }
+  if (tile_run_mode(d)) {
+    while (left > 0) {
+      const int64_t chunk = std::min<int64_t>(left, kTileRunChunk);
+      CUDA_TRY(mix_tile_run(d->P, d->M, d->mvol, d->tr_part, d->tr_bar, chunk, d->tr_shape,
+                            d->stream));
+      d->launches += 1;
+      left -= chunk;
+    }
+  }
   // the split dataflow step launches the geometry and nodal kernels first
   const int per_step = flow_mode(d) ? (d->F.split ? 3 : 1)
                        : sweep_mode(d) ? 3
@@ -2855,7 +2884,8 @@ WF_API wf_status wf_prepare_run(wf_domain *d, int64_t nsteps) {
   if (!d || nsteps < 0) return WF_ERR_ARG;
   if (!d->initialized) return fail(d, WF_ERR_STATE, "wf_init not called");
   if (!(d->dt > 0.0) && !d->nspec) return fail(d, WF_ERR_STATE, "time step not set (SetDT)");
-  if (d->phase_timing || cluster_mode(d)) return WF_OK;   // these runs replay no graph
+  // these runs replay no graph
+  if (d->phase_timing || cluster_mode(d) || tile_run_mode(d)) return WF_OK;
   CUDA_TRY(cudaSetDevice(d->device));
   {
     const wf_status gs = grow_history(d, d->host_step + nsteps);
@@ -3134,8 +3164,8 @@ WF_API wf_status wf_sync(wf_domain *d) {
       d->st_host->status &= ~2u;
       CUDA_TRY(cudaMemcpy(&d->P.st->status, &d->st_host->status, sizeof(unsigned),
                           cudaMemcpyHostToDevice));
-      return fail(d, WF_ERR_TIMEOUT, "a dependency wait of the dataflow step ran out, in the "
-                                     "steps up to step %lld", (long long)st.step);
+      return fail(d, WF_ERR_TIMEOUT, "a wait inside a step's kernel ran out, in the steps up "
+                                     "to step %lld", (long long)st.step);
     }
     if (st.status & 1u) {
       d->st_host->status = 0u;

@@ -407,6 +407,17 @@ bool mix_cluster_smem_fits(const StepParams &P, const MixState &M, float *vol, i
                            ClusterShape &C);
 cudaError_t mix_cluster_smem_run(const StepParams &P, const MixState &M, float *vol, int64_t nsteps,
                                  int blocks, int bs, const ClusterShape &C, cudaStream_t st);
+// The tile run of a box mesh: ta x tb x tc tiles, and the largest counts of a
+// tile: own elements e0, its corner nodes n1, the elements around it e1 and
+// their nodes n2; at most chunk steps a launch.
+constexpr int kTileRunChunk = 256;
+struct TileRunShape {
+  int32_t ta = 0, tb = 0, tc = 0, e0 = 0, n1 = 0, e1 = 0, n2 = 0, chunk = 0, thermal = 0;
+};
+bool mix_tile_run_shape(const StepParams &P, TileRunShape &C);   // false: not run so
+// part: [chunk][tiles] reaction partials; bar: the barrier's counter.
+cudaError_t mix_tile_run(const StepParams &P, const MixState &M, float *vol, double *part,
+                         unsigned *bar, int64_t nsteps, const TileRunShape &C, cudaStream_t st);
 // The mixed state's displacements (or positions) as AoS [nn][3] doubles, as
 // the export forms them, without exporting the other fields.
 void mix_node_aos(const StepParams &P, const MixState &M, bool displacement, double *out,

@@ -58,14 +58,19 @@ __device__ __forceinline__ float pair_rel(float2 a, float2 b) {
   return __fadd_rn(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y));
 }
 
-// Loads of data that other threads write during the run: through the
-// read-only path (__ldg) in the per-phase kernels, where it is constant for
-// the launch, and through L2 (__ldcg) in the persistent cluster kernel, whose
-// phases share one launch.
-template <bool CG, typename T>
+// Loads of data that other threads write during the run. kLdRo: the read-only
+// path (__ldg), in the per-phase kernels, where the data is constant for the
+// launch. kLdL2: through L2 (__ldcg), in the cluster run and the dataflow
+// step, whose phases share one launch. kLdL1: plain loads, in the grid run,
+// whose barrier between phases is an acquire (it drops the SM's L1 lines), so
+// that a phase still shares its gathers in L1.
+enum : int { kLdRo = 0, kLdL2 = 1, kLdL1 = 2 };
+template <int LD, typename T>
 __device__ __forceinline__ T ldx(const T *p) {
-  if constexpr (CG)
+  if constexpr (LD == kLdL2)
     return __ldcg(p);
+  else if constexpr (LD == kLdL1)
+    return *p;
   else
     return __ldg(p);
 }
@@ -94,7 +99,7 @@ __device__ __forceinline__ float weightf() {
   return NPE == 8 ? 8.0f : 1.0f / 6.0f;
 }
 
-template <int NPE, bool CG, bool BOX = false>
+template <int NPE, int LD, bool BOX = false>
 __device__ __forceinline__ void rel_coords(const StepParams &P, const MixState &M, int64_t e,
                                            float (&r)[NPE][3], int32_t (&nid)[NPE]) {
   if constexpr (BOX && NPE == 8) {
@@ -105,13 +110,13 @@ __device__ __forceinline__ void rel_coords(const StepParams &P, const MixState &
   }
   float2 o[3];
 #pragma unroll
-  for (int k = 0; k < 3; k++) o[k] = ldx<CG>(&M.xh[k * P.np + nid[0]]);
+  for (int k = 0; k < 3; k++) o[k] = ldx<LD>(&M.xh[k * P.np + nid[0]]);
 #pragma unroll
   for (int k = 0; k < 3; k++) r[0][k] = 0.0f;
 #pragma unroll
   for (int a = 1; a < NPE; a++)
 #pragma unroll
-    for (int k = 0; k < 3; k++) r[a][k] = pair_rel(ldx<CG>(&M.xh[k * P.np + nid[a]]), o[k]);
+    for (int k = 0; k < 3; k++) r[a][k] = pair_rel(ldx<LD>(&M.xh[k * P.np + nid[a]]), o[k]);
 }
 
 template <int NPE>
@@ -176,12 +181,12 @@ __device__ __forceinline__ void shape_derivs_f(const float J[3][3], float dH[3][
 }
 
 // ---------------------------------------------------------------------------
-template <int NPE, bool CG, bool BOX = false>
+template <int NPE, int LD, bool BOX = false>
 __device__ __forceinline__ void geometry_one(const StepParams &P, const MixState &M, float *vol,
                                              int64_t e) {
   float r[NPE][3];
   int32_t nid[NPE];
-  rel_coords<NPE, CG, BOX>(P, M, e, r, nid);
+  rel_coords<NPE, LD, BOX>(P, M, e, r, nid);
   float J[3][3];
   jacobian_f<NPE>(r, J);
   vol[e] = det3f(J) * weightf<NPE>();
@@ -199,15 +204,15 @@ __global__ void __launch_bounds__(BS) k_mix_geometry(StepParams P, MixState M, f
   for (; e + stride < P.ne; e += 2 * stride) {
     float r0[NPE][3], r1[NPE][3];
     int32_t n0[NPE], n1[NPE];
-    rel_coords<NPE, false, BOX>(P, M, e, r0, n0);
-    rel_coords<NPE, false, BOX>(P, M, e + stride, r1, n1);
+    rel_coords<NPE, kLdRo, BOX>(P, M, e, r0, n0);
+    rel_coords<NPE, kLdRo, BOX>(P, M, e + stride, r1, n1);
     float J0[3][3], J1[3][3];
     jacobian_f<NPE>(r0, J0);
     jacobian_f<NPE>(r1, J1);
     vol[e] = det3f(J0) * weightf<NPE>();
     vol[e + stride] = det3f(J1) * weightf<NPE>();
   }
-  if (e < P.ne) geometry_one<NPE, false, BOX>(P, M, vol, e);
+  if (e < P.ne) geometry_one<NPE, kLdRo, BOX>(P, M, vol, e);
 }
 
 // Rigid triangle-mesh contact of one external node in FP32 (the FP64 step's
@@ -218,7 +223,7 @@ __global__ void __launch_bounds__(BS) k_mix_geometry(StepParams P, MixState M, f
 // friction from the accumulated slip. A node out of contact keeps its last
 // contact force. The node's reaction share (normal-force magnitude, rigid
 // body 0 only) goes to M.cfn.
-template <bool CG>
+template <int LD>
 __device__ __forceinline__ void tri_contact_mixed(const StepParams &P, const MixState &M,
                                                   int64_t n, float mass) {
   const int64_t np = P.np;
@@ -231,19 +236,19 @@ __device__ __forceinline__ void tri_contact_mixed(const StepParams &P, const Mix
   }
   float cfn = 0.f;
   for (int32_t j = 0; j < P.tri_ne; j++) {
-    const float n0 = ldx<CG>(&P.tri_nf[3 * j]), n1 = ldx<CG>(&P.tri_nf[3 * j + 1]),
-                n2 = ldx<CG>(&P.tri_nf[3 * j + 2]);
-    const float dd = (n0 * x[0] + n1 * x[1] + n2 * x[2]) - ldx<CG>(&P.tri_ppf[j]);
+    const float n0 = ldx<LD>(&P.tri_nf[3 * j]), n1 = ldx<LD>(&P.tri_nf[3 * j + 1]),
+                n2 = ldx<LD>(&P.tri_nf[3 * j + 2]);
+    const float dd = (n0 * x[0] + n1 * x[1] + n2 * x[2]) - ldx<LD>(&P.tri_ppf[j]);
     if (!(dd < 0.f)) continue;
     const float Q[3] = {x[0] - n0 * dd, x[1] - n1 * dd, x[2] - n2 * dd};
     bool inside = true;
     for (int l = 0; l < 3 && inside; l++) {
       const int nx = l + 1 > 2 ? 0 : l + 1;
       const int32_t ia = 3 * __ldg(&P.tri_el[3 * j + l]), ib = 3 * __ldg(&P.tri_el[3 * j + nx]);
-      const float a0 = ldx<CG>(&P.tri_xf[ia]), a1 = ldx<CG>(&P.tri_xf[ia + 1]),
-                  a2 = ldx<CG>(&P.tri_xf[ia + 2]);
-      const float e1[3] = {ldx<CG>(&P.tri_xf[ib]) - a0, ldx<CG>(&P.tri_xf[ib + 1]) - a1,
-                           ldx<CG>(&P.tri_xf[ib + 2]) - a2};
+      const float a0 = ldx<LD>(&P.tri_xf[ia]), a1 = ldx<LD>(&P.tri_xf[ia + 1]),
+                  a2 = ldx<LD>(&P.tri_xf[ia + 2]);
+      const float e1[3] = {ldx<LD>(&P.tri_xf[ib]) - a0, ldx<LD>(&P.tri_xf[ib + 1]) - a1,
+                           ldx<LD>(&P.tri_xf[ib + 2]) - a2};
       const float e2[3] = {Q[0] - a0, Q[1] - a1, Q[2] - a2};
       const float crit = (e1[1] * e2[2] - e1[2] * e2[1]) * n0 +
                          (e1[2] * e2[0] - e1[0] * e2[2]) * n1 +
@@ -302,7 +307,7 @@ __device__ __forceinline__ void tri_contact_mixed(const StepParams &P, const Mix
 // zd: the rigid plane's height at the step's time as a (hi, lo) float pair,
 // formed once per thread by the caller (die_height), so that the gap of a
 // contact node takes no FP64 instruction.
-template <int NPE, bool CG, bool BOX = false>
+template <int NPE, int LD, bool BOX = false>
 __device__ __forceinline__ void nodal_gather(const StepParams &P, const MixState &M,
                                              const float *vol, int64_t n, float &s, float2 &nc) {
   s = 0.0f;
@@ -313,7 +318,7 @@ __device__ __forceinline__ void nodal_gather(const StepParams &P, const MixState
     nc = __ldg(&M.nc[n]);
     float g[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) g[j] = (el[j] >= 0) ? ldx<CG>(&vol[el[j]]) : 0.0f;
+    for (int j = 0; j < 8; j++) g[j] = (el[j] >= 0) ? ldx<LD>(&vol[el[j]]) : 0.0f;
 #pragma unroll
     for (int j = 0; j < 8; j++)
       if (el[j] >= 0) s += g[j];
@@ -326,7 +331,7 @@ __device__ __forceinline__ void nodal_gather(const StepParams &P, const MixState
       for (int j = 0; j < 8; j++) sl[j] = (k0 + j < c) ? __ldg(&P.slot[b + k0 + j]) : -1;
       float g[8];
 #pragma unroll
-      for (int j = 0; j < 8; j++) g[j] = (sl[j] >= 0) ? ldx<CG>(&vol[sl[j] / NPE]) : 0.0f;
+      for (int j = 0; j < 8; j++) g[j] = (sl[j] >= 0) ? ldx<LD>(&vol[sl[j] / NPE]) : 0.0f;
 #pragma unroll
       for (int j = 0; j < 8; j++) s += g[j];
     }
@@ -369,7 +374,7 @@ __device__ __forceinline__ bool plane_contact(const StepParams &P, float mass, f
 
 // The rest of a node's nodal phase from its volume sum s and constants nc:
 // J ratio, lumped mass, contact force.
-template <int NPE, bool CG>
+template <int NPE, int LD>
 __device__ __forceinline__ void nodal_rest(const StepParams &P, const MixState &M, int64_t n,
                                            float s, float2 nc, float2 zd) {
   M.jr[n] = s * nc.x;
@@ -381,7 +386,7 @@ __device__ __forceinline__ void nodal_rest(const StepParams &P, const MixState &
     mass = M.mass[n];
   }
   if (P.tri_on) {
-    if (P.nflag[n] & NF_CONTACT) tri_contact_mixed<CG>(P, M, n, mass);
+    if (P.nflag[n] & NF_CONTACT) tri_contact_mixed<LD>(P, M, n, mass);
   } else if (P.contact && (P.nflag[n] & NF_CONTACT)) {
     const int64_t np = P.np;
     const float vp[3] = {M.vp[n], M.vp[np + n], M.vp[2 * np + n]};
@@ -396,13 +401,13 @@ __device__ __forceinline__ void nodal_rest(const StepParams &P, const MixState &
   }
 }
 
-template <int NPE, bool CG, bool BOX = false>
+template <int NPE, int LD, bool BOX = false>
 __device__ __forceinline__ void nodal_one(const StepParams &P, const MixState &M,
                                           const float *vol, int64_t n, float2 zd) {
   float s;
   float2 nc;
-  nodal_gather<NPE, CG, BOX>(P, M, vol, n, s, nc);
-  nodal_rest<NPE, CG>(P, M, n, s, nc, zd);
+  nodal_gather<NPE, LD, BOX>(P, M, vol, n, s, nc);
+  nodal_rest<NPE, LD>(P, M, n, s, nc, zd);
 }
 
 // Two nodes per iteration when the grid strides: both nodes' volume gathers
@@ -420,12 +425,12 @@ __global__ void __launch_bounds__(BS) k_mix_nodal(StepParams P, MixState M, cons
   for (; n + stride < P.nn; n += 2 * stride) {
     float s0, s1;
     float2 c0, c1;
-    nodal_gather<NPE, false, BOX>(P, M, vol, n, s0, c0);
-    nodal_gather<NPE, false, BOX>(P, M, vol, n + stride, s1, c1);
-    nodal_rest<NPE, false>(P, M, n, s0, c0, zd);
-    nodal_rest<NPE, false>(P, M, n + stride, s1, c1, zd);
+    nodal_gather<NPE, kLdRo, BOX>(P, M, vol, n, s0, c0);
+    nodal_gather<NPE, kLdRo, BOX>(P, M, vol, n + stride, s1, c1);
+    nodal_rest<NPE, kLdRo>(P, M, n, s0, c0, zd);
+    nodal_rest<NPE, kLdRo>(P, M, n + stride, s1, c1, zd);
   }
-  if (n < P.nn) nodal_one<NPE, false, BOX>(P, M, vol, n, zd);
+  if (n < P.nn) nodal_one<NPE, kLdRo, BOX>(P, M, vol, n, zd);
 }
 
 // Jaumann rate + radial return, shared by both element types. The
@@ -639,16 +644,15 @@ __device__ __forceinline__ void walsh8_synth(const float (&o)[8], float (&v)[8])
 // the strain rate's diagonal loses exp_T times the mean of the previous step's
 // element-node rates read at the element's node ids, and a Johnson-Cook
 // element's temperature factor uses the mean of its node temperatures.
-template <int NPE, bool CG>
+template <int NPE, class Nodes>
 __device__ __forceinline__ void thermal_pre(const StepParams &P, const MixState &M,
-                                            const MatF &m, const int32_t (&nid)[NPE],
-                                            long long step, float (&sr)[6], float &jTh) {
-  const float *prev = M.dte + ((step + 1) & 1) * P.ne * NPE;
+                                            const MatF &m, const Nodes &nd, long long step,
+                                            float (&sr)[6], float &jTh) {
   float g = 0.f, ts = 0.f;
 #pragma unroll
   for (int a = 0; a < NPE; a++) {
-    g += ldx<CG>(&prev[nid[a]]);
-    ts += ldx<CG>(&M.T[nid[a]]).x;
+    g += nd.rate(P, M, a, step);
+    ts += nd.T(M, a);
   }
   const float c = m.exp_T * (g * (1.0f / NPE));
   sr[0] -= c;
@@ -661,21 +665,36 @@ __device__ __forceinline__ void thermal_pre(const StepParams &P, const MixState 
 }
 
 // After the forces: the element-node temperature rates -(K T)_a / m_a plus the
-// plastic heat 0.9 q vol / n / (m_a cp_T), written to the step's buffer.
-// KT holds (K T)_a / kf; qvol = q vol.
-template <int NPE, bool CG>
+// plastic heat 0.9 q vol / n / (m_a cp_T), written to the step's buffer, one
+// division a node. KT holds (K T)_a / kf; qvol = q vol.
+template <int NPE, class Nodes>
 __device__ __forceinline__ void thermal_rates(const StepParams &P, const MixState &M,
-                                              const MatF &m, int64_t e,
-                                              const int32_t (&nid)[NPE], long long step,
-                                              const float (&KT)[NPE], float kf, float qvol) {
+                                              const MatF &m, int64_t e, const Nodes &nd,
+                                              long long step, const float (&KT)[NPE], float kf,
+                                              float qvol) {
   float *cur = M.dte + (step & 1) * P.ne * NPE + e * NPE;
-  const float ppn = 0.9f * qvol * (1.0f / NPE);
+  const float heat = 0.9f * qvol * (1.0f / NPE) / m.cp_T;
 #pragma unroll
-  for (int a = 0; a < NPE; a++) {
-    const float mi = ldx<CG>(&M.mass[nid[a]]);
-    cur[a] = -(kf * KT[a]) / mi + ppn / (mi * m.cp_T);
-  }
+  for (int a = 0; a < NPE; a++) cur[a] = (heat - kf * KT[a]) / nd.mass(M, a);
 }
+
+// The thermal step's node values from the node arrays, by node id: temperature,
+// lumped mass, and the previous step's element-node temperature rate at the
+// node's id (as the reference indexes that array).
+template <int NPE, int LD>
+struct ThermalNodes {
+  int32_t nid[NPE];
+  __device__ __forceinline__ float T(const MixState &M, int a) const {
+    return ldx<LD>(&M.T[nid[a]]).x;
+  }
+  __device__ __forceinline__ float mass(const MixState &M, int a) const {
+    return ldx<LD>(&M.mass[nid[a]]);
+  }
+  __device__ __forceinline__ float rate(const StepParams &P, const MixState &M, int a,
+                                        long long step) const {
+    return ldx<LD>(&M.dte[((step + 1) & 1) * P.ne * NPE + nid[a]]);
+  }
+};
 
 // Where an element's node values come from. GlobalNodes: the node arrays in
 // HBM through the element's connectivity (per-phase kernels, cluster run);
@@ -685,12 +704,12 @@ __device__ __forceinline__ void thermal_rates(const StepParams &P, const MixStat
 // CGX: positions and predicted velocities through L2 as well (the cluster
 // run); the dataflow step reads them through L1 (no tile of its launch writes
 // them before every read of them is done) and only the J ratios through L2.
-template <bool CG, bool BOX = false, bool CGX = CG>
-struct GlobalNodes {
+template <int LD, bool BOX = false, int LDX = LD>
+struct GlobalNodes : ThermalNodes<8, LD> {
+  using ThermalNodes<8, LD>::nid;
   const float2 *xh;
   const float *vp, *jr;
   int64_t np;
-  int32_t nid[8];
   __device__ __forceinline__ GlobalNodes(const StepParams &P, const MixState &M, int64_t e)
       : xh(M.xh), vp(M.vp), jr(M.jr), np(P.np) {
     if constexpr (BOX) {
@@ -700,9 +719,9 @@ struct GlobalNodes {
       for (int a = 0; a < 8; a++) nid[a] = __ldg(&P.elnod[a * P.ne + e]);
     }
   }
-  __device__ __forceinline__ float2 x(int a, int k) const { return ldx<CGX>(&xh[k * np + nid[a]]); }
-  __device__ __forceinline__ float v(int a, int k) const { return ldx<CGX>(&vp[k * np + nid[a]]); }
-  __device__ __forceinline__ float j(int a) const { return ldx<CG>(&jr[nid[a]]); }
+  __device__ __forceinline__ float2 x(int a, int k) const { return ldx<LDX>(&xh[k * np + nid[a]]); }
+  __device__ __forceinline__ float v(int a, int k) const { return ldx<LDX>(&vp[k * np + nid[a]]); }
+  __device__ __forceinline__ float j(int a) const { return ldx<LD>(&jr[nid[a]]); }
 };
 
 // Artificial viscosity (calcArtificialViscosity, Mechanical.C:1948-1977) of
@@ -828,7 +847,7 @@ __device__ __forceinline__ void element_hex_core(const StepParams &P, const MixS
   const float w12 = 0.5f * (L[2][1] - L[1][2]);
   const float w02 = 0.5f * (L[2][0] - L[0][2]);
   float jTh = m.jc_Th;
-  if constexpr (TH) thermal_pre<8, !EARLY_JR>(P, M, m, nd.nid, step, sr, jTh);
+  if constexpr (TH) thermal_pre<8>(P, M, m, nd, step, sr, jTh);
   float J_bar = J_avg * 0.125f;
   if (J_bar < 0.0f) J_bar = 0.2f;
   const float p = -m.K * (J_bar - 1.0f);
@@ -854,10 +873,9 @@ __device__ __forceinline__ void element_hex_core(const StepParams &P, const MixS
   if constexpr (TH) {
     // conduction in the same Walsh form: grad T detJ = A (Walsh sums of T) / 8,
     // (K T)_a = k_T / detJ * synthesis of A^T grad T detJ (w = 8 cancels 1/8)
-    constexpr bool CG = !EARLY_JR;
     float tv[8], oT[8], KT[8];
 #pragma unroll
-    for (int a = 0; a < 8; a++) tv[a] = ldx<CG>(&M.T[nd.nid[a]]).x;
+    for (int a = 0; a < 8; a++) tv[a] = nd.T(M, a);
     walsh8(tv, oT);
     float BT[3];
 #pragma unroll
@@ -867,22 +885,22 @@ __device__ __forceinline__ void element_hex_core(const StepParams &P, const MixS
 #pragma unroll
     for (int mm = 0; mm < 3; mm++) o[1 + mm] = A[0][mm] * BT[0] + A[1][mm] * BT[1] + A[2][mm] * BT[2];
     walsh8_synth(o, KT);
-    thermal_rates<8, CG>(P, M, m, e, nd.nid, step, KT, m.k_T / detJ, qpl * vol);
+    thermal_rates<8>(P, M, m, e, nd, step, KT, m.k_T / detJ, qpl * vol);
   }
 }
 
 // Per-phase kernels and the cluster run: node values from HBM, forces to HBM.
-template <int LAW, bool CG, bool TH, bool BOX = false>
+template <int LAW, int LD, bool TH, bool BOX = false>
 __device__ __forceinline__ void element_hex(const StepParams &P, const MixState &M, int64_t e,
                                             float *stash, int stride, long long step) {
-  const GlobalNodes<CG, BOX> nd(P, M, e);
+  const GlobalNodes<LD, BOX> nd(P, M, e);
   ForcesToHbm out{M.fe, P.ne, e};
-  element_hex_core<LAW, !CG, TH>(P, M, e, nd, stash, stride, step, out,
-                                 StateInPlace{});
+  element_hex_core<LAW, LD != kLdL2, TH>(P, M, e, nd, stash, stride, step, out,
+                                        StateInPlace{});
 }
 
 // Tetrahedron: per-node shape derivatives (Domain_d.C:1866-1887).
-template <int LAW, bool CG, bool TH>
+template <int LAW, int LD, bool TH>
 __device__ __forceinline__ void element_tet(const StepParams &P, const MixState &M, int64_t e,
                                             long long step) {
   const int64_t ne = P.ne;
@@ -892,15 +910,15 @@ __device__ __forceinline__ void element_tet(const StepParams &P, const MixState 
   float vpn[4][3], jrn[4];
   {
     float r[4][3];
-    rel_coords<4, CG>(P, M, e, r, nid);
+    rel_coords<4, LD>(P, M, e, r, nid);
     // the nodes' predicted velocities and volume ratios, gathered before the
     // Jacobian arithmetic so that their loads are in flight during it
 #pragma unroll
     for (int a = 0; a < 4; a++) {
-      vpn[a][0] = ldx<CG>(&M.vp[nid[a]]);
-      vpn[a][1] = ldx<CG>(&M.vp[P.np + nid[a]]);
-      vpn[a][2] = ldx<CG>(&M.vp[2 * P.np + nid[a]]);
-      jrn[a] = ldx<CG>(&M.jr[nid[a]]);
+      vpn[a][0] = ldx<LD>(&M.vp[nid[a]]);
+      vpn[a][1] = ldx<LD>(&M.vp[P.np + nid[a]]);
+      vpn[a][2] = ldx<LD>(&M.vp[2 * P.np + nid[a]]);
+      jrn[a] = ldx<LD>(&M.jr[nid[a]]);
     }
     float J[3][3];
     jacobian_f<4>(r, J);
@@ -931,7 +949,10 @@ __device__ __forceinline__ void element_tet(const StepParams &P, const MixState 
   float sr[6] = {s00 * f, s11 * f, s22 * f, s01 * fh, s12 * fh, s02 * fh};
   w01 *= fh; w12 *= fh; w02 *= fh;
   float jTh = m.jc_Th;
-  if constexpr (TH) thermal_pre<4, CG>(P, M, m, nid, step, sr, jTh);
+  ThermalNodes<4, LD> tn;
+#pragma unroll
+  for (int a = 0; a < 4; a++) tn.nid[a] = nid[a];
+  if constexpr (TH) thermal_pre<4>(P, M, m, tn, step, sr, jTh);
   J_avg *= 0.25f;
   float J_bar = J_avg;
   if (J_bar < 0.0f) J_bar = 0.2f;
@@ -955,10 +976,10 @@ __device__ __forceinline__ void element_tet(const StepParams &P, const MixState 
     // temperatures relative to node 0's (K's rows sum to zero): no FP32
     // cancellation between the absolute temperatures
     float Te[4], KT[4];
-    const float T0n = ldx<CG>(&M.T[nid[0]]).x;
+    const float T0n = tn.T(M, 0);
     Te[0] = 0.f;
 #pragma unroll
-    for (int a = 1; a < 4; a++) Te[a] = ldx<CG>(&M.T[nid[a]]).x - T0n;
+    for (int a = 1; a < 4; a++) Te[a] = tn.T(M, a) - T0n;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       float t = 0.f;
@@ -967,17 +988,17 @@ __device__ __forceinline__ void element_tet(const StepParams &P, const MixState 
         t += (dH[0][i] * dH[0][k] + dH[1][i] * dH[1][k] + dH[2][i] * dH[2][k]) * Te[k];
       KT[i] = t;
     }
-    thermal_rates<4, CG>(P, M, m, e, nid, step, KT, m.k_T / detJ * w, qpl * (detJ * w));
+    thermal_rates<4>(P, M, m, e, tn, step, KT, m.k_T / detJ * w, qpl * (detJ * w));
   }
 }
 
-template <int NPE, int LAW, bool CG, bool TH, bool BOX = false>
+template <int NPE, int LAW, int LD, bool TH, bool BOX = false>
 __device__ __forceinline__ void element_one(const StepParams &P, const MixState &M, int64_t e,
                                             float *stash, int stride, long long step) {
   if constexpr (NPE == 8)
-    element_hex<LAW, CG, TH, BOX>(P, M, e, stash, stride, step);
+    element_hex<LAW, LD, TH, BOX>(P, M, e, stash, stride, step);
   else
-    element_tet<LAW, CG, TH>(P, M, e, step);
+    element_tet<LAW, LD, TH>(P, M, e, step);
 }
 
 // Resident threads per SM the element kernel is compiled for (1024: at most
@@ -993,7 +1014,7 @@ __global__ void __launch_bounds__(BS, elem_min_blocks(BS)) k_mix_elements(StepPa
   __shared__ float stash[NPE == 8 ? 12 * BS : 1];
   const long long step = TH ? P.st->step : 0;
   for (int64_t e = (int64_t)blockIdx.x * BS + threadIdx.x; e < P.ne; e += (int64_t)gridDim.x * BS)
-    element_one<NPE, LAW, false, TH, BOX>(P, M, e, &stash[threadIdx.x], BS, step);
+    element_one<NPE, LAW, kLdRo, TH, BOX>(P, M, e, &stash[threadIdx.x], BS, step);
 }
 
 // ---------------------------------------------------------------------------
@@ -1048,12 +1069,12 @@ struct NodeIn {
   uint32_t code;
   uint8_t fl;
 };
-template <bool CG = false>
+template <int LD = kLdRo>
 __device__ __forceinline__ NodeIn node_in(const StepParams &P, const MixState &M, int64_t n) {
   NodeIn in;
   const int64_t np = P.np;
   in.fl = P.nflag[n];
-  in.mass = CG ? __ldcg(&M.mass[n]) : M.mass[n];   // written by the nodal phase
+  in.mass = LD == kLdL2 ? __ldcg(&M.mass[n]) : M.mass[n];   // written by the nodal phase
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     in.vold[k] = M.v[k * np + n];
@@ -1082,7 +1103,7 @@ __device__ __forceinline__ void node_component(const StepParams &P, float dt, fl
   if (fixed) vnext = bv;
 }
 
-template <int NPE, bool CG>
+template <int NPE, int LD, bool BOX = false>
 __device__ __forceinline__ float node_finish(const StepParams &P, const MixState &M, int64_t n,
                                              long long step, float fi0, float fi1, float fi2,
                                              float2 (&x)[3], const float (&vp)[3], float2 *xo,
@@ -1109,10 +1130,10 @@ __device__ __forceinline__ float node_finish(const StepParams &P, const MixState
   }
   float cf[3] = {0.f, 0.f, 0.f};
   if (P.contact && (fl & NF_CONTACT)) {
-    cf[0] = ldx<CG>(&M.cf[n]);
-    cf[1] = ldx<CG>(&M.cf[np + n]);
-    cf[2] = ldx<CG>(&M.cf[2 * np + n]);
-    r = P.tri_on ? ldx<CG>(&M.cfn[n]) : fabsf(cf[2]);
+    cf[0] = ldx<LD>(&M.cf[n]);
+    cf[1] = ldx<LD>(&M.cf[np + n]);
+    cf[2] = ldx<LD>(&M.cf[2 * np + n]);
+    r = P.tri_on ? ldx<LD>(&M.cfn[n]) : fabsf(cf[2]);
   }
   if (!P.contact && (fl & NF_REACTION)) {
     if (P.rnode)
@@ -1146,8 +1167,20 @@ __device__ __forceinline__ float node_finish(const StepParams &P, const MixState
     // the die heat over m cp of material 0
     const float *cur = M.dte + (step & 1) * ne * NPE;
     float sT = 0.f;
-    const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
-    for (int32_t k = 0; k < c; k++) sT += ldx<CG>(&cur[__ldg(&P.slot[b + k])]);
+    if constexpr (BOX && NPE == 8) {
+      int32_t el[8], cor[8];
+      box_node_list(P, n, el, cor);
+      float q[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+        q[j] = (el[j] >= 0) ? ldx<LD>(&cur[(int64_t)el[j] * 8 + cor[j]]) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+        if (el[j] >= 0) sT += q[j];
+    } else {
+      const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
+      for (int32_t k = 0; k < c; k++) sT += ldx<LD>(&cur[__ldg(&P.slot[b + k])]);
+    }
     M.T[n] = pair_add(M.T[n], (sT + M.qc[n] / (mass * P.f_cp0)) * c_dt);
   }
   return r;
@@ -1155,7 +1188,7 @@ __device__ __forceinline__ float node_finish(const StepParams &P, const MixState
 
 // Node update of one node: gather of the element forces in list order, then
 // node_finish. Returns the node's reaction contribution.
-template <int NPE, bool CG, bool BOX = false>
+template <int NPE, int LD, bool BOX = false>
 __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M, int64_t n,
                                           long long step) {
   const int64_t ne = P.ne;
@@ -1171,9 +1204,9 @@ __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M
       g0[j] = g1[j] = g2[j] = 0.f;
       if (el[j] >= 0) {
         const int64_t base = (int64_t)cor[j] * 3 * ne + el[j];
-        g0[j] = ldx<CG>(&M.fe[base]);
-        g1[j] = ldx<CG>(&M.fe[base + ne]);
-        g2[j] = ldx<CG>(&M.fe[base + 2 * ne]);
+        g0[j] = ldx<LD>(&M.fe[base]);
+        g1[j] = ldx<LD>(&M.fe[base + ne]);
+        g2[j] = ldx<LD>(&M.fe[base + 2 * ne]);
       }
     }
 #pragma unroll
@@ -1191,8 +1224,8 @@ __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M
       x[k] = M.xh[k * np + n];
       vp[k] = M.vp[k * np + n];
     }
-    return node_finish<NPE, CG>(P, M, n, step, fi0, fi1, fi2, x, vp, M.xh, M.vp,
-                                node_in<CG>(P, M, n));
+    return node_finish<NPE, LD, true>(P, M, n, step, fi0, fi1, fi2, x, vp, M.xh, M.vp,
+                                      node_in<LD>(P, M, n));
   }
   const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
   // gather over the node's element list in list order, eight entries at a
@@ -1207,9 +1240,9 @@ __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M
       g0[j] = g1[j] = g2[j] = 0.f;
       if (sl[j] >= 0) {
         const int64_t base = (int64_t)(sl[j] % NPE) * 3 * ne + sl[j] / NPE;
-        g0[j] = ldx<CG>(&M.fe[base]);
-        g1[j] = ldx<CG>(&M.fe[base + ne]);
-        g2[j] = ldx<CG>(&M.fe[base + 2 * ne]);
+        g0[j] = ldx<LD>(&M.fe[base]);
+        g1[j] = ldx<LD>(&M.fe[base + ne]);
+        g2[j] = ldx<LD>(&M.fe[base + 2 * ne]);
       }
     }
 #pragma unroll
@@ -1227,8 +1260,8 @@ __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M
     x[k] = M.xh[k * np + n];
     vp[k] = M.vp[k * np + n];
   }
-  return node_finish<NPE, CG>(P, M, n, step, fi0, fi1, fi2, x, vp, M.xh, M.vp,
-                              node_in<CG>(P, M, n));
+  return node_finish<NPE, LD>(P, M, n, step, fi0, fi1, fi2, x, vp, M.xh, M.vp,
+                              node_in<LD>(P, M, n));
 }
 
 template <int NPE, bool BOX>
@@ -1237,7 +1270,7 @@ __global__ void __launch_bounds__(kNodeThreads, WF_NODE_MIN_BLOCKS) k_mix_nodes(
   __shared__ double sh[kNodeThreads / 32];
   __shared__ bool am_last;
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const float r = (n < P.nn) ? node_one<NPE, false, BOX>(P, M, n, P.st->step) : 0.0f;
+  const float r = (n < P.nn) ? node_one<NPE, kLdRo, BOX>(P, M, n, P.st->step) : 0.0f;
   // reaction: only warps holding a contribution reduce (FP64, fixed order);
   // the last block to finish sums all block partials with the whole block.
   const double bs = block_sum_sparse(r, sh);
@@ -1381,7 +1414,7 @@ __global__ void __launch_bounds__(kTileElems, 2) k_mix_tile(StepParams P, MixSta
         x[k] = sx[k * kTileNodes + i];
         vp[k] = svp[k * kTileNodes + i];
       }
-      r += (double)node_finish<8, false>(P, M, id, step, acc[i], acc[kTileNodes + i],
+      r += (double)node_finish<8, kLdRo>(P, M, id, step, acc[i], acc[kTileNodes + i],
                                          acc[2 * kTileNodes + i], x, vp, M.xh, M.vp,
                                          node_in(P, M, id));
     }
@@ -1401,7 +1434,7 @@ __global__ void __launch_bounds__(kNodeThreads, WF_NODE_MIN_BLOCKS) k_mix_shared
   __shared__ bool am_last;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const float r =
-      (i < T.nshared) ? node_one<8, false, BOX>(P, M, __ldg(&T.shared[i]), P.st->step) : 0.0f;
+      (i < T.nshared) ? node_one<8, kLdRo, BOX>(P, M, __ldg(&T.shared[i]), P.st->step) : 0.0f;
   const double bs = block_sum_sparse(r, sh);
   if (threadIdx.x == 0) {
     T.partials[T.ntiles + blockIdx.x] = bs;
@@ -1699,7 +1732,7 @@ __global__ void __launch_bounds__(SweepShape<CY>::threads, 2) k_mix_sweep(StepPa
       own_node(k, x, vp);
       const NodeIn cur = nin;
       nin = node_in(P, M, n_col + pxy * (k + 1));   // plane k+1 <= nz exists
-      racc += (double)node_finish<8, false>(P, M, n_col + pxy * k, step, f0, f1, f2, x, vp,
+      racc += (double)node_finish<8, kLdRo>(P, M, n_col + pxy * k, step, f0, f1, f2, x, vp,
                                             W.xh_o, W.vp_o, cur);
       pf0 = u0;
       pf1 = u1;
@@ -1711,7 +1744,7 @@ __global__ void __launch_bounds__(SweepShape<CY>::threads, 2) k_mix_sweep(StepPa
     float2 x[3];
     float vp[3];
     own_node(bz, x, vp);
-    racc += (double)node_finish<8, false>(P, M, n_col + pxy * bz, step, pf0, pf1, pf2, x, vp,
+    racc += (double)node_finish<8, kLdRo>(P, M, n_col + pxy * bz, step, pf0, pf1, pf2, x, vp,
                                           W.xh_o, W.vp_o, nin);
   }
   const double bs = block_sum_dense(racc, sh);
@@ -1872,11 +1905,11 @@ __global__ void __launch_bounds__(kFlowThreads, 1024 / kFlowThreads) k_mix_flow(
       if (kind == 0) {
         // positions: not written before this read (L1 is safe)
         for (int64_t e = e0 + tid; e < e1; e += kFlowThreads)
-          geometry_one<8, false, true>(P, M, vol, e);
+          geometry_one<8, kLdRo, true>(P, M, vol, e);
       } else {
         const long long step = 0;   // thermal coupling is not run here
         for (int64_t e = e0 + tid; e < e1; e += kFlowThreads) {
-          const GlobalNodes<true, true, false> nd(P, M, e);
+          const GlobalNodes<kLdL2, true, kLdRo> nd(P, M, e);
           ForcesToHbm out{M.fe, P.ne, e};
           element_hex_core<LAW, true, false>(P, M, e, nd, &stash[tid], kFlowThreads, step, out,
                                              StateInPlace{});
@@ -1888,11 +1921,11 @@ __global__ void __launch_bounds__(kFlowThreads, 1024 / kFlowThreads) k_mix_flow(
       if (kind == 1) {
         const float2 zd = die_height(P, P.st->time);   // the step's time (set by the finish)
         for (int64_t n = n0 + tid; n < n1; n += kFlowThreads)
-          nodal_one<8, true, true>(P, M, vol, n, zd);
+          nodal_one<8, kLdL2, true>(P, M, vol, n, zd);
       } else {
         double r = 0.0;
         for (int64_t n = n0 + tid; n < n1; n += kFlowThreads)
-          r += (double)node_one<8, true, true>(P, M, n, 0);
+          r += (double)node_one<8, kLdL2, true>(P, M, n, 0);
         const double bs = block_sum_dense(r, sh);
         if (tid == 0) F.partials[(int64_t)l * F.ntiles[3] + tile] = bs;
       }
@@ -1953,19 +1986,19 @@ __global__ void __launch_bounds__(BS) k_mix_cluster_run(StepParams P, MixState M
   for (int64_t it = 0; it < nsteps; it++) {
     // the die height once per block (FP64), read after the barrier
     if (t == 0) s_zd = P.contact ? die_height(P, time) : make_float2(0.f, 0.f);
-    for (int64_t e = e0 + t; e < e1; e += BS) geometry_one<NPE, true>(P, M, vol, e);
+    for (int64_t e = e0 + t; e < e1; e += BS) geometry_one<NPE, kLdL2>(P, M, vol, e);
     cluster_barrier();
     {
       const float2 zd = s_zd;
-      for (int64_t n = n0 + t; n < n1; n += BS) nodal_one<NPE, true>(P, M, vol, n, zd);
+      for (int64_t n = n0 + t; n < n1; n += BS) nodal_one<NPE, kLdL2>(P, M, vol, n, zd);
     }
     cluster_barrier();
     for (int64_t e = e0 + t; e < e1; e += BS)
-      element_one<NPE, LAW, true, TH>(P, M, e, &stash[t], BS, step0 + it);
+      element_one<NPE, LAW, kLdL2, TH>(P, M, e, &stash[t], BS, step0 + it);
     cluster_barrier();
     double r = 0.0;
     for (int64_t n = n0 + t; n < n1; n += BS)
-      r += (double)node_one<NPE, true>(P, M, n, step0 + it);
+      r += (double)node_one<NPE, kLdL2>(P, M, n, step0 + it);
     const double bsum = block_sum_dense(r, sh);
     if (t == 0) part[it * nb + b] = bsum;   // step it, block b
     cluster_barrier();
@@ -2069,7 +2102,6 @@ struct CopyNodes {
   const float4 *q0, *q1;
   const float2 *q2;
   uint32_t c[8];
-  int32_t nid[8];   // unused (thermal coupling)
   __device__ __forceinline__ float2 x(int a, int k) const {
     const float4 q = k < 2 ? q0[c[a]] : q1[c[a]];
     return k == 1 ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
@@ -2451,6 +2483,358 @@ __global__ void __launch_bounds__(BS + 32, 1) k_mix_cluster_smem(StepParams P, M
     }
   }
   cluster_barrier();
+}
+
+// ---------------------------------------------------------------------------
+// Tile run of box meshes: a whole run of steps in one cooperative launch, one
+// block per SM, for boxes between the cluster run's size and what fits in the
+// SMs' shared memory (about 230,000 hexahedra). There a step's four kernels
+// were launch, ramp-up and two or three dependent L2 round trips each: 20 to 25
+// us for a few microseconds of work. A block owns a tile of elements (and the
+// a share of the nodes), and a step is two phases with a barrier over the
+// grid (1.3 us) after each:
+//   A  the positions of the nodes around the tile, two layers out, into shared
+//      memory; the volumes of the elements around it, one layer out, the J
+//      ratios of all the tile's corner nodes (computed again by every block
+//      that needs them: the geometry and nodal phases without a barrier), the
+//      contact of the own nodes; the tile's elements, their stresses kept in
+//      shared memory for the whole launch, their forces to HBM (L2);
+//   B  the own nodes' update from the forces of their elements.
+// Every element and node runs the per-phase arithmetic with its sums in list
+// order, so the state is bitwise the per-phase one. A warp of its own keeps the
+// time and sums the reaction (FP64: 64 cycles an instruction).
+//
+// The barrier is an arrival counter: a release by one thread after a block
+// barrier, bounded polls with acquire loads (which drop the SM's L1 lines, so
+// plain loads see the other blocks' writes). A wait that runs out (never
+// expected: a cooperative launch has all its blocks resident) sets bit 1 of the
+// step status, which wf_sync reports, and every block leaves.
+constexpr int kTileRunThreads = 608;   // working threads: 96 registers each
+constexpr int kGridSpin = 1 << 22;
+
+__device__ __forceinline__ bool grid_barrier(unsigned *c, unsigned target, StepState *st,
+                                             int *s_ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    red_release(c, 1u);
+    int spins = 0, ok = 1;
+    while (ld_acquire(c) < target)
+      if (++spins > kGridSpin) {
+        atomicOr(&st->status, 2u);
+        ok = 0;
+        break;
+      }
+    *s_ok = ok;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+__device__ __forceinline__ FastDiv fastdiv_of(uint32_t d) {
+  FastDiv f{d, 0u, 0};
+  if (d <= 1) return f;
+  f.s = 32 - __clz(d - 1);
+  f.m = (uint32_t)(((1ull << 32) * ((1ull << f.s) - d)) / d + 1);
+  return f;
+}
+
+// A block of a grid of items: first index and extent per dimension, and the
+// (i, j, k) of a linear index.
+struct Block3 {
+  int i0, j0, k0, nx, ny, nz;
+  FastDiv fx, fxy;
+  __device__ __forceinline__ int count() const { return nx * ny * nz; }
+  __device__ __forceinline__ void set(int a0, int a1, int b0, int b1, int c0, int c1) {
+    i0 = a0; j0 = b0; k0 = c0;
+    nx = a1 - a0; ny = b1 - b0; nz = c1 - c0;
+    fx = fastdiv_of((uint32_t)nx);
+    fxy = fastdiv_of((uint32_t)(nx * ny));
+  }
+  __device__ __forceinline__ void at(int q, int &i, int &j, int &k) const {
+    k = (int)fdiv((uint32_t)q, fxy);
+    const int r = q - k * (int)fxy.d;
+    j = (int)fdiv((uint32_t)r, fx);
+    i = r - j * (int)fx.d;
+  }
+  __device__ __forceinline__ int idx(int i, int j, int k) const { return i + nx * (j + ny * k); }
+};
+
+// Shared memory (bytes): positions [3][n2] float2; predicted velocities [3][n1],
+// J ratios, masses, temperatures [n1]; volumes [e1]; tau and eps_p [7][e0];
+// reaction contributions [n1]; partials [chunk].
+struct TileRunSmem {
+  int x, vp, jr, mass, T, vol, tau, r, part, total;
+  __host__ __device__ TileRunSmem(const TileRunShape &C) {
+    part = 0;
+    x = part + 8 * C.chunk;
+    vp = x + 24 * C.n2;
+    jr = vp + 12 * C.n1;
+    mass = jr + 4 * C.n1;
+    T = mass + (C.thermal ? 4 * C.n1 : 0);
+    vol = T + (C.thermal ? 4 * C.n1 : 0);
+    tau = vol + 4 * C.e1;
+    r = tau + 28 * C.e0;
+    total = r + 4 * C.n1;
+  }
+};
+
+// An element's corners in the staged blocks of nodes (b1: its corner 0 among
+// the tile's corner nodes, b2: among the staged positions).
+struct TileRunNodes {
+  const float2 *sx;
+  const float *sv, *sj, *sm, *sT;
+  int n1, n2, b1, b2, px1, pxy1, px2, pxy2;
+  int32_t n0, px, pxy;   // node id of corner 0 and the mesh's strides
+  static __device__ __forceinline__ int off(int a, int px, int pxy) {
+    return ((a & 3) == 0 ? 0 : (a & 3) == 1 ? 1 : (a & 3) == 2 ? px + 1 : px) + (a < 4 ? 0 : pxy);
+  }
+  __device__ __forceinline__ float2 x(int a, int k) const {
+    return sx[k * n2 + b2 + off(a, px2, pxy2)];
+  }
+  __device__ __forceinline__ float v(int a, int k) const {
+    return sv[k * n1 + b1 + off(a, px1, pxy1)];
+  }
+  __device__ __forceinline__ float j(int a) const { return sj[b1 + off(a, px1, pxy1)]; }
+  __device__ __forceinline__ float T(const MixState &, int a) const {
+    return sT[b1 + off(a, px1, pxy1)];
+  }
+  __device__ __forceinline__ float mass(const MixState &, int a) const {
+    return sm[b1 + off(a, px1, pxy1)];
+  }
+  __device__ __forceinline__ float rate(const StepParams &P, const MixState &M, int a,
+                                        long long step) const {
+    return M.dte[((step + 1) & 1) * P.ne * 8 + n0 + off(a, px, pxy)];
+  }
+};
+
+template <int LAW, bool TH>
+__global__ void __launch_bounds__(kTileRunThreads + 32, 1)
+    k_mix_tile_run(StepParams P, MixState M, float *vol, double *part, int64_t nsteps,
+                   unsigned *bar, TileRunShape C) {
+  constexpr int NT = kTileRunThreads;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ Block3 B[5];   // own elements, own nodes, corner nodes, ring elements, staged nodes
+  __shared__ float2 s_zd;
+  __shared__ int s_ok;
+  const TileRunSmem R(C);
+  double *rpart = reinterpret_cast<double *>(smem + R.part);
+  float2 *sx = reinterpret_cast<float2 *>(smem + R.x);
+  float *sv = reinterpret_cast<float *>(smem + R.vp);
+  float *sj = reinterpret_cast<float *>(smem + R.jr);
+  float *sm = reinterpret_cast<float *>(smem + R.mass);
+  float *sT = reinterpret_cast<float *>(smem + R.T);
+  float *svol = reinterpret_cast<float *>(smem + R.vol);
+  float *tau = reinterpret_cast<float *>(smem + R.tau);
+  float *rbuf = reinterpret_cast<float *>(smem + R.r);
+  const int t = threadIdx.x, lane = t - NT;   // lane >= 0: the service warp
+  const int64_t np = P.np, ne = P.ne;
+  const int bx = P.bx, by = P.by, bz = P.bz;
+  const int px = bx + 1, pxy = px * (by + 1);
+  if (t == 0) {
+    const int b = blockIdx.x, bi = b % C.ta, bj = (b / C.ta) % C.tb, bk = b / (C.ta * C.tb);
+    const int i0 = (int)((int64_t)bx * bi / C.ta), i1 = (int)((int64_t)bx * (bi + 1) / C.ta);
+    const int j0 = (int)((int64_t)by * bj / C.tb), j1 = (int)((int64_t)by * (bj + 1) / C.tb);
+    const int k0 = (int)((int64_t)bz * bk / C.tc), k1 = (int)((int64_t)bz * (bk + 1) / C.tc);
+    B[0].set(i0, i1, j0, j1, k0, k1);
+    // own nodes: the node grid cut as evenly (all of them among the tile's
+    // corner nodes, as (n + 1) b / t is less than one above n b / t)
+    auto cut = [](int n, int q, int parts) { return (int)((int64_t)(n + 1) * q / parts); };
+    B[1].set(cut(bx, bi, C.ta), cut(bx, bi + 1, C.ta), cut(by, bj, C.tb), cut(by, bj + 1, C.tb),
+             cut(bz, bk, C.tc), cut(bz, bk + 1, C.tc));
+    B[2].set(i0, i1 + 1, j0, j1 + 1, k0, k1 + 1);
+    const int ea = max(i0 - 1, 0), eb = min(i1 + 1, bx), fa = max(j0 - 1, 0),
+              fb = min(j1 + 1, by), ga = max(k0 - 1, 0), gb = min(k1 + 1, bz);
+    B[3].set(ea, eb, fa, fb, ga, gb);
+    B[4].set(ea, eb + 1, fa, fb + 1, ga, gb + 1);
+  }
+  __syncthreads();
+  const int me = B[0].count(), mo = B[1].count();
+  for (int q = t; q < me; q += NT + 32) {
+    int i, j, k;
+    B[0].at(q, i, j, k);
+    const int64_t e = B[0].i0 + i + (int64_t)bx * (B[0].j0 + j + (int64_t)by * (B[0].k0 + k));
+#pragma unroll
+    for (int c = 0; c < 6; c++) tau[c * C.e0 + q] = M.tau[c * ne + e];
+    tau[6 * C.e0 + q] = M.pls[e];
+  }
+  double time = 0.0;
+  if (lane == 0) {
+    time = P.st->time;
+    s_zd = P.contact ? die_height(P, time) : make_float2(0.f, 0.f);
+  }
+  const long long step0 = P.st->step;
+  // the service warp: the reaction of step it of the chunk (lanes over the
+  // nodes, then a fixed tree); zeros add nothing and are skipped
+  auto sum_reaction = [&](int64_t it) {
+    double v = 0.0;
+    bool any = false;
+    for (int i = lane; i < mo; i += 32) {
+      const float r = rbuf[i];
+      if (r != 0.f) {
+        v += (double)r;
+        any = true;
+      }
+    }
+    if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    }
+    if (lane == 0) rpart[it] = v;
+  };
+  // the working warps among themselves: the service warp joins at the grid
+  // barriers only
+  auto work_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); };
+  __syncthreads();
+  unsigned target = 0;
+  for (int64_t it = 0; it < nsteps; it++) {
+    const long long step = step0 + it;
+    if (lane >= 0) {
+      if (it > 0) sum_reaction(it - 1);
+    } else {
+      // staged positions; predicted velocities (temperatures) of the corner nodes
+      const Block3 b4 = B[4];
+      for (int q = t; q < b4.count(); q += NT) {
+        int i, j, k;
+        b4.at(q, i, j, k);
+        const int64_t n = b4.i0 + i + (int64_t)px * (b4.j0 + j) + (int64_t)pxy * (b4.k0 + k);
+#pragma unroll
+        for (int c = 0; c < 3; c++) cp_async8(&sx[c * C.n2 + q], &M.xh[c * np + n]);
+      }
+      const Block3 b2 = B[2];
+      for (int q = t; q < b2.count(); q += NT) {
+        int i, j, k;
+        b2.at(q, i, j, k);
+        const int64_t n = b2.i0 + i + (int64_t)px * (b2.j0 + j) + (int64_t)pxy * (b2.k0 + k);
+#pragma unroll
+        for (int c = 0; c < 3; c++) cp_async4(&sv[c * C.n1 + q], &M.vp[c * np + n]);
+        if constexpr (TH) cp_async4(&sT[q], &M.T[n].x);
+      }
+      cp_async_wait_all();
+      work_barrier();
+      const Block3 b3 = B[3];
+      const int px2 = B[4].nx, pxy2 = B[4].nx * B[4].ny;
+      for (int q = t; q < b3.count(); q += NT) {
+        int i, j, k;
+        b3.at(q, i, j, k);
+        const float2 *x = sx + i + px2 * j + pxy2 * k;
+        float r[8][3], J[3][3];
+        float2 o[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          o[c] = x[c * C.n2];
+          r[0][c] = 0.0f;
+        }
+#pragma unroll
+        for (int a = 1; a < 8; a++)
+#pragma unroll
+          for (int c = 0; c < 3; c++)
+            r[a][c] = pair_rel(x[c * C.n2 + TileRunNodes::off(a, px2, pxy2)], o[c]);
+        jacobian_f<8>(r, J);
+        svol[q] = det3f(J) * weightf<8>();
+      }
+    }
+    if (lane < 0) {
+      work_barrier();
+      const Block3 b1 = B[1], b2 = B[2], b3 = B[3];
+      const float2 zd = s_zd;
+      for (int q = t; q < b2.count(); q += NT) {
+        int i, j, k;
+        b2.at(q, i, j, k);
+        const int gi = b2.i0 + i, gj = b2.j0 + j, gk = b2.k0 + k;
+        const int64_t n = gi + (int64_t)px * gj + (int64_t)pxy * gk;
+        const float2 nc = __ldg(&M.nc[n]);
+        // the node's elements in list order
+        float s = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+          const int ii = gi - 1 + (c & 1), jj = gj - 1 + ((c >> 1) & 1), kk = gk - 1 + (c >> 2);
+          if (ii >= 0 && ii < bx && jj >= 0 && jj < by && kk >= 0 && kk < bz)
+            s += svol[b3.idx(ii - b3.i0, jj - b3.j0, kk - b3.k0)];
+        }
+        sj[q] = s * nc.x;
+        if constexpr (TH) sm[q] = P.mass_mode == 0 ? (s * (1.0f / 8)) * nc.y : M.mass[n];
+        if ((unsigned)(gi - b1.i0) < (unsigned)b1.nx && (unsigned)(gj - b1.j0) < (unsigned)b1.ny &&
+            (unsigned)(gk - b1.k0) < (unsigned)b1.nz)
+          nodal_rest<8, kLdL1>(P, M, n, s, nc, zd);
+      }
+    }
+    if (lane < 0) {
+      work_barrier();
+      const Block3 b0 = B[0], b3 = B[3];
+      TileRunNodes nd;
+      nd.sx = sx;
+      nd.sv = sv;
+      nd.sj = sj;
+      nd.sm = sm;
+      nd.sT = sT;
+      nd.n1 = C.n1;
+      nd.n2 = C.n2;
+      nd.px1 = B[2].nx;
+      nd.pxy1 = B[2].nx * B[2].ny;
+      nd.px2 = B[4].nx;
+      nd.pxy2 = B[4].nx * B[4].ny;
+      nd.px = px;
+      nd.pxy = pxy;
+      for (int q = t; q < me; q += NT) {
+        int i, j, k;
+        b0.at(q, i, j, k);
+        const int gi = b0.i0 + i, gj = b0.j0 + j, gk = b0.k0 + k;
+        const int64_t e = gi + (int64_t)bx * (gj + (int64_t)by * gk);
+        nd.b1 = i + nd.px1 * j + nd.pxy1 * k;
+        nd.b2 = (gi - b3.i0) + nd.px2 * (gj - b3.j0) + nd.pxy2 * (gk - b3.k0);
+        nd.n0 = gi + px * gj + pxy * gk;
+        if (it + 1 == nsteps) vol[e] = svol[b3.idx(gi - b3.i0, gj - b3.j0, gk - b3.k0)];
+        ForcesToHbm out{M.fe, ne, e};
+        float stash[12];
+        element_hex_core<LAW, true, TH>(P, M, e, nd, stash, 1, step, out,
+                                        StateSmem{tau + q, C.e0});
+      }
+    }
+    if (!grid_barrier(bar, target += gridDim.x, P.st, &s_ok)) return;
+    if (lane == 0) {   // the next step's time and die height
+      time = time + P.dt;
+      s_zd = P.contact ? die_height(P, time) : make_float2(0.f, 0.f);
+    }
+    if (lane < 0) {
+      const Block3 b1 = B[1];
+      for (int q = t; q < mo; q += NT) {
+        int i, j, k;
+        b1.at(q, i, j, k);
+        const int64_t n = b1.i0 + i + (int64_t)px * (b1.j0 + j) + (int64_t)pxy * (b1.k0 + k);
+        rbuf[q] = node_one<8, kLdL1, true>(P, M, n, step);
+      }
+    }
+    if (!grid_barrier(bar, target += gridDim.x, P.st, &s_ok)) return;
+  }
+  if (lane >= 0) {
+    sum_reaction(nsteps - 1);
+    __syncwarp();
+    for (int64_t it = lane; it < nsteps; it += 32) part[it * gridDim.x + blockIdx.x] = rpart[it];
+  }
+  for (int q = t; q < me; q += NT + 32) {
+    int i, j, k;
+    B[0].at(q, i, j, k);
+    const int64_t e = B[0].i0 + i + (int64_t)bx * (B[0].j0 + j + (int64_t)by * (B[0].k0 + k));
+#pragma unroll
+    for (int c = 0; c < 6; c++) M.tau[c * ne + e] = tau[c * C.e0 + q];
+    M.pls[e] = tau[6 * C.e0 + q];
+  }
+  if (!grid_barrier(bar, target += gridDim.x, P.st, &s_ok)) return;
+  // reaction history: block partials of each step added in block order
+  if (blockIdx.x == 0) {
+    for (int64_t it = t; it < nsteps; it += NT + 32) {
+      double tot = 0.0;
+      for (unsigned i = 0; i < gridDim.x; i++) {
+        const double v = part[it * gridDim.x + i];
+        if (__double_as_longlong(v) << 1 != 0) tot += v;
+      }
+      if (step0 + it < P.hist_cap) P.hist[step0 + it] = tot;
+    }
+    if (lane == 0) {
+      P.st->step = step0 + nsteps;
+      P.st->time = time;
+    }
+  }
 }
 
 __global__ void k_mix_predict(StepParams P, MixState M) {
@@ -3082,6 +3466,93 @@ cudaError_t mix_cluster_smem_run(const StepParams &P, const MixState &M, float *
 cudaError_t mix_cluster_run(const StepParams &P, const MixState &M, float *vol, double *part,
                             int64_t nsteps, int blocks, int bs, cudaStream_t st) {
   return cluster_dispatch(P, M, vol, part, nsteps, blocks, bs, st, false, nullptr);
+}
+
+namespace {
+using TileRunKernel = void (*)(StepParams, MixState, float *, double *, int64_t, unsigned *,
+                               TileRunShape);
+TileRunKernel tile_run_kernel(const StepParams &P) {
+  if (P.thermal) return P.mat_general ? k_mix_tile_run<1, true> : k_mix_tile_run<0, true>;
+  return P.mat_general ? k_mix_tile_run<1, false> : k_mix_tile_run<0, false>;
+}
+}  // namespace
+
+bool mix_tile_run_shape(const StepParams &P, TileRunShape &C) {
+  constexpr double kRowCost = 0.3;
+  if (!P.box || P.tri_on) return false;
+  // the split of the box into at most one tile per SM with the least work in
+  // the largest tile, in instructions of a warp: passes of the working threads
+  // over the elements (800 each), the ring elements (170), the corner and own
+  // nodes (60 and 350) and the staged nodes (40)
+  const int n[3] = {P.bx, P.by, P.bz};
+  double best = 0.0;
+  bool found = false;
+  for (int a = 1; a <= P.sms && a <= n[0]; a++)
+    for (int b = 1; a * b <= P.sms && b <= n[1]; b++) {
+      const int c = std::min(P.sms / (a * b), n[2]);
+      const int64_t x = (n[0] + a - 1) / a, y = (n[1] + b - 1) / b, z = (n[2] + c - 1) / c;
+      TileRunShape S;
+      S.ta = a;
+      S.tb = b;
+      S.tc = c;
+      S.chunk = kTileRunChunk;
+      S.thermal = P.thermal;
+      const int64_t n2 = (x + 3) * (y + 3) * (z + 3);
+      if (n2 > 8000) continue;   // beyond the shared memory in any case
+      S.e0 = (int)(x * y * z);
+      S.n1 = (int)((x + 1) * (y + 1) * (z + 1));
+      S.e1 = (int)((x + 2) * (y + 2) * (z + 2));
+      S.n2 = (int)n2;
+      if (TileRunSmem(S).total > 225 * 1024) continue;
+      auto passes = [](int64_t items) {
+        return (double)((items + kTileRunThreads - 1) / kTileRunThreads);
+      };
+      const double cost = 800 * passes(S.e0) + 170 * passes(S.e1) + 60 * passes(S.n1) +
+                          350 * passes(S.e0) + 40 * passes(S.n2) + 0.1 * (S.e0 + S.e1 + S.n2);
+      // a warp over several short rows meets bank conflicts and partial sectors
+      const double rows = 1.0 + kRowCost * (32.0 / x > 1.0 ? 32.0 / x - 1.0 : 0.0);
+      const double work = cost * rows;
+      if (!found || work < best) {
+        best = work;
+        C = S;
+        found = true;
+      }
+    }
+  if (!found) return false;
+  const TileRunKernel k = tile_run_kernel(P);
+  const int bytes = TileRunSmem(C).total;
+  int dev = 0, coop = 0, per = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kTileRunThreads + 32, bytes) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return per >= 1;
+}
+
+cudaError_t mix_tile_run(const StepParams &P, const MixState &M, float *vol, double *part,
+                         unsigned *bar, int64_t nsteps, const TileRunShape &C, cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(unsigned), st);
+  if (e != cudaSuccess) return e;
+  const TileRunKernel k = tile_run_kernel(P);
+  const int bytes = TileRunSmem(C).total;
+  const cudaError_t a =
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+  if (a != cudaSuccess) return a;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.gridDim = dim3((unsigned)(C.ta * C.tb * C.tc));
+  cfg.blockDim = dim3(kTileRunThreads + 32);
+  cfg.dynamicSmemBytes = (size_t)bytes;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, P, M, vol, part, nsteps, bar, C);
 }
 
 void mix_predict(const StepParams &P, const MixState &M, cudaStream_t st) {
