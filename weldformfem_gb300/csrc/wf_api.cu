@@ -1353,12 +1353,16 @@ WF_API wf_status wf_get_specimen_reaction(wf_domain *d, int32_t spec, double *ou
   if (n) *n = have;
   const int64_t m = std::min(cap, have);
   if (out && m > 0) {
-    std::vector<double> all((size_t)m * d->nspec);
-    d->d2h_bytes += (int64_t)(sizeof(double) * all.size());
-    CUDA_TRY(cudaMemcpyAsync(all.data(), d->P.hist_spec, sizeof(double) * all.size(),
-                             cudaMemcpyDeviceToHost, d->stream));
+    // the specimen's column of hist_spec [step][specimen], gathered on the device
+    double *col = nullptr;
+    CUDA_TRY(pool_alloc(d, reinterpret_cast<void **>(&col), sizeof(double) * m));
+    copy_column(d->P.hist_spec + spec, d->nspec, m, col, d->stream);
+    const cudaError_t e = cudaMemcpyAsync(out, col, sizeof(double) * m, cudaMemcpyDeviceToHost,
+                                          d->stream);
+    cudaFreeAsync(col, d->stream);
+    CUDA_TRY(e);
     CUDA_TRY(cudaStreamSynchronize(d->stream));
-    for (int64_t i = 0; i < m; i++) out[i] = all[(size_t)i * d->nspec + spec];
+    d->d2h_bytes += (int64_t)sizeof(double) * m;
   }
   return WF_OK;
 }
@@ -1519,6 +1523,26 @@ void box_dims(const wf_domain *d, int *nx, int *ny, int *nz) {
   *nz = (int)ez;
 }
 
+// The box of a specimen from its first element's corners (as box_dims), if its
+// counts are a box's.
+bool spec_box(const int32_t *first, int64_t e0, int64_t e1, int64_t n0, int64_t n1, SpecBox &b) {
+  const int64_t px = (int64_t)first[3] - first[0], pxy = (int64_t)first[4] - first[0];
+  if (first[0] != n0 || px < 2 || pxy < 2 * px || pxy % px != 0) return false;
+  const int64_t exy = (px - 1) * (pxy / px - 1), ne = e1 - e0;
+  if (ne % exy != 0 || pxy * (ne / exy + 1) != n1 - n0 || e1 > INT32_MAX || n1 > INT32_MAX)
+    return false;
+  b.e0 = (int32_t)e0;
+  b.n0 = (int32_t)n0;
+  b.bx = (int32_t)(px - 1);
+  b.by = (int32_t)(pxy / px - 1);
+  b.bz = (int32_t)(ne / exy);
+  b.fd_ex = make_fastdiv((uint32_t)b.bx);
+  b.fd_exy = make_fastdiv((uint32_t)exy);
+  b.fd_nx = make_fastdiv((uint32_t)px);
+  b.fd_nxy = make_fastdiv((uint32_t)pxy);
+  return true;
+}
+
 // Device allocation kept with the domain (build_tiles' tables).
 cudaError_t keep_alloc(void *ctx, void **p, size_t bytes) {
   return dalloc_raw(static_cast<wf_domain *>(ctx), reinterpret_cast<char **>(p), bytes);
@@ -1534,6 +1558,7 @@ cudaError_t keep_alloc(void *ctx, void **p, size_t bytes) {
 // the same mesh shape takes them instead of timing the candidates again.
 struct TuneKey {
   int device;
+  // specimens: 0 none, 1 from the arrays, 2 boxes
   int32_t npe, mat_general, thermal, contact, tri_on, energy_on, specimens, tiled;
   int64_t ne, nn;
   bool operator<(const TuneKey &o) const {
@@ -1562,7 +1587,7 @@ bool runs_element_kernel(const wf_domain *d) {
 TuneKey tune_key(const wf_domain *d) {
   const StepParams &P = d->P;
   return TuneKey{d->device, P.npe, P.mat_general, P.thermal, P.contact, P.tri_on, P.energy_on,
-                 P.nspec ? 1 : 0, runs_element_kernel(d) ? 0 : 1, d->ne, d->nn};
+                 P.nspec ? (P.sbox ? 2 : 1) : 0, runs_element_kernel(d) ? 0 : 1, d->ne, d->nn};
 }
 
 wf_status autotune_launches(wf_domain *d) {
@@ -2000,14 +2025,51 @@ WF_API wf_status wf_init(wf_domain *d) {
   const double *x_aos = d->mesh_x;
   CUDA_TRY(build_connectivity(d->mesh_el, ne, d->npe, nn, el, nullptr, nullptr, nullptr,
                               d->stream));
+  if (d->nspec) {
+    // the specimen of each element and node, filled on the device
+    int64_t *eo = nullptr, *no = nullptr;
+    uint16_t *es = nullptr, *ns = nullptr;
+    CUDA_TRY(upload(d, &eo, d->spec_eoff));
+    CUDA_TRY(upload(d, &no, d->spec_noff));
+    CUDA_TRY(dalloc_raw(d, &es, ne));
+    CUDA_TRY(dalloc_raw(d, &ns, nn));
+    fill_owner(eo, d->nspec, ne, es, d->stream);
+    fill_owner(no, d->nspec, nn, ns, d->stream);
+    CUDA_TRY(cudaGetLastError());
+    P.espec = es;
+    P.nspec_of = ns;
+    // specimens that are all boxes (AddBoxLength numbering): like a box mesh
+    // below, with the specimen's dimensions from a table
+    if (d->precision == WF_MIXED && d->npe == 8 && d->use_box) {
+      const wf_status hs = host_mesh(d);
+      if (hs) return hs;
+      std::vector<SpecBox> sb(d->nspec);
+      bool all = true;
+      for (int32_t k = 0; k < d->nspec && all; k++)
+        all = spec_box(d->elnod.data() + 8 * d->spec_eoff[k], d->spec_eoff[k], d->spec_eoff[k + 1],
+                       d->spec_noff[k], d->spec_noff[k + 1], sb[k]);
+      if (all) {
+        SpecBox *sbd = nullptr;
+        CUDA_TRY(upload(d, &sbd, sb));
+        int ok = 0;
+        int32_t *flag = nullptr;
+        CUDA_TRY(dalloc_raw(d, &flag, 1));
+        CUDA_TRY(check_spec_boxes(P.elnod, ne, P.espec, sbd, flag, d->stream, &ok));
+        if (ok) P.sbox = sbd;
+      }
+    }
+  }
   // a box mesh (AddBoxLength numbering, however it was uploaded; mixed
   // precision): the mixed kernels compute corners and node lists instead of
   // loading them
   if (d->precision == WF_MIXED) {
     int bnx = 0, bny = 0, bnz = 0, is_box = 0;
     box_dims(d, &bnx, &bny, &bnz);
-    if (d->npe == 8 && !d->nspec && d->use_box && bnx > 0)
-      CUDA_TRY(check_box(P.elnod, ne, nn, bnx, bny, bnz, d->stream, &is_box));
+    if (d->npe == 8 && !d->nspec && d->use_box && bnx > 0) {
+      int32_t *flag = nullptr;
+      CUDA_TRY(dalloc_raw(d, &flag, 1));
+      CUDA_TRY(check_box(P.elnod, ne, nn, bnx, bny, bnz, flag, d->stream, &is_box));
+    }
     P.box = is_box;
     if (is_box) {
       P.bx = bnx;
@@ -2024,7 +2086,7 @@ WF_API wf_status wf_init(wf_domain *d) {
   // cluster run, and no tiled steps (host lists are then built from the host
   // mirror if a host caller asks)
   const bool lists = !(P.box && !d->thermal && !d->tri && d->step_mode != 3 &&
-                       ne > kClusterMaxElems);
+                       ne > kClusterMaxElems) && !P.sbox;
   if (lists) {
     int32_t *off = nullptr, *sl = nullptr;
     CUDA_TRY(dalloc_raw(d, &off, nn + 1));
@@ -2198,11 +2260,6 @@ WF_API wf_status wf_init(wf_domain *d) {
   if (d->nspec) {
     const int32_t S_ = d->nspec;
     P.nspec = S_;
-    std::vector<uint16_t> es(ne), ns(nn);
-    for (int32_t k = 0; k < S_; k++) {
-      for (int64_t e = d->spec_eoff[k]; e < d->spec_eoff[k + 1]; e++) es[e] = (uint16_t)k;
-      for (int64_t n = d->spec_noff[k]; n < d->spec_noff[k + 1]; n++) ns[n] = (uint16_t)k;
-    }
     std::vector<SpecF> sf(S_);
     for (int32_t k = 0; k < S_; k++) {
       const double dt = d->spec_dt[k];
@@ -2210,22 +2267,18 @@ WF_API wf_status wf_init(wf_domain *d) {
                     (float)(P.gamma * dt), (float)((1.0 - P.gamma) * dt), 0.f, 0.f, 0.f};
     }
     std::vector<int32_t> rl(d->react_nodes.begin(), d->react_nodes.end());
-    std::sort(rl.begin(), rl.end());
+    if (!std::is_sorted(rl.begin(), rl.end())) std::sort(rl.begin(), rl.end());
     std::vector<int32_t> rloff(S_ + 1, 0);
-    for (int32_t n : rl) rloff[ns[n] + 1]++;
-    for (int32_t k = 0; k < S_; k++) rloff[k + 1] += rloff[k];
-    uint16_t *esd = nullptr, *nsd = nullptr;
+    for (int32_t k = 0; k < S_; k++)
+      rloff[k + 1] = (int32_t)(std::lower_bound(rl.begin() + rloff[k], rl.end(),
+                                                d->spec_noff[k + 1]) - rl.begin());
     double *sdt = nullptr;
     SpecF *sfd = nullptr;
     int32_t *rld = nullptr, *rlo = nullptr;
-    CUDA_TRY(upload(d, &esd, es));
-    CUDA_TRY(upload(d, &nsd, ns));
     CUDA_TRY(upload(d, &sdt, d->spec_dt));
     CUDA_TRY(upload(d, &sfd, sf));
     CUDA_TRY(upload(d, &rld, rl));
     CUDA_TRY(upload(d, &rlo, rloff));
-    P.espec = esd;
-    P.nspec_of = nsd;
     P.spec_dt = sdt;
     P.specf = sfd;
     P.rlist = rld;

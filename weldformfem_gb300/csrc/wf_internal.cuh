@@ -96,6 +96,13 @@ struct StepState {
 // Node flags (uint8 per node).
 enum : uint8_t { NF_REACTION = 1, NF_CONTACT = 2 };
 
+// A specimen of a batched ensemble that is a box mesh of bx x by x bz hexahedra
+// in the AddBoxLength numbering from element e0 and node n0 on.
+struct SpecBox {
+  int32_t e0, n0, bx, by, bz;
+  FastDiv fd_ex, fd_exy, fd_nx, fd_nxy;
+};
+
 // Kernel parameters shared by both precisions. Node arrays are SoA with
 // component stride np (padded node count); element arrays are SoA with
 // component stride ne unless noted.
@@ -191,7 +198,12 @@ struct StepParams {
   int32_t box, bx, by, bz;
   FastDiv fd_ex, fd_exy;  // bx, bx by: element index -> (i, j, k)
   FastDiv fd_nx, fd_nxy;  // bx + 1, (bx + 1)(by + 1): node index -> (i, j, k)
+  const SpecBox *sbox;    // [nspec] the same of every specimen, all of them boxes (else null)
 };
+
+// Where the mixed kernels take an element's corners and a node's list from: the
+// arrays, the box's numbering, or the numbering of the specimen's box.
+enum : int { kBoxNone = 0, kBoxOne = 1, kBoxSpec = 2 };
 
 // FP64 state (all doubles).
 struct Fp64State {
@@ -429,6 +441,8 @@ int mix_node_grid(int64_t nn);
 // ---- reductions (wf_reduce.cu) ---------------------------------------------
 // Per-specimen reaction sums of the step just completed (batched ensemble).
 void spec_reaction(const StepParams &P, cudaStream_t st);
+// dst[i] = src[i * stride], i < n.
+void copy_column(const double *src, int64_t stride, int64_t n, double *dst, cudaStream_t st);
 // Kinetic energy and internal-energy increment of the step just completed,
 // appended to the energy history (fixed-order reduction).
 int energy_grid(const StepParams &P);
@@ -448,13 +462,32 @@ void min_edge_length_box(const double *x, int64_t np, int32_t bx, int32_t by, in
 // order) and n's corner in each; el[q] = -1 where the box has none. q = dk * 4
 // + dj * 2 + di for the element (i - 1 + di, j - 1 + dj, k - 1 + dk); the
 // corner at (1 - di, 1 - dj, 1 - dk) of the element is 4 z + (x ^ 3 y).
+template <int BOX = kBoxOne>
 __device__ __forceinline__ void box_node_list(const StepParams &P, int64_t n, int32_t (&el)[8],
                                               int32_t (&cor)[8]) {
-  const uint32_t un = (uint32_t)n;
-  const int32_t k = (int32_t)fdiv(un, P.fd_nxy);
-  const uint32_t r = un - (uint32_t)k * P.fd_nxy.d;
-  const int32_t j = (int32_t)fdiv(r, P.fd_nx);
-  const int32_t i = (int32_t)(r - (uint32_t)j * P.fd_nx.d);
+  uint32_t un = (uint32_t)n;
+  FastDiv fx, fxy;
+  int32_t bx, by, bz, e0 = 0;
+  if constexpr (BOX == kBoxSpec) {
+    const SpecBox &s = P.sbox[P.nspec_of[n]];
+    un -= (uint32_t)s.n0;
+    fx = s.fd_nx;
+    fxy = s.fd_nxy;
+    bx = s.bx;
+    by = s.by;
+    bz = s.bz;
+    e0 = s.e0;
+  } else {
+    fx = P.fd_nx;
+    fxy = P.fd_nxy;
+    bx = P.bx;
+    by = P.by;
+    bz = P.bz;
+  }
+  const int32_t k = (int32_t)fdiv(un, fxy);
+  const uint32_t r = un - (uint32_t)k * fxy.d;
+  const int32_t j = (int32_t)fdiv(r, fx);
+  const int32_t i = (int32_t)(r - (uint32_t)j * fx.d);
 #pragma unroll
   for (int dk = 0; dk < 2; dk++)
 #pragma unroll
@@ -462,9 +495,9 @@ __device__ __forceinline__ void box_node_list(const StepParams &P, int64_t n, in
 #pragma unroll
       for (int di = 0; di < 2; di++) {
         const int32_t ii = i - 1 + di, jj = j - 1 + dj, kk = k - 1 + dk;
-        const bool ok = ii >= 0 && ii < P.bx && jj >= 0 && jj < P.by && kk >= 0 && kk < P.bz;
+        const bool ok = ii >= 0 && ii < bx && jj >= 0 && jj < by && kk >= 0 && kk < bz;
         const int q = dk * 4 + dj * 2 + di;
-        el[q] = ok ? ii + P.bx * (jj + P.by * kk) : -1;
+        el[q] = ok ? e0 + ii + bx * (jj + by * kk) : -1;
         cor[q] = 4 * (1 - dk) + ((1 - di) ^ (3 * (1 - dj)));
       }
 }
@@ -481,6 +514,8 @@ int64_t connectivity_scratch_ints(int64_t nn);
 // dst[idx[i]] = val[i] and dst[idx[i]] |= bit for i < n (distinct indices).
 void scatter_u32(uint32_t *dst, const int32_t *idx, const uint32_t *val, int64_t n,
                  cudaStream_t st);
+// dst[i] = k for off[k] <= i < off[k + 1], k < parts: the owner of each of n items.
+void fill_owner(const int64_t *off, int parts, int64_t n, uint16_t *dst, cudaStream_t st);
 void or_flags(uint8_t *dst, const int32_t *idx, uint8_t bit, int64_t n, cudaStream_t st);
 // Whether every entry of el[0, n) names a node in [0, nn) (*bad = 0), on the
 // device; flag: one device int of scratch. Synchronises st.
@@ -504,8 +539,14 @@ cudaError_t build_tiles(const int32_t *el_soa, const double *x_soa, int64_t np, 
 
 // Whether the SoA connectivity is the AddBoxLength numbering of nx x ny x nz
 // hexahedra (*is_box = 1): a device check of every element.
+// flag: one device int of scratch, here and below.
 cudaError_t check_box(const int32_t *el_soa, int64_t ne, int64_t nn, int nx, int ny, int nz,
-                      cudaStream_t st, int *is_box);
+                      int32_t *flag, cudaStream_t st, int *is_box);
+
+// Whether every specimen's elements are the AddBoxLength numbering of its box
+// (*all = 1): a device check of every element.
+cudaError_t check_spec_boxes(const int32_t *el_soa, int64_t ne, const uint16_t *espec,
+                             const SpecBox *sbox, int32_t *flag, cudaStream_t st, int *all);
 
 // AoS [nn][3] -> SoA [3][np], zero padded
 void coords_soa(const double *x_aos, int64_t nn, int64_t np, double *out, cudaStream_t st);

@@ -75,15 +75,32 @@ __device__ __forceinline__ T ldx(const T *p) {
     return __ldg(p);
 }
 
-// Box meshes (P.box): the corners of element e in the AddBoxLength numbering.
+// Box meshes (P.box, or the element's specimen in P.sbox): the corners of element
+// e in the AddBoxLength numbering.
+template <int BOX>
 __device__ __forceinline__ void box_corners(const StepParams &P, int64_t e, int32_t (&nid)[8]) {
-  const uint32_t ue = (uint32_t)e;
-  const uint32_t k = fdiv(ue, P.fd_exy);
-  const uint32_t r = ue - k * P.fd_exy.d;
-  const uint32_t j = fdiv(r, P.fd_ex);
-  const uint32_t i = r - j * P.fd_ex.d;
-  const int32_t px = (int32_t)P.fd_nx.d, pxy = (int32_t)P.fd_nxy.d;
-  const int32_t n0 = (int32_t)i + px * (int32_t)j + pxy * (int32_t)k;
+  uint32_t ue = (uint32_t)e;
+  FastDiv fx, fxy;
+  int32_t px, pxy, nbase = 0;
+  if constexpr (BOX == kBoxSpec) {
+    const SpecBox &s = P.sbox[P.espec[e]];
+    ue -= (uint32_t)s.e0;
+    fx = s.fd_ex;
+    fxy = s.fd_exy;
+    px = (int32_t)s.fd_nx.d;
+    pxy = (int32_t)s.fd_nxy.d;
+    nbase = s.n0;
+  } else {
+    fx = P.fd_ex;
+    fxy = P.fd_exy;
+    px = (int32_t)P.fd_nx.d;
+    pxy = (int32_t)P.fd_nxy.d;
+  }
+  const uint32_t k = fdiv(ue, fxy);
+  const uint32_t r = ue - k * fxy.d;
+  const uint32_t j = fdiv(r, fx);
+  const uint32_t i = r - j * fx.d;
+  const int32_t n0 = nbase + (int32_t)i + px * (int32_t)j + pxy * (int32_t)k;
   nid[0] = n0;
   nid[1] = n0 + 1;
   nid[2] = n0 + 1 + px;
@@ -99,11 +116,11 @@ __device__ __forceinline__ float weightf() {
   return NPE == 8 ? 8.0f : 1.0f / 6.0f;
 }
 
-template <int NPE, int LD, bool BOX = false>
+template <int NPE, int LD, int BOX = kBoxNone>
 __device__ __forceinline__ void rel_coords(const StepParams &P, const MixState &M, int64_t e,
                                            float (&r)[NPE][3], int32_t (&nid)[NPE]) {
   if constexpr (BOX && NPE == 8) {
-    box_corners(P, e, nid);
+    box_corners<BOX>(P, e, nid);
   } else {
 #pragma unroll
     for (int a = 0; a < NPE; a++) nid[a] = __ldg(&P.elnod[a * P.ne + e]);
@@ -181,7 +198,7 @@ __device__ __forceinline__ void shape_derivs_f(const float J[3][3], float dH[3][
 }
 
 // ---------------------------------------------------------------------------
-template <int NPE, int LD, bool BOX = false>
+template <int NPE, int LD, int BOX = kBoxNone>
 __device__ __forceinline__ void geometry_one(const StepParams &P, const MixState &M, float *vol,
                                              int64_t e) {
   float r[NPE][3];
@@ -197,7 +214,7 @@ __device__ __forceinline__ void geometry_one(const StepParams &P, const MixState
 // Two elements per iteration when the grid strides (a persistent grid or
 // several items per thread): both elements' coordinate gathers are issued
 // before either's arithmetic, so twice the loads are in flight.
-template <int NPE, int BS, bool BOX>
+template <int NPE, int BS, int BOX>
 __global__ void __launch_bounds__(BS) k_mix_geometry(StepParams P, MixState M, float *vol) {
   const int64_t stride = (int64_t)gridDim.x * BS;
   int64_t e = (int64_t)blockIdx.x * BS + threadIdx.x;
@@ -307,14 +324,14 @@ __device__ __forceinline__ void tri_contact_mixed(const StepParams &P, const Mix
 // zd: the rigid plane's height at the step's time as a (hi, lo) float pair,
 // formed once per thread by the caller (die_height), so that the gap of a
 // contact node takes no FP64 instruction.
-template <int NPE, int LD, bool BOX = false>
+template <int NPE, int LD, int BOX = kBoxNone>
 __device__ __forceinline__ void nodal_gather(const StepParams &P, const MixState &M,
                                              const float *vol, int64_t n, float &s, float2 &nc) {
   s = 0.0f;
   if constexpr (BOX && NPE == 8) {
     // the node's elements in list order, computed from its indices
     int32_t el[8], cor[8];
-    box_node_list(P, n, el, cor);
+    box_node_list<BOX>(P, n, el, cor);
     nc = __ldg(&M.nc[n]);
     float g[8];
 #pragma unroll
@@ -401,7 +418,7 @@ __device__ __forceinline__ void nodal_rest(const StepParams &P, const MixState &
   }
 }
 
-template <int NPE, int LD, bool BOX = false>
+template <int NPE, int LD, int BOX = kBoxNone>
 __device__ __forceinline__ void nodal_one(const StepParams &P, const MixState &M,
                                           const float *vol, int64_t n, float2 zd) {
   float s;
@@ -412,7 +429,7 @@ __device__ __forceinline__ void nodal_one(const StepParams &P, const MixState &M
 
 // Two nodes per iteration when the grid strides: both nodes' volume gathers
 // are in flight before either's rest.
-template <int NPE, int BS, bool BOX>
+template <int NPE, int BS, int BOX>
 __global__ void __launch_bounds__(BS) k_mix_nodal(StepParams P, MixState M, const float *vol) {
   // the die height once per block: FP64 runs at 1/64 of the FP32 rate, and
   // formed by every thread it kept the FP64 pipe two-thirds busy
@@ -704,7 +721,7 @@ struct ThermalNodes {
 // CGX: positions and predicted velocities through L2 as well (the cluster
 // run); the dataflow step reads them through L1 (no tile of its launch writes
 // them before every read of them is done) and only the J ratios through L2.
-template <int LD, bool BOX = false, int LDX = LD>
+template <int LD, int BOX = kBoxNone, int LDX = LD>
 struct GlobalNodes : ThermalNodes<8, LD> {
   using ThermalNodes<8, LD>::nid;
   const float2 *xh;
@@ -713,7 +730,7 @@ struct GlobalNodes : ThermalNodes<8, LD> {
   __device__ __forceinline__ GlobalNodes(const StepParams &P, const MixState &M, int64_t e)
       : xh(M.xh), vp(M.vp), jr(M.jr), np(P.np) {
     if constexpr (BOX) {
-      box_corners(P, e, nid);
+      box_corners<BOX>(P, e, nid);
     } else {
 #pragma unroll
       for (int a = 0; a < 8; a++) nid[a] = __ldg(&P.elnod[a * P.ne + e]);
@@ -890,7 +907,7 @@ __device__ __forceinline__ void element_hex_core(const StepParams &P, const MixS
 }
 
 // Per-phase kernels and the cluster run: node values from HBM, forces to HBM.
-template <int LAW, int LD, bool TH, bool BOX = false>
+template <int LAW, int LD, bool TH, int BOX = kBoxNone>
 __device__ __forceinline__ void element_hex(const StepParams &P, const MixState &M, int64_t e,
                                             float *stash, int stride, long long step) {
   const GlobalNodes<LD, BOX> nd(P, M, e);
@@ -992,7 +1009,7 @@ __device__ __forceinline__ void element_tet(const StepParams &P, const MixState 
   }
 }
 
-template <int NPE, int LAW, int LD, bool TH, bool BOX = false>
+template <int NPE, int LAW, int LD, bool TH, int BOX = kBoxNone>
 __device__ __forceinline__ void element_one(const StepParams &P, const MixState &M, int64_t e,
                                             float *stash, int stride, long long step) {
   if constexpr (NPE == 8)
@@ -1008,7 +1025,7 @@ __device__ __forceinline__ void element_one(const StepParams &P, const MixState 
 #endif
 constexpr int elem_min_blocks(int bs) { return WF_ELEM_THREADS_PER_SM / bs; }
 
-template <int NPE, int BS, int LAW, bool TH, bool BOX>
+template <int NPE, int BS, int LAW, bool TH, int BOX>
 __global__ void __launch_bounds__(BS, elem_min_blocks(BS)) k_mix_elements(StepParams P,
                                                                           MixState M) {
   __shared__ float stash[NPE == 8 ? 12 * BS : 1];
@@ -1103,7 +1120,7 @@ __device__ __forceinline__ void node_component(const StepParams &P, float dt, fl
   if (fixed) vnext = bv;
 }
 
-template <int NPE, int LD, bool BOX = false>
+template <int NPE, int LD, int BOX = kBoxNone>
 __device__ __forceinline__ float node_finish(const StepParams &P, const MixState &M, int64_t n,
                                              long long step, float fi0, float fi1, float fi2,
                                              float2 (&x)[3], const float (&vp)[3], float2 *xo,
@@ -1169,7 +1186,7 @@ __device__ __forceinline__ float node_finish(const StepParams &P, const MixState
     float sT = 0.f;
     if constexpr (BOX && NPE == 8) {
       int32_t el[8], cor[8];
-      box_node_list(P, n, el, cor);
+      box_node_list<BOX>(P, n, el, cor);
       float q[8];
 #pragma unroll
       for (int j = 0; j < 8; j++)
@@ -1188,7 +1205,7 @@ __device__ __forceinline__ float node_finish(const StepParams &P, const MixState
 
 // Node update of one node: gather of the element forces in list order, then
 // node_finish. Returns the node's reaction contribution.
-template <int NPE, int LD, bool BOX = false>
+template <int NPE, int LD, int BOX = kBoxNone>
 __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M, int64_t n,
                                           long long step) {
   const int64_t ne = P.ne;
@@ -1197,7 +1214,7 @@ __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M
     // the node's elements in list order, from its indices; all loads issued
     // before the sum, which adds the existing entries in list order
     int32_t el[8], cor[8];
-    box_node_list(P, n, el, cor);
+    box_node_list<BOX>(P, n, el, cor);
     float g0[8], g1[8], g2[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
@@ -1224,7 +1241,7 @@ __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M
       x[k] = M.xh[k * np + n];
       vp[k] = M.vp[k * np + n];
     }
-    return node_finish<NPE, LD, true>(P, M, n, step, fi0, fi1, fi2, x, vp, M.xh, M.vp,
+    return node_finish<NPE, LD, BOX>(P, M, n, step, fi0, fi1, fi2, x, vp, M.xh, M.vp,
                                       node_in<LD>(P, M, n));
   }
   const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
@@ -1264,7 +1281,7 @@ __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M
                               node_in<LD>(P, M, n));
 }
 
-template <int NPE, bool BOX>
+template <int NPE, int BOX>
 __global__ void __launch_bounds__(kNodeThreads, WF_NODE_MIN_BLOCKS) k_mix_nodes(StepParams P,
                                                                              MixState M) {
   __shared__ double sh[kNodeThreads / 32];
@@ -1426,7 +1443,7 @@ __global__ void __launch_bounds__(kTileElems, 2) k_mix_tile(StepParams P, MixSta
 // The shared nodes: list-order gather from HBM and node update; the last
 // block adds the reaction partials of the tiles and of its own blocks in a
 // fixed order and advances the step state.
-template <bool BOX>
+template <int BOX>
 __global__ void __launch_bounds__(kNodeThreads, WF_NODE_MIN_BLOCKS) k_mix_shared(StepParams P,
                                                                               MixState M,
                                                                               TileParams T) {
@@ -2878,9 +2895,10 @@ __global__ void k_mix_init_nodal(StepParams P, MixState M, Fp64State S, const fl
   float s = 0.0f;
   double rs = 0.0;
   int32_t c = 0;
-  if (NPE == 8 && P.box) {
+  if (NPE == 8 && (P.box || P.sbox)) {
     int32_t el[8], cor[8];
-    box_node_list(P, n, el, cor);
+    if (P.box) box_node_list(P, n, el, cor);
+    else box_node_list<kBoxSpec>(P, n, el, cor);
 #pragma unroll
     for (int j = 0; j < 8; j++)
       if (el[j] >= 0) {
@@ -3031,7 +3049,7 @@ unsigned tuned_grid(Kernel kernel, int bs, int ept, int64_t n) {
   return g < full ? g : full;
 }
 
-template <int NPE, bool BOX>
+template <int NPE, int BOX>
 void launch_geometry_box(const StepParams &P, const MixState &M, float *vol, cudaStream_t st,
                          LaunchCfg c) {
   switch (c.bs) {
@@ -3056,11 +3074,14 @@ void launch_geometry_box(const StepParams &P, const MixState &M, float *vol, cud
 template <int NPE>
 void launch_geometry(const StepParams &P, const MixState &M, float *vol, cudaStream_t st,
                      LaunchCfg c) {
-  if (NPE == 8 && P.box) launch_geometry_box<NPE, true>(P, M, vol, st, c);
-  else launch_geometry_box<NPE, false>(P, M, vol, st, c);
+  if constexpr (NPE == 8) {
+    if (P.box) return launch_geometry_box<NPE, kBoxOne>(P, M, vol, st, c);
+    if (P.sbox) return launch_geometry_box<NPE, kBoxSpec>(P, M, vol, st, c);
+  }
+  launch_geometry_box<NPE, kBoxNone>(P, M, vol, st, c);
 }
 
-template <int NPE, bool BOX>
+template <int NPE, int BOX>
 void launch_nodal_box(const StepParams &P, const MixState &M, const float *vol, cudaStream_t st,
                       LaunchCfg c) {
   switch (c.bs) {
@@ -3085,11 +3106,14 @@ void launch_nodal_box(const StepParams &P, const MixState &M, const float *vol, 
 template <int NPE>
 void launch_nodal(const StepParams &P, const MixState &M, const float *vol, cudaStream_t st,
                   LaunchCfg c) {
-  if (NPE == 8 && P.box) launch_nodal_box<NPE, true>(P, M, vol, st, c);
-  else launch_nodal_box<NPE, false>(P, M, vol, st, c);
+  if constexpr (NPE == 8) {
+    if (P.box) return launch_nodal_box<NPE, kBoxOne>(P, M, vol, st, c);
+    if (P.sbox) return launch_nodal_box<NPE, kBoxSpec>(P, M, vol, st, c);
+  }
+  launch_nodal_box<NPE, kBoxNone>(P, M, vol, st, c);
 }
 
-template <int NPE, int LAW, bool TH, bool BOX>
+template <int NPE, int LAW, bool TH, int BOX>
 void launch_elements_box(const StepParams &P, const MixState &M, cudaStream_t st, LaunchCfg c) {
   switch (c.bs) {
     case 64: {
@@ -3115,12 +3139,10 @@ void launch_elements_box(const StepParams &P, const MixState &M, cudaStream_t st
 template <int NPE, int LAW, bool TH>
 void launch_elements_law(const StepParams &P, const MixState &M, cudaStream_t st, LaunchCfg c) {
   if constexpr (NPE == 8 && !TH) {
-    if (P.box) {
-      launch_elements_box<NPE, LAW, TH, true>(P, M, st, c);
-      return;
-    }
+    if (P.box) return launch_elements_box<NPE, LAW, TH, kBoxOne>(P, M, st, c);
+    if (P.sbox) return launch_elements_box<NPE, LAW, TH, kBoxSpec>(P, M, st, c);
   }
-  launch_elements_box<NPE, LAW, TH, false>(P, M, st, c);
+  launch_elements_box<NPE, LAW, TH, kBoxNone>(P, M, st, c);
 }
 
 template <int NPE>
@@ -3259,11 +3281,13 @@ void mix_elements(const StepParams &P, const MixState &M, const float *, cudaStr
 
 void mix_nodes(const StepParams &P, const MixState &M, cudaStream_t st, int node_grid) {
   if (P.npe == 8 && P.box)
-    k_mix_nodes<8, true><<<node_grid, kNodeThreads, 0, st>>>(P, M);
+    k_mix_nodes<8, kBoxOne><<<node_grid, kNodeThreads, 0, st>>>(P, M);
+  else if (P.npe == 8 && P.sbox)
+    k_mix_nodes<8, kBoxSpec><<<node_grid, kNodeThreads, 0, st>>>(P, M);
   else if (P.npe == 8)
-    k_mix_nodes<8, false><<<node_grid, kNodeThreads, 0, st>>>(P, M);
+    k_mix_nodes<8, kBoxNone><<<node_grid, kNodeThreads, 0, st>>>(P, M);
   else
-    k_mix_nodes<4, false><<<node_grid, kNodeThreads, 0, st>>>(P, M);
+    k_mix_nodes<4, kBoxNone><<<node_grid, kNodeThreads, 0, st>>>(P, M);
 }
 
 static_assert(kSharedThreads == kNodeThreads, "the shared-node kernel runs node-kernel blocks");

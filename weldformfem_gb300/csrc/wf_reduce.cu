@@ -192,6 +192,17 @@ void energy_mixed(const StepParams &P, const MixState &M, cudaStream_t st) {
   k_energy_mixed<<<energy_grid(P), kThreads, 0, st>>>(P, M);
 }
 
+namespace {
+__global__ void k_copy_column(const double *src, int64_t stride, int64_t n, double *dst) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) dst[i] = src[i * stride];
+}
+}  // namespace
+
+void copy_column(const double *src, int64_t stride, int64_t n, double *dst, cudaStream_t st) {
+  if (n > 0) k_copy_column<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(src, stride, n, dst);
+}
+
 void spec_reaction(const StepParams &P, cudaStream_t st) {
   k_spec_reaction<<<P.nspec, 128, 0, st>>>(P);
 }

@@ -402,6 +402,24 @@ void scatter_u32(uint32_t *dst, const int32_t *idx, const uint32_t *val, int64_t
   if (n > 0) k_scatter_u32<<<grid_for(n), kThreads, 0, st>>>(dst, idx, val, n);
 }
 
+namespace {
+__global__ void k_fill_owner(const int64_t *off, int parts, int64_t n, uint16_t *dst) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int lo = 0, hi = parts - 1;   // the last part that starts at or before i
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (off[mid] <= i) lo = mid;
+    else hi = mid - 1;
+  }
+  dst[i] = (uint16_t)lo;
+}
+}  // namespace
+
+void fill_owner(const int64_t *off, int parts, int64_t n, uint16_t *dst, cudaStream_t st) {
+  if (n > 0) k_fill_owner<<<grid_for(n), kThreads, 0, st>>>(off, parts, n, dst);
+}
+
 void or_flags(uint8_t *dst, const int32_t *idx, uint8_t bit, int64_t n, cudaStream_t st) {
   if (n > 0) k_or_u8<<<grid_for(n), kThreads, 0, st>>>(dst, idx, bit, n);
 }
@@ -423,14 +441,12 @@ cudaError_t check_connectivity(const int32_t *el, int64_t n, int64_t nn, int32_t
 }
 
 cudaError_t check_box(const int32_t *el_soa, int64_t ne, int64_t nn, int nx, int ny, int nz,
-                      cudaStream_t st, int *is_box) {
+                      int32_t *err, cudaStream_t st, int *is_box) {
   *is_box = 0;
   if (nx <= 0 || ny <= 0 || nz <= 0 || (int64_t)nx * ny * nz != ne ||
       (int64_t)(nx + 1) * (ny + 1) * (nz + 1) != nn)
     return cudaSuccess;
-  int32_t *err = nullptr;
-  cudaError_t e = cudaMalloc(&err, sizeof(int32_t));
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   int32_t herr = 1;
   if ((e = cudaMemsetAsync(err, 0, sizeof(int32_t), st)) == cudaSuccess) {
     k_box_check<<<grid_for(ne), kThreads, 0, st>>>(el_soa, ne, nx, ny, err);
@@ -438,8 +454,38 @@ cudaError_t check_box(const int32_t *el_soa, int64_t ne, int64_t nn, int nx, int
         cudaSuccess)
       e = cudaStreamSynchronize(st);
   }
-  cudaFree(err);
   if (e == cudaSuccess && herr == 0) *is_box = 1;
+  return e;
+}
+
+namespace {
+__global__ void k_spec_box_check(const int32_t *el, int64_t ne, const uint16_t *espec,
+                                 const SpecBox *sbox, int32_t *err) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= ne) return;
+  const SpecBox &s = sbox[espec[e]];
+  const int32_t q = (int32_t)(e - s.e0), i = q % s.bx, j = q / s.bx % s.by, k = q / (s.bx * s.by);
+  const int32_t px = s.bx + 1, pxy = px * (s.by + 1), n0 = s.n0 + i + px * j + pxy * k;
+  const int32_t c[8] = {n0, n0 + 1, n0 + 1 + px, n0 + px, n0 + pxy, n0 + 1 + pxy, n0 + 1 + px + pxy,
+                        n0 + px + pxy};
+  bool ok = k < s.bz;
+  for (int a = 0; a < 8; a++) ok = ok && el[a * ne + e] == c[a];
+  if (!ok) *err = 1;
+}
+}  // namespace
+
+cudaError_t check_spec_boxes(const int32_t *el_soa, int64_t ne, const uint16_t *espec,
+                             const SpecBox *sbox, int32_t *err, cudaStream_t st, int *all) {
+  *all = 0;
+  int32_t herr = 1;
+  cudaError_t e = cudaSuccess;
+  if ((e = cudaMemsetAsync(err, 0, sizeof(int32_t), st)) == cudaSuccess) {
+    k_spec_box_check<<<grid_for(ne), kThreads, 0, st>>>(el_soa, ne, espec, sbox, err);
+    if ((e = cudaMemcpyAsync(&herr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, st)) ==
+        cudaSuccess)
+      e = cudaStreamSynchronize(st);
+  }
+  if (e == cudaSuccess && herr == 0) *all = 1;
   return e;
 }
 
