@@ -278,7 +278,7 @@ struct wf_domain {
   std::vector<int64_t> spec_eoff, spec_noff;
   std::vector<double> spec_dt;
   // adjoint recording: checkpoints of the forward run and reverse-pass buffers
-  std::vector<void *> adj_allocs;
+  std::vector<void *> adj_allocs, adj_pooled;  // see adj_alloc
   int64_t adj_steps = 0, adj_every = 0, adj_first = 0;
   bool adj_store_all = false;     // every step stashed in the forward, no recompute
   int64_t adj_nck = 0;
@@ -382,7 +382,9 @@ cudaError_t dalloc(wf_domain *d, T **p, size_t count) {
 }
 
 void free_adjoint(wf_domain *d) {
+  for (void *p : d->adj_pooled) cudaFreeAsync(p, d->stream);
   for (void *p : d->adj_allocs) cudaFree(p);
+  d->adj_pooled.clear();
   d->adj_allocs.clear();
   d->adj_steps = d->adj_every = d->adj_nck = 0;
   d->adj_store_all = false;
@@ -402,8 +404,6 @@ void free_device(wf_domain *d) {
   if (d->out_stream) cudaStreamSynchronize(d->out_stream);
   for (void *p : d->allocs) cudaFreeAsync(p, d->stream);
   d->allocs.clear();
-  if (d->st_host) cudaFreeHost(d->st_host);
-  d->st_host = nullptr;
   d->st_pending = false;
   for (auto &sn : d->snap) {
     if (sn.dev) cudaFree(sn.dev);
@@ -854,6 +854,7 @@ WF_API wf_status wf_domain_destroy(wf_domain *d) {
   if (d->out_stream) cudaStreamSynchronize(d->out_stream);
   free_device(d);
   free_mesh_dev(d);
+  if (d->st_host) cudaFreeHost(d->st_host);
   if (d->stream) cudaStreamDestroy(d->stream);
   if (d->out_stream) cudaStreamDestroy(d->out_stream);
   for (cudaEvent_t ev : d->side_ev)
@@ -2293,7 +2294,7 @@ WF_API wf_status wf_init(wf_domain *d) {
   if (d->nspec) CUDA_TRY(dalloc(d, &P.hist_spec, (size_t)d->hist_cap * d->nspec));
   P.hist_cap = d->hist_cap;
   CUDA_TRY(dalloc(d, &P.st, 1));
-  CUDA_TRY(cudaMallocHost(&d->st_host, sizeof(StepState)));
+  if (!d->st_host) CUDA_TRY(cudaMallocHost(&d->st_host, sizeof(StepState)));
   *d->st_host = StepState{};
   d->st_host->first_bad_node = LLONG_MAX;
   CUDA_TRY(cudaMemcpyAsync(&P.st->first_bad_node, &d->st_host->first_bad_node, sizeof(long long),
@@ -3719,12 +3720,20 @@ WF_API wf_status wf_get_transfer_bytes(const wf_domain *d, int64_t *h2d, int64_t
 // ---- adjoint ----------------------------------------------------------------------
 namespace {
 
+// The recording's arrays up to this size come from the device pool, larger
+// ones from the driver: a call that records and reverses 64 steps of a 32^3
+// block made 19 of the driver's allocations and as many frees, each of which
+// also waits for the device; what the pool keeps afterwards stays bounded.
+constexpr size_t kAdjPooledBytes = size_t(64) << 20;
+
 template <typename T>
 cudaError_t adj_alloc(wf_domain *d, T **p, size_t count) {
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  const bool pooled = bytes <= kAdjPooledBytes;
   void *q = nullptr;
-  cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
+  cudaError_t e = pooled ? pool_alloc(d, &q, bytes) : cudaMalloc(&q, bytes);
   if (e != cudaSuccess) return e;
-  d->adj_allocs.push_back(q);
+  (pooled ? d->adj_pooled : d->adj_allocs).push_back(q);
   *p = static_cast<T *>(q);
   return cudaMemsetAsync(q, 0, std::max<size_t>(count, 1) * sizeof(T), d->stream);
 }
