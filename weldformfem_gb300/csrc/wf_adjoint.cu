@@ -15,18 +15,21 @@
 //                             derivative), pressure -K (J_avg - 1), the
 //                             reference's Jaumann terms, D/W, dN/dx and J
 //                             -> per element-node contributions
-//   k_adj_gather   (node)   : gathers those contributions over the node's
-//                             element list (deterministic, no atomics), the
-//                             predictor v_pred = v + (1-gamma) dt a_prev, and
-//                             the adjoint of the nodal volume sum
-//   k_adj_volume   (element): volume -> detJ -> J -> x contributions, gathered
-//                             by the next reverse step's node kernel.
+//   k_adj_gather   (node)   : gathers the velocity and J ratio contributions
+//                             over the node's element list (deterministic, no
+//                             atomics), the predictor v_pred = v + (1-gamma)
+//                             dt a_prev, and the adjoint of the nodal volume
+//                             sum
+//   k_adj_volume   (element): volume -> detJ -> J, added to the element
+//                             kernel's J -> x contributions, gathered by the
+//                             next reverse step's node kernel.
 // Material gradients accumulate per element and are summed per material on
 // the host in element order. The element kernel is templated on the scalar
 // type of its arithmetic (FP64, or FP32 for the reduced-precision adjoint).
 #include <vector>
 
 #include "wf_adjoint.cuh"
+#include "wf_hex.cuh"
 
 namespace wf {
 namespace {
@@ -121,20 +124,37 @@ __device__ __forceinline__ void adj_reverse(const T J[3][3], const T Ab[3][3], T
 
 // ---------------------------------------------------------------------------
 // Reverse of the node phase of step s.
+// The gathers here and in k_adj_gather keep eight entries' loads in flight and
+// add them in list order.
+template <int NPE, int NF>
+__device__ __forceinline__ void gather_entry(const double *f, int64_t ne, int32_t sl,
+                                             double (&g)[NF]) {
+#pragma unroll
+  for (int k = 0; k < NF; k++)
+    g[k] = sl >= 0 ? __ldg(&f[(int64_t)((sl % NPE) * 3 + k) * ne + sl / NPE]) : 0.0;
+}
+
+template <int NPE>
 __global__ void k_adj_nodes(StepParams P, AdjArgs A, int s, long long gstep, int have_geo) {
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= P.nn) return;
   const int64_t np = P.np, ne = P.ne;
-  const int npe = P.npe;
   double xb[3];
   for (int k = 0; k < 3; k++) xb[k] = A.X[k * np + n];
   if (have_geo) {
-    // geometry contributions of the step after this one, in list order
+    // position contributions of the step after this one, in list order
     const int32_t b = P.off[n], c = P.off[n + 1] - b;
-    for (int32_t q = 0; q < c; q++) {
-      const int32_t sl = P.slot[b + q];
-      const int64_t e = sl / npe, loc = sl % npe;
-      for (int k = 0; k < 3; k++) xb[k] += A.cgeo[(loc * 3 + k) * ne + e];
+    for (int32_t q0 = 0; q0 < c; q0 += 8) {
+      int32_t sl[8];
+      double g[8][3];
+#pragma unroll
+      for (int j = 0; j < 8; j++) sl[j] = (q0 + j < c) ? __ldg(&P.slot[b + q0 + j]) : -1;
+#pragma unroll
+      for (int j = 0; j < 8; j++) gather_entry<NPE, 3>(A.cgeo, ne, sl[j], g[j]);
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+        if (sl[j] >= 0)
+          for (int k = 0; k < 3; k++) xb[k] += g[j][k];
     }
   }
   const double dt = P.dt;
@@ -166,8 +186,8 @@ __global__ void __launch_bounds__(kThreads) k_adj_elements(StepParams P, AdjArgs
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= P.ne) return;
   const int64_t np = P.np, ne = P.ne;
-  const double *sx = A.sx + (int64_t)s * 3 * np, *sv = A.sv + (int64_t)s * 3 * np;
-  const double *spa = A.spa + (int64_t)s * 3 * np, *sjr = A.sjr + (int64_t)s * np;
+  const double *sx = A.sx + (int64_t)s * 3 * np, *svp = A.svp + (int64_t)s * 3 * np;
+  const double *sjr = A.sjr + (int64_t)s * np;
   const double *stau = A.stau + (int64_t)s * 6 * ne, *spls = A.spls + (int64_t)s * ne;
   const double dt_d = P.dt;
   const T dt = (T)dt_d;
@@ -175,12 +195,9 @@ __global__ void __launch_bounds__(kThreads) k_adj_elements(StepParams P, AdjArgs
   T x[NPE][3], vp[NPE][3];
   for (int a = 0; a < NPE; a++) {
     nid[a] = P.elnod[a * ne + e];
-    const uint32_t code = P.bc[nid[a]];
     for (int k = 0; k < 3; k++) {
       x[a][k] = (T)sx[k * np + nid[a]];
-      double v = sv[k * np + nid[a]] + (1.0 - P.gamma) * dt_d * spa[k * np + nid[a]];
-      if ((code >> k) & 1u) v = P.bcval[3 * (code >> 3) + k];
-      vp[a][k] = (T)v;
+      vp[a][k] = (T)svp[k * np + nid[a]];
     }
   }
   const MatDev m = P.mats[P.emat ? P.emat[e] : 0];
@@ -433,293 +450,280 @@ __global__ void __launch_bounds__(kThreads) k_adj_elements(StepParams P, AdjArgs
   A.gth[2 * ne + e] += (double)Hb;
 }
 
-// Walsh transform over the hexahedron's corners and its transpose (node a at
-// the signs of (xi, eta, zeta) of the AddBoxLength numbering): o = sums of v
-// weighted by {1, xi, eta, zeta, eta zeta, xi zeta, xi eta, xi eta zeta};
-// the synthesis returns the node values of sum_b o[b] phi_b for b = 1..7.
-template <typename T>
-__device__ __forceinline__ void walsh8t(const T (&v)[8], T (&o)[8]) {
-  const T a0 = v[1] + v[0], b0 = v[1] - v[0], a1 = v[2] + v[3], b1 = v[2] - v[3];
-  const T a2 = v[5] + v[4], b2 = v[5] - v[4], a3 = v[6] + v[7], b3 = v[6] - v[7];
-  const T c0 = a1 + a0, d0 = a1 - a0, e0 = b1 + b0, f0 = b1 - b0;
-  const T c1 = a3 + a2, d1 = a3 - a2, e1 = b3 + b2, f1 = b3 - b2;
-  o[0] = c1 + c0; o[3] = c1 - c0; o[2] = d1 + d0; o[4] = d1 - d0;
-  o[1] = e1 + e0; o[5] = e1 - e0; o[6] = f1 + f0; o[7] = f1 - f0;
-}
-template <typename T>
-__device__ __forceinline__ void walsh8t_synth(const T (&o)[8], T (&v)[8]) {
-  const T c1 = o[3], c0 = -o[3];
-  const T d1 = o[2] + o[4], d0 = o[2] - o[4], e1 = o[1] + o[5], e0 = o[1] - o[5];
-  const T f1 = o[6] + o[7], f0 = o[6] - o[7];
-  const T a1 = c0 + d0, a0 = c0 - d0, b1 = e0 + f0, b0 = e0 - f0;
-  const T a3 = c1 + d1, a2 = c1 - d1, b3 = e1 + f1, b2 = e1 - f1;
-  v[1] = a0 + b0; v[0] = a0 - b0; v[2] = a1 + b1; v[3] = a1 - b1;
-  v[5] = a2 + b2; v[4] = a2 - b2; v[6] = a3 + b3; v[7] = a3 - b3;
-}
-
-// Reverse of the element phase of step s for hexahedra, in the Walsh form:
-// J = W(x)/8, the velocity gradient adj(J) W(v) / (8 detJ), the forces the
-// synthesis of adj(J)^T sigma and of the hourglass terms ch h_j (the same
-// quantities as the per-node formulation of the forward kernel). Outputs as
-// k_adj_elements. Coordinates enter relative to the element's first node.
+// Reverse of the element phase of step s for hexahedra, in the Walsh form of the
+// forward kernel: X = W(x) = 8 J, D = det X = 64 vol, the velocity gradient
+// adj(X) W(v) / D, the forces the synthesis of adj(X)^T sigma / 64 and of the
+// hourglass terms ch h_j. Outputs as k_adj_elements, but the adjoint of X and
+// adj(X) in cx: k_adj_volume adds the volume's part before the one synthesis to
+// the corners.
+// Bound by the FP64 rate (one warp instruction per SM quarter every 64 cycles,
+// whatever the lanes do), so by its FP64 instructions: every quotient is a
+// product with one of three reciprocals (1 / D, 1 / seq, and per material), the
+// predicted velocities come from the stash with their boundary values, and the
+// hourglass power is the forward step's.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_adj_hex(StepParams P, AdjArgs A, int s) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= P.ne) return;
   const int64_t np = P.np, ne = P.ne;
-  const double *sx = A.sx + (int64_t)s * 3 * np, *sv = A.sv + (int64_t)s * 3 * np;
-  const double *spa = A.spa + (int64_t)s * 3 * np, *sjr = A.sjr + (int64_t)s * np;
+  const double *sx = A.sx + (int64_t)s * 3 * np, *svp = A.svp + (int64_t)s * 3 * np;
+  const double *sjr = A.sjr + (int64_t)s * np;
   const double *stau = A.stau + (int64_t)s * 6 * ne, *spls = A.spls + (int64_t)s * ne;
-  const double dt_d = P.dt;
-  const T dt = (T)dt_d;
+  const T dt = (T)P.dt;
   int32_t nid[8];
-  for (int a = 0; a < 8; a++) nid[a] = P.elnod[a * ne + e];
-  // Jacobian from relative coordinates
-  T J[3][3];
-  for (int k = 0; k < 3; k++) {
-    const double x0 = sx[k * np + nid[0]];
-    T v[8], o[8];
-    for (int a = 0; a < 8; a++) v[a] = (T)(sx[k * np + nid[a]] - x0);
-    walsh8t(v, o);
-    for (int mm = 0; mm < 3; mm++) J[mm][k] = (T)0.125 * o[1 + mm];
-  }
-  T Am[3][3];  // adj(J): Am[k][m] = cofactor[m][k]
-  Am[0][0] = (J[1][1] * J[2][2] - J[1][2] * J[2][1]);
-  Am[1][0] = -(J[1][0] * J[2][2] - J[1][2] * J[2][0]);
-  Am[2][0] = (J[1][0] * J[2][1] - J[1][1] * J[2][0]);
-  Am[0][1] = -(J[0][1] * J[2][2] - J[0][2] * J[2][1]);
-  Am[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]);
-  Am[2][1] = -(J[0][0] * J[2][1] - J[0][1] * J[2][0]);
-  Am[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]);
-  Am[1][2] = -(J[0][0] * J[1][2] - J[0][2] * J[1][0]);
-  Am[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]);
-  const T detJ = J[0][0] * Am[0][0] + J[0][1] * Am[1][0] + J[0][2] * Am[2][0];
-  const T vol = detJ * (T)8;
-  // predicted velocities: Walsh sums G (derivative directions) and hm (hourglass)
-  T G[3][3], hm[3][4];
-  for (int k = 0; k < 3; k++) {
-    T v[8], o[8];
-    for (int a = 0; a < 8; a++) {
-      const uint32_t code = P.bc[nid[a]];
-      double vv = sv[k * np + nid[a]] + (1.0 - P.gamma) * dt_d * spa[k * np + nid[a]];
-      if ((code >> k) & 1u) vv = P.bcval[3 * (code >> 3) + k];
-      v[a] = (T)vv;
+#pragma unroll
+  for (int a = 0; a < 8; a++) nid[a] = __ldg(&P.elnod[a * ne + e]);
+  T X[3][3], Am[3][3];   // 8 J and its adjugate
+  {
+    T x[8][3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      // FP32: relative to the first corner before the rounding
+      const double x0 = sizeof(T) == 8 ? 0.0 : __ldg(&sx[k * np + nid[0]]);
+#pragma unroll
+      for (int a = 0; a < 8; a++) {
+        const double v = __ldg(&sx[k * np + nid[a]]);
+        x[a][k] = sizeof(T) == 8 ? (T)v : (T)(v - x0);
+      }
     }
-    walsh8t(v, o);
+    corner_sums(x, X);
+  }
+  const T D = adjugate8(X, Am);
+  const T r = (T)1 / D;
+  T G[3][3], hm[3][4];   // Walsh sums of the predicted velocities
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    T v[8], o[8];
+#pragma unroll
+    for (int a = 0; a < 8; a++) v[a] = (T)__ldg(&svp[k * np + nid[a]]);
+    walsh8d(v, o);
+#pragma unroll
     for (int mm = 0; mm < 3; mm++) G[mm][k] = o[1 + mm];
+#pragma unroll
     for (int j = 0; j < 4; j++) hm[k][j] = o[4 + j];
   }
-  const MatDev m = P.mats[P.emat ? P.emat[e] : 0];
-  const T K = (T)m.K, Gm = (T)m.G, H = (T)m.H, sy0 = (T)m.sy0;
-  const T fl = (T)0.125 / detJ;
+  const MatDev &m = P.mats[P.emat ? __ldg(&P.emat[e]) : 0];
+  const T K = (T)m.K, Gm = (T)m.G, H = (T)m.H, sy0 = (T)m.sy0, i3GH = (T)m.i3GH;
   T L[3][3];
+#pragma unroll
   for (int i = 0; i < 3; i++)
+#pragma unroll
     for (int k = 0; k < 3; k++)
-      L[i][k] = fl * (Am[i][0] * G[0][k] + Am[i][1] * G[1][k] + Am[i][2] * G[2][k]);
-  const T D[6] = {L[0][0], L[1][1], L[2][2], (T)0.5 * (L[1][0] + L[0][1]),
-                  (T)0.5 * (L[2][1] + L[1][2]), (T)0.5 * (L[2][0] + L[0][2])};
+      L[i][k] = r * fma(Am[i][2], G[2][k], fma(Am[i][1], G[1][k], Am[i][0] * G[0][k]));
   const T w01 = (T)0.5 * (L[1][0] - L[0][1]);
   const T w12 = (T)0.5 * (L[2][1] - L[1][2]);
   const T w02 = (T)0.5 * (L[2][0] - L[0][2]);
   T Javg = 0;
-  for (int a = 0; a < 8; a++) Javg += (T)sjr[nid[a]];
-  Javg /= (T)8;
-  const T p = -K * (Javg - (T)1);
+#pragma unroll
+  for (int a = 0; a < 8; a++) Javg += (T)__ldg(&sjr[nid[a]]);
+  const T dJ = fma(Javg, (T)0.125, (T)-1);
+  const T p = -K * dJ;
   T t[6];
-  for (int c = 0; c < 6; c++) t[c] = (T)stau[c * ne + e];
-  const T epl = (T)spls[e];
-  T Q[6];
-  Q[0] = (T)2 * (t[3] * w01 + t[5] * w02);
-  Q[1] = 0;
-  Q[2] = 0;
-  Q[3] = w01 * (t[0] + t[1]) - t[5] * w12 + w02 * t[4];
-  Q[4] = t[3] * w02 + w12 * (t[1] + t[2]) - w01 * t[5];
-  Q[5] = w02 * (t[0] + t[2]) + t[3] * w12 + w01 * t[4];
-  const T c3 = (D[0] + D[1] + D[2]) / (T)3;
-  const T Dd[6] = {D[0] - c3, D[1] - c3, D[2] - c3, D[3], D[4], D[5]};
-  T ts[6];
-  for (int c = 0; c < 6; c++) ts[c] = t[c] + dt * ((T)2 * Gm * Dd[c] + Q[c]);
-  const T tr3 = (ts[0] + ts[1] + ts[2]) / (T)3;
-  const T sdev[6] = {ts[0] - tr3, ts[1] - tr3, ts[2] - tr3, ts[3], ts[4], ts[5]};
-  const T J2 = (T)0.5 * (sdev[0] * sdev[0] + sdev[1] * sdev[1] + sdev[2] * sdev[2] +
-                         (T)2 * (sdev[3] * sdev[3] + sdev[4] * sdev[4] + sdev[5] * sdev[5]));
-  const T seq = sqrt((T)3 * J2);
-  const T sy = sy0 + H * epl;
+#pragma unroll
+  for (int c = 0; c < 6; c++) t[c] = (T)__ldg(&stau[c * ne + e]);
+  const T epl = (T)__ldg(&spls[e]);
+  const T t01 = t[0] + t[1], t12 = t[1] + t[2], t02 = t[0] + t[2];
+  const T q0 = (T)2 * fma(t[5], w02, t[3] * w01);
+  const T q3 = fma(w02, t[4], fma(-t[5], w12, w01 * t01));
+  const T q4 = fma(-w01, t[5], fma(w12, t12, t[3] * w02));
+  const T q5 = fma(w01, t[4], fma(t[3], w12, w02 * t02));
+  constexpr T third = (T)(1.0 / 3.0);
+  // the trial stress's deviator; the mean of the strain rate leaves it, and is
+  // needed for the elastic trial stress alone
+  const T c3 = third * (L[0][0] + L[1][1] + L[2][2]);
+  const T Dd[6] = {L[0][0] - c3, L[1][1] - c3, L[2][2] - c3, (T)0.5 * (L[1][0] + L[0][1]),
+                   (T)0.5 * (L[2][1] + L[1][2]), (T)0.5 * (L[2][0] + L[0][2])};
+  const T gdt = (T)2 * Gm * dt;
+  const T ts[6] = {fma(dt, q0, fma(gdt, Dd[0], t[0])), fma(gdt, Dd[1], t[1]), fma(gdt, Dd[2], t[2]),
+                   fma(dt, q3, fma(gdt, Dd[3], t[3])), fma(dt, q4, fma(gdt, Dd[4], t[4])),
+                   fma(dt, q5, fma(gdt, Dd[5], t[5]))};
+  const T tr3 = third * (ts[0] + ts[1] + ts[2]);
+  const T sd[6] = {ts[0] - tr3, ts[1] - tr3, ts[2] - tr3, ts[3], ts[4], ts[5]};
+  // seq^2 = 3 J2
+  const T nd = fma(sd[2], sd[2], fma(sd[1], sd[1], sd[0] * sd[0]));
+  const T ns = fma(sd[5], sd[5], fma(sd[4], sd[4], sd[3] * sd[3]));
+  const T seq = sqrt(fma((T)3, ns, (T)1.5 * nd));
+  const T sy = fma(H, epl, sy0);
   const bool plastic = sy < seq;
-  T tn[6], dgam = 0, fac = 1;
+  T tn[6], dgam = 0, a3 = 0, rs = 0;
   if (plastic) {
-    dgam = (seq - sy) / ((T)3 * Gm + H);
-    fac = (T)1 - (T)3 * Gm * dgam / seq;
-    for (int c = 0; c < 6; c++) tn[c] = sdev[c] * fac;
+    rs = (T)1 / seq;
+    dgam = (seq - sy) * i3GH;
+    a3 = (T)3 * Gm * dgam * rs;
+#pragma unroll
+    for (int c = 0; c < 6; c++) tn[c] = sd[c] * ((T)1 - a3);
   } else {
+#pragma unroll
     for (int c = 0; c < 6; c++) tn[c] = ts[c];
   }
   const T S[3][3] = {{tn[0] - p, tn[3], tn[5]}, {tn[3], tn[1] - p, tn[4]}, {tn[5], tn[4], tn[2] - p}};
-  const T ch = P.hg_on ? (T)P.hg_coef * pow(vol, (T)0.6666666) * (T)A.rho[e] * (T)0.25 * (T)m.cs0
-                       : (T)0;
+  T ch = 0;
+  if (P.hg_on) {
+    T pw;
+    if constexpr (sizeof(T) == 8) pw = pow_two_thirds(D * (1.0 / 64.0));
+    else pw = pow(D * (T)(1.0 / 64.0), (T)0.6666666);
+    ch = (T)P.hg_coef * pw * (T)__ldg(&A.rho[e]) * (T)0.25 * (T)m.cs0;
+  }
 
   // ---- reverse ------------------------------------------------------------
-  // forces: f = synth(T, ch hm) with T = adj(J)^T S; the transpose is W(fb)
-  T Tb[3][3], hmb[3][4];
-  T chb = 0;
+  // forces: f = synth(adj(X)^T S / 64, ch hm); the transpose is W(fb)
+  T Tb[3][3], hmb[3][4], chb = 0;
+#pragma unroll
   for (int k = 0; k < 3; k++) {
     T v[8], o[8];
-    for (int a = 0; a < 8; a++) v[a] = (T)A.fib[k * np + nid[a]];
-    walsh8t(v, o);
-    for (int mm = 0; mm < 3; mm++) Tb[mm][k] = o[1 + mm];
+#pragma unroll
+    for (int a = 0; a < 8; a++) v[a] = (T)__ldg(&A.fib[k * np + nid[a]]);
+    walsh8d(v, o);
+#pragma unroll
+    for (int mm = 0; mm < 3; mm++) Tb[mm][k] = o[1 + mm] * (T)(1.0 / 64.0);
+#pragma unroll
     for (int j = 0; j < 4; j++) {
-      chb += o[4 + j] * hm[k][j];
+      chb = fma(o[4 + j], hm[k][j], chb);
       hmb[k][j] = ch * o[4 + j];
     }
   }
-  T Ab[3][3];
-  T Sb[3][3];
+  T Ab[3][3], Sb[3][3];
+#pragma unroll
   for (int i = 0; i < 3; i++)
-    for (int mm = 0; mm < 3; mm++) {
-      T acc = 0;
-      for (int k = 0; k < 3; k++) acc += S[i][k] * Tb[mm][k];
-      Ab[i][mm] = acc;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      Ab[i][k] = fma(S[i][2], Tb[k][2], fma(S[i][1], Tb[k][1], S[i][0] * Tb[k][0]));
+      Sb[i][k] = fma(Am[i][2], Tb[2][k], fma(Am[i][1], Tb[1][k], Am[i][0] * Tb[0][k]));
     }
-  for (int i = 0; i < 3; i++)
-    for (int k = 0; k < 3; k++)
-      Sb[i][k] = Am[i][0] * Tb[0][k] + Am[i][1] * Tb[1][k] + Am[i][2] * Tb[2][k];
-  T sigb[6] = {Sb[0][0], Sb[1][1], Sb[2][2], Sb[0][1] + Sb[1][0], Sb[1][2] + Sb[2][1],
-               Sb[0][2] + Sb[2][0]};
-  T volb = 0, Kb = 0, Gb = 0, Hb = 0, sy0b = 0;
-  if (P.hg_on) {
-    volb += chb * ch * (T)0.6666666 / vol;
-    Kb += chb * ch * (T)0.5 / K;  // cs0 = sqrt(K / rho)
-  }
-  // sigma = tau_new - p I
+  const T sigb[6] = {Sb[0][0], Sb[1][1], Sb[2][2], Sb[0][1] + Sb[1][0], Sb[1][2] + Sb[2][1],
+                     Sb[0][2] + Sb[2][0]};
+  // E enters K, G (both proportional to it) and cs0 = sqrt(K / rho):
+  // E dL/dE = K Kb + G Gb + chb ch / 2
+  const T cc = chb * ch;
+  const T volb = cc * (T)(0.6666666 * 64.0) * r;
   T tnb[6];
+#pragma unroll
   for (int c = 0; c < 6; c++) tnb[c] = sigb[c] + (T)A.T[c * ne + e];
   const T pb = -(sigb[0] + sigb[1] + sigb[2]);
   T eplb = (T)A.EP[e];
+  T Gb = 0, Hb = 0, sy0b = 0;
   T tsb[6];
   if (plastic) {
     T facb = 0;
-    T sdb[6];
-    for (int c = 0; c < 6; c++) {
-      facb += tnb[c] * sdev[c];
-      sdb[c] = tnb[c] * fac;
-    }
-    const T den = (T)3 * Gm + H;
-    const T dgb = eplb + facb * (-(T)3 * Gm / seq);
-    const T seqb = facb * ((T)3 * Gm * dgam / (seq * seq)) + dgb / den;
-    const T syb = -dgb / den;
-    Gb += facb * (-(T)3 * dgam / seq) + dgb * (-(T)3 * (seq - sy) / (den * den));
-    Hb += dgb * (-(seq - sy) / (den * den)) + syb * epl;
-    sy0b += syb;
-    eplb = eplb + syb * H;
-    const T q = (T)1.5 / seq * seqb;
-    for (int c = 0; c < 3; c++) sdb[c] += q * sdev[c];
-    for (int c = 3; c < 6; c++) sdb[c] += q * (T)2 * sdev[c];
-    const T mean = (sdb[0] + sdb[1] + sdb[2]) / (T)3;
-    for (int c = 0; c < 3; c++) tsb[c] = sdb[c] - mean;
-    for (int c = 3; c < 6; c++) tsb[c] = sdb[c];
+#pragma unroll
+    for (int c = 0; c < 6; c++) facb = fma(tnb[c], sd[c], facb);
+    const T u = facb * rs;
+    const T dgb = fma((T)-3 * Gm, u, eplb);
+    const T di = dgb * i3GH;
+    const T seqb = fma(u, a3, di);
+    sy0b = -di;
+    Gb = (T)-3 * dgam * (u + di);
+    Hb = sy0b * (dgam + epl);   // dgamma's denominator, and sigma_y = sy0 + H eps_p
+    eplb = fma(sy0b, H, eplb);
+    const T q = (T)1.5 * rs * seqb;
+#pragma unroll
+    for (int c = 0; c < 6; c++)
+      tsb[c] = fma(c < 3 ? q : (T)2 * q, sd[c], tnb[c] * ((T)1 - a3));
+    const T mean = third * (tsb[0] + tsb[1] + tsb[2]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) tsb[c] -= mean;
   } else {
+#pragma unroll
     for (int c = 0; c < 6; c++) tsb[c] = tnb[c];
   }
-  const T Javgb = -K * pb;
-  Kb += -(Javg - (T)1) * pb;
-  T tb[6], Qb[6], Ddb[6];
-  for (int c = 0; c < 6; c++) {
-    tb[c] = tsb[c];
-    Qb[c] = dt * tsb[c];
-    Ddb[c] = dt * (T)2 * Gm * tsb[c];
-    Gb += dt * (T)2 * Dd[c] * tsb[c];
-  }
-  T w01b = 0, w12b = 0, w02b = 0;
-  tb[3] += Qb[0] * (T)2 * w01; tb[5] += Qb[0] * (T)2 * w02;
-  w01b += Qb[0] * (T)2 * t[3]; w02b += Qb[0] * (T)2 * t[5];
-  tb[0] += Qb[3] * w01; tb[1] += Qb[3] * w01; tb[5] -= Qb[3] * w12; tb[4] += Qb[3] * w02;
-  w01b += Qb[3] * (t[0] + t[1]); w12b -= Qb[3] * t[5]; w02b += Qb[3] * t[4];
-  tb[3] += Qb[4] * w02; tb[1] += Qb[4] * w12; tb[2] += Qb[4] * w12; tb[5] -= Qb[4] * w01;
-  w02b += Qb[4] * t[3]; w12b += Qb[4] * (t[1] + t[2]); w01b -= Qb[4] * t[5];
-  tb[0] += Qb[5] * w02; tb[2] += Qb[5] * w02; tb[3] += Qb[5] * w12; tb[4] += Qb[5] * w01;
-  w02b += Qb[5] * (t[0] + t[2]); w12b += Qb[5] * t[3]; w01b += Qb[5] * t[4];
-  T Db[6];
+  // Jaumann terms: ts = t + dt (2 G Dd + Q(t, W))
   {
-    const T mean = (Ddb[0] + Ddb[1] + Ddb[2]) / (T)3;
-    for (int c = 0; c < 3; c++) Db[c] = Ddb[c] - mean;
-    for (int c = 3; c < 6; c++) Db[c] = Ddb[c];
+    T sum = 0;
+#pragma unroll
+    for (int c = 0; c < 6; c++) sum = fma(Dd[c], tsb[c], sum);
+    Gb = fma((T)2 * dt, sum, Gb);
   }
-  // D, W from the velocity gradient L
-  T Lb[3][3] = {{Db[0], 0, 0}, {0, Db[1], 0}, {0, 0, Db[2]}};
-  Lb[1][0] += (T)0.5 * (Db[3] + w01b);
-  Lb[0][1] += (T)0.5 * (Db[3] - w01b);
-  Lb[2][1] += (T)0.5 * (Db[4] + w12b);
-  Lb[1][2] += (T)0.5 * (Db[4] - w12b);
-  Lb[2][0] += (T)0.5 * (Db[5] + w02b);
-  Lb[0][2] += (T)0.5 * (Db[5] - w02b);
-  // L = fl adj(J) G
-  T flb = 0;
-  for (int i = 0; i < 3; i++)
-    for (int k = 0; k < 3; k++) flb += Lb[i][k] * L[i][k];
-  flb /= fl;
-  T Gbar[3][3];
-  for (int mm = 0; mm < 3; mm++)
-    for (int k = 0; k < 3; k++)
-      Gbar[mm][k] = fl * (Am[0][mm] * Lb[0][k] + Am[1][mm] * Lb[1][k] + Am[2][mm] * Lb[2][k]);
-  for (int i = 0; i < 3; i++)
-    for (int mm = 0; mm < 3; mm++)
-      Ab[i][mm] += fl * (Lb[i][0] * G[mm][0] + Lb[i][1] * G[mm][1] + Lb[i][2] * G[mm][2]);
-  const T detJb = -flb * fl / detJ;
-  // predicted velocities: the transpose of the Walsh analysis
-  for (int k = 0; k < 3; k++) {
-    T o[8], v[8];
-    o[0] = 0;
-    for (int mm = 0; mm < 3; mm++) o[1 + mm] = Gbar[mm][k];
-    for (int j = 0; j < 4; j++) o[4 + j] = hmb[k][j];
-    walsh8t_synth(o, v);
-    for (int a = 0; a < 8; a++) A.cv[(a * 3 + k) * ne + e] = (double)v[a];
-  }
-  // adj(J) and detJ back to J, then to the coordinates
-  T Jb[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-  adj_reverse<T>(J, Ab, Jb);
-  for (int mm = 0; mm < 3; mm++)
-    for (int k = 0; k < 3; k++) Jb[mm][k] += detJb * Am[k][mm];
-  for (int k = 0; k < 3; k++) {
-    T o[8], v[8];
-    o[0] = 0;
-    for (int mm = 0; mm < 3; mm++) o[1 + mm] = (T)0.125 * Jb[mm][k];
-    for (int j = 4; j < 8; j++) o[j] = 0;
-    walsh8t_synth(o, v);
-    for (int a = 0; a < 8; a++) A.cx[(a * 3 + k) * ne + e] = (double)v[a];
-  }
-  A.cj[e] = (double)(Javgb / (T)8);
-  A.volb[e] = (double)volb;
-  for (int c = 0; c < 6; c++) A.T[c * ne + e] = (double)tb[c];
+  const T Q0 = (T)2 * dt * tsb[0], Q3 = dt * tsb[3], Q4 = dt * tsb[4], Q5 = dt * tsb[5];
+  A.T[e] = (double)fma(Q5, w02, fma(Q3, w01, tsb[0]));
+  A.T[ne + e] = (double)fma(Q4, w12, fma(Q3, w01, tsb[1]));
+  A.T[2 * ne + e] = (double)fma(Q5, w02, fma(Q4, w12, tsb[2]));
+  A.T[3 * ne + e] = (double)fma(Q5, w12, fma(Q4, w02, fma(Q0, w01, tsb[3])));
+  A.T[4 * ne + e] = (double)fma(Q5, w01, fma(Q3, w02, tsb[4]));
+  A.T[5 * ne + e] = (double)fma(-Q4, w01, fma(-Q3, w12, fma(Q0, w02, tsb[5])));
   A.EP[e] = (double)eplb;
-  const double Eb = (double)Kb * (m.K / m.E) + (double)Gb * (m.G / m.E);
-  A.gth[e] += Eb;
+  const T w01b = fma(Q5, t[4], fma(-Q4, t[5], fma(Q3, t01, Q0 * t[3])));
+  const T w02b = fma(Q5, t02, fma(Q4, t[3], fma(Q3, t[4], Q0 * t[5])));
+  const T w12b = fma(Q5, t[3], fma(Q4, t12, -Q3 * t[5]));
+  // adjoint of L times 1 / D: the deviator of D and the halves of D, W
+  const T rg = r * gdt, rh = (T)0.5 * r;
+  const T mean = third * (tsb[0] + tsb[1] + tsb[2]);
+  const T h01 = (T)0.5 * rg * tsb[3], h12 = (T)0.5 * rg * tsb[4], h02 = (T)0.5 * rg * tsb[5];
+  const T Lr[3][3] = {{rg * (tsb[0] - mean), fma(-rh, w01b, h01), fma(-rh, w02b, h02)},
+                      {fma(rh, w01b, h01), rg * (tsb[1] - mean), fma(-rh, w12b, h12)},
+                      {fma(rh, w02b, h02), fma(rh, w12b, h12), rg * (tsb[2] - mean)}};
+  // L = adj(X) G / D
+  T Db = 0;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      Db = fma(-Lr[i][k], L[i][k], Db);
+      Ab[i][k] = fma(Lr[i][2], G[k][2], fma(Lr[i][1], G[k][1], fma(Lr[i][0], G[k][0], Ab[i][k])));
+    }
+  // predicted velocities: the transpose of the Walsh analysis
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    T Gk[3], v[8], h[8];
+#pragma unroll
+    for (int mm = 0; mm < 3; mm++)
+      Gk[mm] = fma(Am[2][mm], Lr[2][k], fma(Am[1][mm], Lr[1][k], Am[0][mm] * Lr[0][k]));
+    synth_linear(Gk[0], Gk[1], Gk[2], v);
+    synth_hourglass(hmb[k][0], hmb[k][1], hmb[k][2], hmb[k][3], h);
+#pragma unroll
+    for (int a = 0; a < 8; a++) A.cv[(a * 3 + k) * ne + e] = (double)(v[a] + h[a]);
+  }
+  // adj(X) and D back to X
+  T Xb[3][3];
+#pragma unroll
+  for (int mm = 0; mm < 3; mm++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) Xb[mm][k] = Db * Am[k][mm];
+  adj_reverse<T>(X, Ab, Xb);
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+#pragma unroll
+    for (int mm = 0; mm < 3; mm++) {
+      A.cx[(3 * k + mm) * ne + e] = (double)Xb[mm][k];
+      A.cx[(9 + 3 * k + mm) * ne + e] = (double)Am[k][mm];
+    }
+  A.cj[e] = (double)(-K * pb * (T)0.125);
+  A.volb[e] = (double)volb;
+  const double EbE = (double)(fma(-dJ * pb, K, fma(Gb, Gm, (T)0.5 * cc)));
+  A.gth[e] = fma(EbE, m.iE, A.gth[e]);
   A.gth[ne + e] += (double)sy0b;
   A.gth[2 * ne + e] += (double)Hb;
 }
 
-// Node gather of the element contributions; predictor and nodal-volume reverse.
+// Node gather of the element contributions to the predicted velocity and the J
+// ratio; predictor and nodal-volume reverse.
+template <int NPE>
 __global__ void k_adj_gather(StepParams P, AdjArgs A) {
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= P.nn) return;
   const int64_t np = P.np, ne = P.ne;
-  const int npe = P.npe;
   const int32_t b = P.off[n], c = P.off[n + 1] - b;
   double vpb[3] = {A.vpb[n], A.vpb[np + n], A.vpb[2 * np + n]};
-  double xb[3] = {0, 0, 0};
   double jrb = 0.0;
-  for (int32_t q = 0; q < c; q++) {
-    const int32_t sl = P.slot[b + q];
-    const int64_t e = sl / npe, loc = sl % npe;
-    for (int k = 0; k < 3; k++) {
-      vpb[k] += A.cv[(loc * 3 + k) * ne + e];
-      xb[k] += A.cx[(loc * 3 + k) * ne + e];
+  for (int32_t q0 = 0; q0 < c; q0 += 8) {
+    int32_t sl[8];
+    double g[8][3], gj[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) sl[j] = (q0 + j < c) ? __ldg(&P.slot[b + q0 + j]) : -1;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      gather_entry<NPE, 3>(A.cv, ne, sl[j], g[j]);
+      gj[j] = sl[j] >= 0 ? __ldg(&A.cj[sl[j] / NPE]) : 0.0;
     }
-    jrb += A.cj[e];
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (sl[j] >= 0) {
+        for (int k = 0; k < 3; k++) vpb[k] += g[j][k];
+        jrb += gj[j];
+      }
   }
   const uint32_t code = P.bc[n];
   const double dt = P.dt;
   for (int k = 0; k < 3; k++) {
-    A.X[k * np + n] += xb[k];
     if (!((code >> k) & 1u)) {
       A.V[k * np + n] += vpb[k];
       A.PA[k * np + n] += (1.0 - P.gamma) * dt * vpb[k];
@@ -731,83 +735,73 @@ __global__ void k_adj_gather(StepParams P, AdjArgs A) {
   A.sb[n] = sb;
 }
 
-// Volume adjoint (hourglass part + nodal sums) through detJ and J to x.
+// Volume adjoint (hourglass part + nodal sums) through detJ and J, with the
+// element phase's adjoint of J, to the corners' positions. Hexahedra: vol =
+// D / 64 and dD/dX[m][k] = adj(X)[k][m], both left by k_adj_hex; one synthesis
+// for the two (50 FP64 instructions; forming 8 J and its adjugate again and a
+// synthesis for each took 180 here and 33 in k_adj_hex).
 template <int NPE>
 __global__ void k_adj_volume(StepParams P, AdjArgs A, int s) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= P.ne) return;
   const int64_t np = P.np, ne = P.ne;
-  const double *sx = A.sx + (int64_t)s * 3 * np;
-  double x[NPE][3];
+  int32_t nid[NPE];
+#pragma unroll
+  for (int a = 0; a < NPE; a++) nid[a] = __ldg(&P.elnod[a * ne + e]);
   double volb = A.volb[e];
-  for (int a = 0; a < NPE; a++) {
-    const int32_t n = P.elnod[a * ne + e];
-    volb += A.sb[n];
-    for (int k = 0; k < 3; k++) x[a][k] = sx[k * np + n];
-  }
-  const double w = (NPE == 8) ? 8.0 : 1.0 / 6.0;
-  const double detJb = w * volb;
+#pragma unroll
+  for (int a = 0; a < NPE; a++) volb += __ldg(&A.sb[nid[a]]);
   if constexpr (NPE == 8) {
-    // d detJ / d J = cofactors; J = W(x) / 8 relative to node 0, x-bar its transpose
-    double J[3][3];
+    const double Db = volb * (1.0 / 64.0);
+#pragma unroll
     for (int k = 0; k < 3; k++) {
-      double v[8], o[8];
-      for (int a = 0; a < 8; a++) v[a] = x[a][k] - x[0][k];
-      walsh8t(v, o);
-      for (int mm = 0; mm < 3; mm++) J[mm][k] = 0.125 * o[1 + mm];
-    }
-    double C[3][3];  // cofactors C[m][k] = d detJ / d J[m][k]
-    C[0][0] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
-    C[0][1] = J[1][2] * J[2][0] - J[1][0] * J[2][2];
-    C[0][2] = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-    C[1][0] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
-    C[1][1] = J[0][0] * J[2][2] - J[0][2] * J[2][0];
-    C[1][2] = J[0][1] * J[2][0] - J[0][0] * J[2][1];
-    C[2][0] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
-    C[2][1] = J[0][2] * J[1][0] - J[0][0] * J[1][2];
-    C[2][2] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
-    for (int k = 0; k < 3; k++) {
-      double o[8], v[8];
-      o[0] = 0.0;
-      for (int mm = 0; mm < 3; mm++) o[1 + mm] = 0.125 * detJb * C[mm][k];
-      for (int j = 4; j < 8; j++) o[j] = 0.0;
-      walsh8t_synth(o, v);
+      double o[3], v[8];
+#pragma unroll
+      for (int mm = 0; mm < 3; mm++)
+        o[mm] = fma(Db, __ldg(&A.cx[(9 + 3 * k + mm) * ne + e]), __ldg(&A.cx[(3 * k + mm) * ne + e]));
+      synth_linear(o[0], o[1], o[2], v);
+#pragma unroll
       for (int a = 0; a < 8; a++) A.cgeo[(a * 3 + k) * ne + e] = v[a];
     }
   } else {
+    const double *sx = A.sx + (int64_t)s * 3 * np;
+    double x[NPE][3];
+#pragma unroll
+    for (int a = 0; a < NPE; a++)
+      for (int k = 0; k < 3; k++) x[a][k] = sx[k * np + nid[a]];
+    const double detJb = 1.0 / 6.0 * volb;
     ElemGeom<double, NPE> g;
     geom_forward<double, NPE>(x, g);
     for (int a = 0; a < NPE; a++)
       for (int k = 0; k < 3; k++) {
-        double xb = 0;
+        double xb = A.cx[(a * 3 + k) * ne + e];
         for (int mm = 0; mm < 3; mm++) xb += detJb * g.A[k][mm] * tj<NPE>(mm, a);
         A.cgeo[(a * 3 + k) * ne + e] = xb;
       }
   }
 }
 
-// Copies the start-of-step state into the stash slot s.
-__global__ void k_adj_stash(StepParams P, Fp64State S, AdjArgs A, int s) {
+// Copies into the stash the nodal quantities of the step just made (slot
+// `made`, after its nodal and node phases) and the state the next step starts
+// from (slot `next`); a negative slot: not.
+__global__ void k_adj_stash(StepParams P, Fp64State S, AdjArgs A, int made, int next) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t np = P.np, ne = P.ne;
-  if (i < 3 * np) {
-    A.sx[(int64_t)s * 3 * np + i] = S.x[i];
-    A.sv[(int64_t)s * 3 * np + i] = S.v[i];
-    A.spa[(int64_t)s * 3 * np + i] = S.pa[i];
+  if (made >= 0) {
+    if (i < np) {
+      A.sjr[(int64_t)made * np + i] = S.jr[i];
+      A.smass[(int64_t)made * np + i] = S.mass[i];
+    }
+    if (i < 3 * np) A.sfi[(int64_t)made * 3 * np + i] = S.fi[i];
   }
-  if (i < 6 * ne) A.stau[(int64_t)s * 6 * ne + i] = S.tau[i];
-  if (i < ne) A.spls[(int64_t)s * ne + i] = S.pls[i];
-}
-
-// Copies the nodal quantities of step s (after its nodal and node phases).
-__global__ void k_adj_stash_step(StepParams P, Fp64State S, AdjArgs A, int s) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t np = P.np;
-  if (i < np) {
-    A.sjr[(int64_t)s * np + i] = S.jr[i];
-    A.smass[(int64_t)s * np + i] = S.mass[i];
+  if (next >= 0) {
+    if (i < 3 * np) {
+      A.sx[(int64_t)next * 3 * np + i] = S.x[i];
+      A.svp[(int64_t)next * 3 * np + i] = S.vp[i];
+    }
+    if (i < 6 * ne) A.stau[(int64_t)next * 6 * ne + i] = S.tau[i];
+    if (i < ne) A.spls[(int64_t)next * ne + i] = S.pls[i];
   }
-  if (i < 3 * np) A.sfi[(int64_t)s * 3 * np + i] = S.fi[i];
 }
 
 // Per-node constants of the reverse: 1 / s0 and d(mass)/d(sum of element
@@ -830,36 +824,34 @@ void adj_node_constants(const StepParams &P, const AdjArgs &A, cudaStream_t st) 
   k_adj_node_constants<<<grid_for(P.nn), kThreads, 0, st>>>(P, A);
 }
 
-void adj_stash_state(const StepParams &P, const Fp64State &S, const AdjArgs &A, int s,
-                     cudaStream_t st) {
-  const int64_t n = std::max<int64_t>(3 * P.np, 6 * P.ne);
-  k_adj_stash<<<grid_for(n), kThreads, 0, st>>>(P, S, A, s);
-}
-
-void adj_stash_step(const StepParams &P, const Fp64State &S, const AdjArgs &A, int s,
-                    cudaStream_t st) {
-  k_adj_stash_step<<<grid_for(3 * P.np), kThreads, 0, st>>>(P, S, A, s);
+void adj_stash(const StepParams &P, const Fp64State &S, const AdjArgs &A, int made, int next,
+               cudaStream_t st) {
+  const int64_t n = std::max<int64_t>(3 * P.np, next >= 0 ? 6 * P.ne : 0);
+  k_adj_stash<<<grid_for(n), kThreads, 0, st>>>(P, S, A, made, next);
 }
 
 void adj_reverse_step(const StepParams &P, const AdjArgs &A, int s, long long gstep, int have_geo,
                       bool fp32, cudaStream_t st) {
-  k_adj_nodes<<<grid_for(P.nn), kThreads, 0, st>>>(P, A, s, gstep, have_geo);
   if (P.npe == 8) {
+    k_adj_nodes<8><<<grid_for(P.nn), kThreads, 0, st>>>(P, A, s, gstep, have_geo);
     if (fp32)
       k_adj_hex<float><<<grid_for(P.ne), kThreads, 0, st>>>(P, A, s);
     else
       k_adj_hex<double><<<grid_for(P.ne), kThreads, 0, st>>>(P, A, s);
   } else {
+    k_adj_nodes<4><<<grid_for(P.nn), kThreads, 0, st>>>(P, A, s, gstep, have_geo);
     if (fp32)
       k_adj_elements<float, 4><<<grid_for(P.ne), kThreads, 0, st>>>(P, A, s);
     else
       k_adj_elements<double, 4><<<grid_for(P.ne), kThreads, 0, st>>>(P, A, s);
   }
-  k_adj_gather<<<grid_for(P.nn), kThreads, 0, st>>>(P, A);
-  if (P.npe == 8)
+  if (P.npe == 8) {
+    k_adj_gather<8><<<grid_for(P.nn), kThreads, 0, st>>>(P, A);
     k_adj_volume<8><<<grid_for(P.ne), kThreads, 0, st>>>(P, A, s);
-  else
+  } else {
+    k_adj_gather<4><<<grid_for(P.nn), kThreads, 0, st>>>(P, A);
     k_adj_volume<4><<<grid_for(P.ne), kThreads, 0, st>>>(P, A, s);
+  }
 }
 
 }  // namespace wf

@@ -2213,6 +2213,7 @@ WF_API wf_status wf_init(wf_domain *d) {
     t.H = m.H;
     t.cs0 = std::sqrt(t.K / m.rho);
     t.i3GH = 1.0 / (3.0 * t.G + t.H);
+    t.iE = 1.0 / m.E;
     t.model = m.model;
     t.hol_K = m.hol_K;
     t.hol_m = m.hol_m;
@@ -3766,8 +3767,7 @@ wf_status adjoint_buffers(wf_domain *d) {
   const size_t np = d->np, ne = d->ne, seg = d->adj_every, npe = d->npe;
   AdjArgs &A = d->A;
   CUDA_TRY(adj_alloc(d, &A.sx, seg * 3 * np));
-  CUDA_TRY(adj_alloc(d, &A.sv, seg * 3 * np));
-  CUDA_TRY(adj_alloc(d, &A.spa, seg * 3 * np));
+  CUDA_TRY(adj_alloc(d, &A.svp, seg * 3 * np));
   CUDA_TRY(adj_alloc(d, &A.sjr, seg * np));
   CUDA_TRY(adj_alloc(d, &A.smass, seg * np));
   CUDA_TRY(adj_alloc(d, &A.sfi, seg * 3 * np));
@@ -3812,16 +3812,16 @@ void run_stashed(wf_domain *d, int64_t first, int64_t L) {
   const Fp64State &S = d->S;
   const AdjArgs &A = d->A;
   fp64_predict(P, S, d->stream);
+  adj_stash(P, S, A, -1, (int)first, d->stream);
   for (int64_t j = 0; j < L; j++) {
-    adj_stash_state(P, S, A, (int)(first + j), d->stream);
     fp64_geometry(P, S, d->stream, false);
     fp64_nodal(P, S, d->stream, 0);
     fp64_elements(P, S, d->stream);
     fp64_nodes(P, S, d->stream, d->node_grid);
     if (P.energy_on) energy_fp64(P, S, d->stream);
-    adj_stash_step(P, S, A, (int)(first + j), d->stream);
+    adj_stash(P, S, A, (int)(first + j), j + 1 < L ? (int)(first + j + 1) : -1, d->stream);
   }
-  d->launches += 1 + (6 + (P.energy_on ? 1 : 0)) * L;
+  d->launches += 2 + (5 + (P.energy_on ? 1 : 0)) * L;
 }
 
 }  // namespace
@@ -3846,7 +3846,7 @@ WF_API wf_status wf_adjoint_forward(wf_domain *d, int64_t nsteps, int64_t every)
   if (every == -1) {
     // keep every step's inputs: no checkpoints, no recompute in the reverse pass
     free_adjoint(d);
-    const double need = (double)nsteps * (14.0 * d->np + 7.0 * d->ne) * sizeof(double);
+    const double need = (double)nsteps * (11.0 * d->np + 7.0 * d->ne) * sizeof(double);
     size_t free_b = 0, total_b = 0;
     CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
     if (need > 0.9 * (double)free_b)

@@ -15,7 +15,7 @@ namespace wf {
 // Per-material constants on the device (Elastic_ / Material_, Material.cuh).
 struct MatDev {
   double K, G, sy0, H, cs0, hol_K, hol_m, eps0, eps1, E;
-  double i3GH;                               // 1 / (3 G + H), bilinear return
+  double i3GH, iE;                           // 1 / (3 G + H), bilinear return; 1 / E
   double jc_B, jc_n, jc_C, jc_eps0, jc_Th;  // Johnson-Cook; jc_Th = 1 - T_h^m (host-computed)
   double jc_m, jc_Tm, jc_Tt;                 // its temperature terms (thermal coupling)
   double k_T, cp_T, exp_T;                   // conductivity, heat capacity, expansion
