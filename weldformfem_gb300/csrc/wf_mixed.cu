@@ -91,8 +91,10 @@ struct F2 {
 };
 
 // a - b for nearby points: hi parts subtract exactly when within a factor 2.
+template <bool PACKED = true>
 __device__ __forceinline__ float pair_rel(float2 a, float2 b) {
-  const F2<> d = F2<>{a.x, a.y} - F2<>{b.x, b.y};
+  using V2 = F2<PACKED>;
+  const V2 d = V2{a.x, a.y} - V2{b.x, b.y};
   return __fadd_rn(d.x, d.y);
 }
 
@@ -171,7 +173,8 @@ __device__ __forceinline__ void rel_coords(const StepParams &P, const MixState &
 #pragma unroll
   for (int a = 1; a < NPE; a++)
 #pragma unroll
-    for (int k = 0; k < 3; k++) r[a][k] = pair_rel(ldx<LD>(&M.xh[k * P.np + nid[a]]), o[k]);
+    for (int k = 0; k < 3; k++)
+      r[a][k] = pair_rel<NPE == 8>(ldx<LD>(&M.xh[k * P.np + nid[a]]), o[k]);
 }
 
 template <typename V>
@@ -398,12 +401,13 @@ __device__ __forceinline__ void nodal_gather(const StepParams &P, const MixState
     for (int j = 0; j < 8; j++)
       if (el[j] >= 0) s += g[j];
   } else {
-    const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
+    const NodeSlots ls = node_slots<NPE>(P, n);
+    const int32_t c = ls.c;
     nc = __ldg(&M.nc[n]);   // issued before the gather, used after it
     for (int32_t k0 = 0; k0 < c; k0 += 8) {
       int32_t sl[8];
 #pragma unroll
-      for (int j = 0; j < 8; j++) sl[j] = (k0 + j < c) ? __ldg(&P.slot[b + k0 + j]) : -1;
+      for (int j = 0; j < 8; j++) sl[j] = (k0 + j < c) ? ls[k0 + j] : -1;
       float g[8];
 #pragma unroll
       for (int j = 0; j < 8; j++) g[j] = (sl[j] >= 0) ? ldx<LD>(&vol[sl[j] / NPE]) : 0.0f;
@@ -1295,8 +1299,8 @@ __device__ __forceinline__ float node_finish(const StepParams &P, const MixState
       for (int j = 0; j < 8; j++)
         if (el[j] >= 0) sT += q[j];
     } else {
-      const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
-      for (int32_t k = 0; k < c; k++) sT += ldx<LD>(&cur[__ldg(&P.slot[b + k])]);
+      const NodeSlots ls = node_slots<NPE>(P, n);
+      for (int32_t k = 0; k < ls.c; k++) sT += ldx<LD>(&cur[ls[k]]);
     }
     M.T[n] = pair_add(M.T[n], (sT + M.qc[n] / (mass * P.f_cp0)) * c_dt);
   }
@@ -1344,13 +1348,14 @@ __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M
     return node_finish<NPE, LD, BOX>(P, M, n, step, fi0, fi1, fi2, x, vp, M.xh, M.vp,
                                       node_in<LD>(P, M, n));
   }
-  const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
+  const NodeSlots ls = node_slots<NPE>(P, n);
+  const int32_t c = ls.c;
   // gather over the node's element list in list order, eight entries at a
   // time so that the slot and force loads of a chunk are all in flight
   for (int32_t k0 = 0; k0 < c; k0 += 8) {
     int32_t sl[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) sl[j] = (k0 + j < c) ? __ldg(&P.slot[b + k0 + j]) : -1;
+    for (int j = 0; j < 8; j++) sl[j] = (k0 + j < c) ? ls[k0 + j] : -1;
     float g0[8], g1[8], g2[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
@@ -1382,8 +1387,9 @@ __device__ __forceinline__ float node_one(const StepParams &P, const MixState &M
 }
 
 template <int NPE, int BOX>
-__global__ void __launch_bounds__(kNodeThreads, WF_NODE_MIN_BLOCKS) k_mix_nodes(StepParams P,
-                                                                             MixState M) {
+__global__ void __launch_bounds__(kNodeThreads, NPE == 4 ? 4 : WF_NODE_MIN_BLOCKS)
+    k_mix_nodes(StepParams P, MixState M) {   // tetrahedra: the list's addresses would spill
+
   __shared__ double sh[kNodeThreads / 32];
   __shared__ bool am_last;
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

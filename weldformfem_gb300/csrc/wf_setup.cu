@@ -403,6 +403,37 @@ void scatter_u32(uint32_t *dst, const int32_t *idx, const uint32_t *val, int64_t
 }
 
 namespace {
+__global__ void k_longest_list(const int32_t *off, int64_t nn, int32_t *most) {
+  const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t c = n < nn ? off[n + 1] - off[n] : 0;
+  const int32_t m = __reduce_max_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) atomicMax(most, m);
+}
+__global__ void k_list_cols(const int32_t *off, const int32_t *slot, int64_t nn, int64_t np,
+                            int32_t width, int32_t *cols) {
+  const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= nn) return;
+  const int32_t b = off[n], c = off[n + 1] - b;
+  for (int32_t k = 0; k < width; k++) cols[(int64_t)k * np + n] = k < c ? slot[b + k] : -1;
+}
+}  // namespace
+
+cudaError_t longest_list(const int32_t *off, int64_t nn, int32_t *flag, cudaStream_t st,
+                         int32_t *most) {
+  cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int32_t), st);
+  if (e != cudaSuccess) return e;
+  k_longest_list<<<grid_for(nn), kThreads, 0, st>>>(off, nn, flag);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  e = cudaMemcpyAsync(most, flag, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(st);
+}
+
+void list_cols(const int32_t *off, const int32_t *slot, int64_t nn, int64_t np, int32_t width,
+               int32_t *cols, cudaStream_t st) {
+  k_list_cols<<<grid_for(nn), kThreads, 0, st>>>(off, slot, nn, np, width, cols);
+}
+
+namespace {
 __global__ void k_fill_owner(const int64_t *off, int parts, int64_t n, uint16_t *dst) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
