@@ -746,17 +746,22 @@ __device__ __forceinline__ void thermal_pre(const StepParams &P, const MixState 
 }
 
 // After the forces: the element-node temperature rates -(K T)_a / m_a plus the
-// plastic heat 0.9 q vol / n / (m_a cp_T), written to the step's buffer, one
-// division a node. KT holds (K T)_a / kf; qvol = q vol.
+// plastic heat 0.9 q vol / n / (m_a cp_T), written to the step's buffer.
+// KT holds (K T)_a / kf; qvol = q vol. (Two divisions a node: one, with the heat
+// over cp_T first, rounds otherwise, and a Johnson-Cook run ahead of the first
+// stress wave amplifies a rounding by 1e4 and more.)
 template <int NPE, class Nodes>
 __device__ __forceinline__ void thermal_rates(const StepParams &P, const MixState &M,
                                               const MatF &m, int64_t e, const Nodes &nd,
                                               long long step, const float (&KT)[NPE], float kf,
                                               float qvol) {
   float *cur = M.dte + (step & 1) * P.ne * NPE + e * NPE;
-  const float heat = 0.9f * qvol * (1.0f / NPE) / m.cp_T;
+  const float ppn = 0.9f * qvol * (1.0f / NPE);
 #pragma unroll
-  for (int a = 0; a < NPE; a++) cur[a] = (heat - kf * KT[a]) / nd.mass(M, a);
+  for (int a = 0; a < NPE; a++) {
+    const float mi = nd.mass(M, a);
+    cur[a] = -(kf * KT[a]) / mi + ppn / (mi * m.cp_T);
+  }
 }
 
 // The thermal step's node values from the node arrays, by node id: temperature,
@@ -1127,11 +1132,16 @@ __device__ __forceinline__ void element_one(const StepParams &P, const MixState 
 #ifndef WF_ELEM_THREADS_PER_SM
 #define WF_ELEM_THREADS_PER_SM 1024
 #endif
-constexpr int elem_min_blocks(int bs) { return WF_ELEM_THREADS_PER_SM / bs; }
+// The thermal hexahedra take 80: at 64 they spill 108 bytes (446,000 Johnson-Cook
+// hexahedra: 84.2 -> 81.4 us a step; 96 registers, 86.7).
+template <int NPE, bool TH>
+constexpr int elem_min_blocks(int bs) {
+  return (NPE == 8 && TH ? 768 : WF_ELEM_THREADS_PER_SM) / bs;
+}
 
 template <int NPE, int BS, int LAW, bool TH, int BOX>
-__global__ void __launch_bounds__(BS, elem_min_blocks(BS)) k_mix_elements(StepParams P,
-                                                                          MixState M) {
+__global__ void __launch_bounds__(BS, elem_min_blocks<NPE, TH>(BS)) k_mix_elements(StepParams P,
+                                                                                   MixState M) {
   __shared__ float stash[NPE == 8 ? 12 * BS : 1];
   const long long step = TH ? P.st->step : 0;
   for (int64_t e = (int64_t)blockIdx.x * BS + threadIdx.x; e < P.ne; e += (int64_t)gridDim.x * BS)
@@ -3649,6 +3659,11 @@ bool mix_tile_run_shape(const StepParams &P, TileRunShape &C) {
       }
     }
   if (!found) return false;
+  // thermal elements in more than two passes are faster per phase (Johnson-Cook,
+  // tile run and per phase: 168,000 in two passes 32.7 and 34.4 us a step, 195,000
+  // in three 38.0 and 38.3, 226,000 47.5 and 44.4; without heat 226,000 take 27.7
+  // and 29.9)
+  if (P.thermal && C.e0 > 2 * kTileRunThreads) return false;
   const TileRunKernel k = tile_run_kernel(P);
   const int bytes = TileRunSmem(C).total;
   int dev = 0, coop = 0, per = 0;
