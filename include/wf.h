@@ -392,7 +392,9 @@ WF_API wf_status wf_set_launch_config(wf_domain *d, int32_t phase, int32_t block
  * blocks, sized at wf_init for meshes of at most 65536 elements) whose blocks
  * own fixed element and node ranges and meet at cluster barriers between the
  * phases: same per-element and per-node arithmetic, so the state is bitwise
- * that of mode 1; the reaction sum runs in another order. Not with specimens,
+ * that of mode 1; the reaction sum runs in another order. Hexahedra without
+ * thermal coupling and triangle-mesh contact keep the run's state in the
+ * cluster's shared memory where it fits. Not with specimens,
  * the energy history or phase timing. Mode 3 (hexahedra): the element and
  * node phases become a tiled kernel and a shared-node kernel. At wf_init the
  * elements are binned by centroid into cubes of about 8 element sizes and cut
@@ -429,12 +431,20 @@ WF_API wf_status wf_set_launch_config(wf_domain *d, int32_t phase, int32_t block
  * expected) makes the next wf_sync return WF_ERR_TIMEOUT. On GB300 mode 5 is
  * slower than modes 4 and 1 (the blocks' waits and ticket traffic cost more
  * than the L2 reuse saves) and is only run when asked for. Mode 0 (default)
- * picks mode 2 for meshes of at most 3000 elements, else mode 4 where the mesh
- * is swept and its columns fill the GPU (at least 95 % of two per SM: a
- * column is a sequence of layers), else mode 1. wf_get_step_mode reports the mode the next wf_run uses and,
- * for mode 2, the cluster's blocks and block size, for mode 3 the tiles and
- * threads per tile, for mode 4 the columns and threads per column, for mode 5
- * the blocks and threads per block (0 otherwise). */
+ * picks mode 2 for meshes of at most 3000 elements, or of at most 6500
+ * hexahedra whose run fits the cluster's shared memory; else, for box meshes of
+ * hexahedra whose tiles fit the SMs' shared memory (up to about 230,000; with
+ * thermal coupling 185,000; no specimens, energy history or phase timing), whole spans of steps as one
+ * cooperative launch, each block keeping its tile's stresses on the chip, with
+ * two bounded barriers over the grid a step (mode 1's arithmetic and order of
+ * sums; a barrier that runs out makes wf_sync return WF_ERR_TIMEOUT); else mode
+ * 4 where the mesh is swept and its columns fill the GPU (at least 95 % of two
+ * per SM: a column is a sequence of layers), else mode 1.
+ * wf_get_step_mode reports the mode the next wf_run uses (1 for the cooperative
+ * launch and for a cluster run of more than 3000 elements) and, for mode 2, the
+ * cluster's blocks and block size, for mode 3 the tiles and threads per tile,
+ * for mode 4 the columns and threads per column, for mode 5 the blocks and
+ * threads per block (0 otherwise). */
 WF_API wf_status wf_set_step_mode(wf_domain *d, int32_t mode);
 /* No counterpart in the reference. Node rows per column of the column sweep
  * (4 or 8, default 8), before wf_init. wf_get_sweep: the columns along x and
@@ -524,7 +534,7 @@ WF_API wf_status wf_nodal_volumes_noalloc(const double *xyz, const int32_t *elno
  * does, and keeps an in-memory checkpoint of the state (x, v, prev_a, u, tau,
  * eps, eps_p) every `every` steps (0: about sqrt(nsteps); -1: keep every
  * step's inputs instead, no checkpoints and no recompute in the reverse pass,
- * when the device has room: nsteps (14 nn + 7 ne) doubles). Supported: FP64
+ * when the device has room: nsteps (11 nn + 7 ne) doubles). Supported: FP64
  * precision, bilinear materials, pressure algorithm 0 with default
  * stabilisation, no artificial viscosity, no contact, no specimens.
  * wf_adjoint_backward takes dL_dR[nsteps] (host) and writes
@@ -533,7 +543,9 @@ WF_API wf_status wf_nodal_volumes_noalloc(const double *xyz, const int32_t *elno
  * (node update, internal-force gather, element stress update with the
  * consistent derivative of the radial return, hourglass forces, nodal volumes
  * and masses), and leaves the domain in the state at the end of the forward
- * run, so it may be called again with another dL_dR. reverse_fp32 != 0 runs
+ * run, so it may be called again with another dL_dR. Where a second segment's
+ * inputs take at most a quarter of the free memory, a segment is recomputed
+ * while the one after it is reversed. reverse_fp32 != 0 runs
  * the element reverse arithmetic in FP32 (the recomputed forward stays FP64).
  * The domain must not step between the two calls. */
 WF_API wf_status wf_adjoint_forward(wf_domain *d, int64_t nsteps, int64_t every);
