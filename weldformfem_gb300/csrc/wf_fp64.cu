@@ -879,7 +879,9 @@ __device__ __forceinline__ bool tri_hit(const StepParams &P, int32_t j, const do
 // exact value; a distance is rejected above 1e-5 R, an edge test below
 // -1e-4 R^2, and a comparison that involves an infinity or NaN rejects nothing.
 // 98 triangles over 13,671 nodes: 255 -> 85 us a step, the contact force and
-// the die's motion included.
+// the die's motion included; with the kernel beside the element kernel and the
+// FP64 tests of a warp taken together the whole step of 72,000 tetrahedra is
+// 93 us, 393 before.
 constexpr int kTriChunk = 64;
 struct TriFilter {
   float n[3], pp, v[3][3], r;

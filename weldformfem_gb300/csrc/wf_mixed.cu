@@ -101,7 +101,7 @@ __device__ __forceinline__ float pair_rel(float2 a, float2 b) {
 // Loads of data that other threads write during the run. kLdRo: the read-only
 // path (__ldg), in the per-phase kernels, where the data is constant for the
 // launch. kLdL2: through L2 (__ldcg), in the cluster run and the dataflow
-// step, whose phases share one launch. kLdL1: plain loads, in the grid run,
+// step, whose phases share one launch. kLdL1: plain loads, in the tile run,
 // whose barrier between phases is an acquire (it drops the SM's L1 lines), so
 // that a phase still shares its gathers in L1.
 enum : int { kLdRo = 0, kLdL2 = 1, kLdL1 = 2 };
