@@ -8,6 +8,7 @@ round exactly as the reference CPU code (built without FMA contraction).
 from __future__ import annotations
 
 import concurrent.futures as cf
+import glob
 import os
 import shutil
 import subprocess
@@ -43,10 +44,8 @@ def nvcc() -> str:
 
 
 def _sources():
-    return [os.path.join(CSRC, u) for u in UNITS] + [
-        os.path.join(CSRC, "wf_internal.cuh"), os.path.join(CSRC, "wf_adjoint.cuh"),
-        os.path.join(CSRC, "wf_trimesh.cuh"),
-        os.path.join(ROOT, "include", "wf.h")]
+    return ([os.path.join(CSRC, u) for u in UNITS] + sorted(glob.glob(os.path.join(CSRC, "*.cuh")))
+            + [os.path.join(ROOT, "include", "wf.h")])
 
 
 def up_to_date() -> bool:
