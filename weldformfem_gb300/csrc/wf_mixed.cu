@@ -2197,6 +2197,7 @@ struct SmemRun {
     total = stash + 4 * 12 * bs;
   }
 };
+constexpr int kClusterSmemMax = 220 * 1024;   // the launch's dynamic shared memory at most
 // rows of the own node state
 enum { kSv = 0, kSpa = 3, kScf = 6, kSut = 9, kSm = 11, kSnc = 12, kSx = 14, kSvp = 20 };
 
@@ -2644,6 +2645,7 @@ __global__ void __launch_bounds__(BS + 32, 1) k_mix_cluster_smem(StepParams P, M
 // step status, which wf_sync reports, and every block leaves.
 constexpr int kTileRunThreads = 608;   // working threads: 96 registers each
 constexpr int kGridSpin = 1 << 22;
+constexpr int kTileRunSmemMax = 225 * 1024;   // the launch's dynamic shared memory at most
 
 __device__ __forceinline__ bool grid_barrier(unsigned *c, unsigned target, StepState *st,
                                              int *s_ok) {
@@ -3303,6 +3305,24 @@ cudaError_t cluster_launch(const StepParams &P, const MixState &M, float *vol, d
   return cudaLaunchKernelEx(&cfg, kern, P, M, vol, part, nsteps);
 }
 
+// Allows a kernel its dynamic shared memory: once per kernel and device, `bytes`
+// a constant of the kernel. The limit belongs to the function and not to a
+// domain: lowered by one host thread between another's call and its launch, it
+// makes that launch fail.
+cudaError_t allow_smem(const void *kern, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<const void *, int>, bool> set;   // (kernel, device)
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  bool &done = set[std::make_pair(kern, dev)];
+  if (done) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  done = e == cudaSuccess;
+  return e;
+}
+
 // The run in shared memory: its launch, or (query) whether a cluster of it can
 // be resident.
 template <int BS, int LAW>
@@ -3313,7 +3333,7 @@ cudaError_t smem_launch(const StepParams &P, const MixState &M, float *vol, int6
   const int bytes = SmemRun(C, BS).total;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    e = allow_smem((const void *)kern, kClusterSmemMax);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
@@ -3413,18 +3433,7 @@ int mix_shared_grid(const TileParams &T) {
 
 void mix_tile(const StepParams &P, const MixState &M, const TileParams &T, cudaStream_t st) {
   auto kern = P.mat_general ? k_mix_tile<1> : k_mix_tile<0>;
-  static std::mutex mu;
-  static std::map<std::pair<const void *, int>, bool> set;   // (kernel, device)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    bool &done = set[std::make_pair((const void *)kern, dev)];
-    if (!done) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem);
-      done = true;
-    }
-  }
+  allow_smem((const void *)kern, kTileSmem);
   kern<<<(unsigned)T.ntiles, kTileElems, kTileSmem, st>>>(P, M, T);
 }
 
@@ -3454,16 +3463,7 @@ SweepKernel sweep_kernel(const StepParams &P, const SweepParams &W, int *threads
     *threads = SweepShape<8>::threads;
     *smem = SweepShape<8>::smem;
   }
-  static std::mutex mu;
-  static std::map<std::pair<const void *, int>, bool> set;   // (kernel, device)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  bool &done = set[std::make_pair((const void *)k, dev)];
-  if (!done) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
-    done = true;
-  }
+  allow_smem((const void *)k, *smem);
   return k;
 }
 }  // namespace
@@ -3498,18 +3498,7 @@ int flow_grid(const StepParams &P) {
   auto kern = P.mat_general ? k_mix_flow<1> : k_mix_flow<0>;
   // the stage table's shared memory at the largest mesh the step takes
   const size_t smem = sizeof(int) * (kFlowMaxLayers + 20);
-  static std::mutex mu;
-  static std::map<std::pair<const void *, int>, bool> set;   // (kernel, device)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    bool &done = set[std::make_pair((const void *)kern, dev)];
-    if (!done) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      done = true;
-    }
-  }
+  allow_smem((const void *)kern, smem);
   int per = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kFlowThreads, smem) != cudaSuccess) {
     cudaGetLastError();
@@ -3587,7 +3576,7 @@ bool mix_cluster_smem_fits(const StepParams &P, const MixState &M, float *vol, i
   C.nt = (int)max_targets;
   C.words = (int)((P.nn + 31) / 32);
   C.chunk = kClusterSmemChunk;
-  if (SmemRun(C, bs).total > 220 * 1024) return false;
+  if (SmemRun(C, bs).total > kClusterSmemMax) return false;
   int fits = 0;
   const cudaError_t e =
       P.mat_general ? smem_dispatch<1>(P, M, vol, 0, blocks, bs, C, nullptr, true, &fits)
@@ -3643,7 +3632,7 @@ bool mix_tile_run_shape(const StepParams &P, TileRunShape &C) {
       S.n1 = (int)((x + 1) * (y + 1) * (z + 1));
       S.e1 = (int)((x + 2) * (y + 2) * (z + 2));
       S.n2 = (int)n2;
-      if (TileRunSmem(S).total > 225 * 1024) continue;
+      if (TileRunSmem(S).total > kTileRunSmemMax) continue;
       auto passes = [](int64_t items) {
         return (double)((items + kTileRunThreads - 1) / kTileRunThreads);
       };
@@ -3669,7 +3658,7 @@ bool mix_tile_run_shape(const StepParams &P, TileRunShape &C) {
   int dev = 0, coop = 0, per = 0;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
+      allow_smem((const void *)k, kTileRunSmemMax) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kTileRunThreads + 32, bytes) !=
           cudaSuccess) {
     cudaGetLastError();
@@ -3684,8 +3673,7 @@ cudaError_t mix_tile_run(const StepParams &P, const MixState &M, float *vol, dou
   if (e != cudaSuccess) return e;
   const TileRunKernel k = tile_run_kernel(P);
   const int bytes = TileRunSmem(C).total;
-  const cudaError_t a =
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+  const cudaError_t a = allow_smem((const void *)k, kTileRunSmemMax);
   if (a != cudaSuccess) return a;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
