@@ -76,25 +76,41 @@ __device__ __forceinline__ T adjugate8(const T (&X)[3][3], T (&A)[3][3]) {
 }
 
 // v^0.6666666 (the hourglass coefficient's exponent, test_1el_3D.cpp:185) for
-// v > 0: the inverse cube root from its FP32 value by one third-order
-// correction, y (1 + e / 3 + 2 e^2 / 9) with e = 1 - v y^3 of about 1e-7, then
-// v^(2/3) = v y, and v^(0.6666666 - 2/3) = exp(z) with |z| < 5e-6 as
-// 1 + z + z^2 / 2; in z the logarithm of the mantissa is FP32 (3e-8 absolute,
-// 2e-15 in the result). About 15 FP64 instructions; values out of the FP32
-// range take pow.
+// v > 0, as p (1 + u) with p = v y0 and y0 the FP32 inverse cube root, u of about
+// 1e-6 and one rounding at the end: y = y0 (1 + t), t = e / 3 + 2 e^2 / 9 with
+// e = 1 - v y0^3 of about 1e-7 (a third-order correction; v y0 in two parts and
+// y0^2 exact), v^(2/3) = v y, and v^(0.6666666 - 2/3) = exp(z) with |z| < 5e-6 as
+// 1 + z + z^2 / 2. The exponent's difference is its own literal (formed from the
+// two doubles it is off by 4e-17), and the logarithm is within 1e-9: of the
+// mantissa m = (1 + s) / (1 - s) the series 2 (s + s^3 / 3 + ...) with s in two
+// floats, all FP32 (logf alone is 4e-8 off, 4e-15 in the result). At most
+// 1.5e-16 relative, as pow's; 17 FP64 instructions; values out of the FP32 range
+// take pow.
 __device__ __forceinline__ double pow_two_thirds(double v) {
   if (!(v > 1e-30 && v < 1e30)) return pow(v, 0.6666666);
   const double y0 = (double)rcbrtf((float)v);
-  const double e = fma(-(v * y0), y0 * y0, 1.0);
-  const double y = fma(y0 * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), y0);
-  // v = m 2^q with m in [1, 2): ln m from its FP32 rounding and the rest
+  const double p = v * y0, pe = fma(v, y0, -p), y2 = y0 * y0;
+  const double e = fma(-pe, y2, fma(-p, y2, 1.0));
+  const double t = e * fma(e, 2.0 / 9.0, 1.0 / 3.0);
+  // v = m 2^q with m in [0.7, 1.42)
   const int hi = __double2hiint(v);
   const double md = __hiloint2double(0x3ff00000 | (hi & 0xfffff), __double2loint(v));
-  const float m = (float)md;
-  const double ln = fma((double)((hi >> 20) - 1023), 0.693147180559945309,
-                        (double)logf(m) + (double)((float)(md - (double)m) / m));
-  const double z = (0.6666666 - 2.0 / 3.0) * ln;
-  return (v * y) * fma(z, fma(z, 0.5, 1.0), 1.0);
+  int q = (hi >> 20) - 1023;
+  float m = (float)md, ml = (float)(md - (double)m);
+  if (m > 1.4142f) {
+    m *= 0.5f;
+    ml *= 0.5f;
+    q += 1;
+  }
+  // s = (m + ml - 1) / (m + ml + 1) = a + al; the differences are exact
+  const float n = m - 1.0f, d = m + 1.0f, dl = (m - (d - 1.0f)) + ml;
+  const float a = n / d, al = (fmaf(-a, d, n) + fmaf(-a, dl, ml)) / d;
+  const float w = a * a;
+  const float c = fmaf(w, fmaf(w, fmaf(w, fmaf(w, 1.f / 11, 1.f / 9), 1.f / 7), 0.2f), 1.f / 3);
+  const float rest = 2.0f * fmaf(a * w, c, fmaf(w, al, al));
+  const double ln = fma((double)q, 0.693147180559945309, (double)(2.0f * a) + (double)rest);
+  const double z = -6.666666666858372e-08 * ln, x = fma(0.5 * z, z, z);
+  return p + fma(p, fma(t, x, t) + x, pe);
 }
 
 // X[m][k] = sum of the corners' coordinates k weighted by the sign of
