@@ -2967,13 +2967,13 @@ WF_API wf_status wf_prepare_run(wf_domain *d, int64_t nsteps) {
   if (!d || nsteps < 0) return WF_ERR_ARG;
   if (!d->initialized) return fail(d, WF_ERR_STATE, "wf_init not called");
   if (!(d->dt > 0.0) && !d->nspec) return fail(d, WF_ERR_STATE, "time step not set (SetDT)");
-  // these runs replay no graph
-  if (d->phase_timing || cluster_mode(d) || tile_run_mode(d)) return WF_OK;
   CUDA_TRY(cudaSetDevice(d->device));
   {
     const wf_status gs = grow_history(d, d->host_step + nsteps);
     if (gs) return gs;
   }
+  // these runs replay no graph
+  if (d->phase_timing || cluster_mode(d) || tile_run_mode(d)) return WF_OK;
   set_dt_constants(d->P, d->dt);
   cudaGraphExec_t g = nullptr;
   if (nsteps >= kGraphSteps) {
