@@ -272,6 +272,7 @@ struct wf_domain {
   TileRunShape tr_shape;
   double *tr_part = nullptr;      // [kTileRunChunk][tiles] reaction partials
   unsigned *tr_bar = nullptr;     // the barrier's counter
+  unsigned tr_base = 0;           // what the next launch finds in it
   double *edge_min = nullptr;     // the shortest edge (wf_min_edge_length's device result)
   // batched ensemble
   int32_t nspec = 0;
@@ -2634,6 +2635,7 @@ WF_API wf_status wf_init(wf_domain *d) {
     const TileRunShape &C = d->tr_shape;
     CUDA_TRY(dalloc(d, &d->tr_part, (size_t)kTileRunChunk * C.ta * C.tb * C.tc));
     CUDA_TRY(dalloc(d, &d->tr_bar, 1));
+    d->tr_base = 0;
   }
   CUDA_TRY(cudaStreamSynchronize(d->stream));
   if (d->init_stage) CUDA_TRY(cudaFreeAsync(d->init_stage, d->stream));
@@ -2921,8 +2923,8 @@ WF_API wf_status wf_run(wf_domain *d, int64_t nsteps) {
   if (tile_run_mode(d)) {
     while (left > 0) {
       const int64_t chunk = std::min<int64_t>(left, kTileRunChunk);
-      CUDA_TRY(mix_tile_run(d->P, d->M, d->mvol, d->tr_part, d->tr_bar, chunk, d->tr_shape,
-                            d->stream));
+      CUDA_TRY(mix_tile_run(d->P, d->M, d->mvol, d->tr_part, d->tr_bar, d->tr_base, chunk,
+                            d->tr_shape, d->stream));
       d->launches += 1;
       left -= chunk;
     }
@@ -3247,6 +3249,10 @@ WF_API wf_status wf_sync(wf_domain *d) {
       d->st_host->status &= ~2u;
       CUDA_TRY(cudaMemcpy(&d->P.st->status, &d->st_host->status, sizeof(unsigned),
                           cudaMemcpyHostToDevice));
+      if (d->tile_run) {   // blocks left a tile run's barriers
+        CUDA_TRY(cudaMemsetAsync(d->tr_bar, 0, sizeof(unsigned), d->stream));
+        d->tr_base = 0;
+      }
       return fail(d, WF_ERR_TIMEOUT, "a wait inside a step's kernel ran out, in the steps up "
                                      "to step %lld", (long long)st.step);
     }

@@ -428,9 +428,12 @@ struct TileRunShape {
   int32_t ta = 0, tb = 0, tc = 0, e0 = 0, n1 = 0, e1 = 0, n2 = 0, chunk = 0, thermal = 0;
 };
 bool mix_tile_run_shape(const StepParams &P, TileRunShape &C);   // false: not run so
-// part: [chunk][tiles] reaction partials; bar: the barrier's counter.
+// part: [chunk][tiles] reaction partials; bar: the barrier's counter, base: what
+// it reads before the launch (advanced by the launch's arrivals; both start at 0
+// and again after a wait that ran out).
 cudaError_t mix_tile_run(const StepParams &P, const MixState &M, float *vol, double *part,
-                         unsigned *bar, int64_t nsteps, const TileRunShape &C, cudaStream_t st);
+                         unsigned *bar, unsigned &base, int64_t nsteps, const TileRunShape &C,
+                         cudaStream_t st);
 // The mixed state's displacements (or positions) as AoS [nn][3] doubles, as
 // the export forms them, without exporting the other fields.
 void mix_node_aos(const StepParams &P, const MixState &M, bool displacement, double *out,

@@ -2653,13 +2653,26 @@ __device__ __forceinline__ bool grid_barrier(unsigned *c, unsigned target, StepS
   if (threadIdx.x == 0) {
     red_release(c, 1u);
     int spins = 0, ok = 1;
-    while (ld_acquire(c) < target)
+    while ((int)(ld_acquire(c) - target) < 0)
       if (++spins > kGridSpin) {
         atomicOr(&st->status, 2u);
         ok = 0;
         break;
       }
     *s_ok = ok;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+// The block's arrival without a wait: whether it is the last of the launch, whose
+// threads then see what the others stored before theirs.
+__device__ __forceinline__ bool last_arrival(unsigned *c, unsigned target, int *s_ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;\n" : "=r"(old) : "l"(c) : "memory");
+    *s_ok = old + 1u == target;
   }
   __syncthreads();
   return *s_ok != 0;
@@ -2745,7 +2758,7 @@ struct TileRunNodes {
 template <int LAW, bool TH>
 __global__ void __launch_bounds__(kTileRunThreads + 32, 1)
     k_mix_tile_run(StepParams P, MixState M, float *vol, double *part, int64_t nsteps,
-                   unsigned *bar, TileRunShape C) {
+                   unsigned *bar, unsigned base, TileRunShape C) {
   constexpr int NT = kTileRunThreads;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ Block3 B[5];   // own elements, own nodes, corner nodes, ring elements, staged nodes
@@ -2765,32 +2778,43 @@ __global__ void __launch_bounds__(kTileRunThreads + 32, 1)
   const int64_t np = P.np, ne = P.ne;
   const int bx = P.bx, by = P.by, bz = P.bz;
   const int px = bx + 1, pxy = px * (by + 1);
-  if (t == 0) {
-    const int b = blockIdx.x, bi = b % C.ta, bj = (b / C.ta) % C.tb, bk = b / (C.ta * C.tb);
-    const int i0 = (int)((int64_t)bx * bi / C.ta), i1 = (int)((int64_t)bx * (bi + 1) / C.ta);
-    const int j0 = (int)((int64_t)by * bj / C.tb), j1 = (int)((int64_t)by * (bj + 1) / C.tb);
-    const int k0 = (int)((int64_t)bz * bk / C.tc), k1 = (int)((int64_t)bz * (bk + 1) / C.tc);
-    B[0].set(i0, i1, j0, j1, k0, k1);
-    // own nodes: the node grid cut as evenly (all of them among the tile's
-    // corner nodes, as (n + 1) b / t is less than one above n b / t)
-    auto cut = [](int n, int q, int parts) { return (int)((int64_t)(n + 1) * q / parts); };
-    B[1].set(cut(bx, bi, C.ta), cut(bx, bi + 1, C.ta), cut(by, bj, C.tb), cut(by, bj + 1, C.tb),
-             cut(bz, bk, C.tc), cut(bz, bk + 1, C.tc));
-    B[2].set(i0, i1 + 1, j0, j1 + 1, k0, k1 + 1);
-    const int ea = max(i0 - 1, 0), eb = min(i1 + 1, bx), fa = max(j0 - 1, 0),
-              fb = min(j1 + 1, by), ga = max(k0 - 1, 0), gb = min(k1 + 1, bz);
-    B[3].set(ea, eb, fa, fb, ga, gb);
-    B[4].set(ea, eb + 1, fa, fb + 1, ga, gb + 1);
+  const unsigned status = P.st->status;
+  if (t < 5) {
+    // a thread a block (32-bit products: at most 152 tiles of fewer than 8000 nodes)
+    const int b = blockIdx.x;
+    auto range = [&](int n, int q, int parts, int &lo, int &hi) {
+      lo = n * q / parts;
+      hi = n * (q + 1) / parts;
+      if (t == 1) {
+        // own nodes: the node grid cut as evenly (all of them among the tile's
+        // corner nodes, as (n + 1) q / parts is less than one above n q / parts)
+        lo = (n + 1) * q / parts;
+        hi = (n + 1) * (q + 1) / parts;
+      }
+      if (t >= 3) {
+        lo = max(lo - 1, 0);
+        hi = min(hi + 1, n);
+      }
+      if (t == 2 || t == 4) hi++;
+    };
+    int l[3], h[3];
+    range(bx, b % C.ta, C.ta, l[0], h[0]);
+    range(by, b / C.ta % C.tb, C.tb, l[1], h[1]);
+    range(bz, b / (C.ta * C.tb), C.tc, l[2], h[2]);
+    B[t].set(l[0], h[0], l[1], h[1], l[2], h[2]);
   }
   __syncthreads();
+  if (status & 2u) return;   // a wait of an earlier launch ran out: its counter is short
   const int me = B[0].count(), mo = B[1].count();
-  for (int q = t; q < me; q += NT + 32) {
+  // the stresses arrive with the first step's positions; a thread's elements are
+  // its own in the element phase as well
+  for (int q = t < NT ? t : me; q < me; q += NT) {
     int i, j, k;
     B[0].at(q, i, j, k);
     const int64_t e = B[0].i0 + i + (int64_t)bx * (B[0].j0 + j + (int64_t)by * (B[0].k0 + k));
 #pragma unroll
-    for (int c = 0; c < 6; c++) tau[c * C.e0 + q] = M.tau[c * ne + e];
-    tau[6 * C.e0 + q] = M.pls[e];
+    for (int c = 0; c < 6; c++) cp_async4(&tau[c * C.e0 + q], &M.tau[c * ne + e]);
+    cp_async4(&tau[6 * C.e0 + q], &M.pls[e]);
   }
   double time = 0.0;
   if (lane == 0) {
@@ -2820,7 +2844,7 @@ __global__ void __launch_bounds__(kTileRunThreads + 32, 1)
   // barriers only
   auto work_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); };
   __syncthreads();
-  unsigned target = 0;
+  unsigned target = base;
   for (int64_t it = 0; it < nsteps; it++) {
     const long long step = step0 + it;
     if (lane >= 0) {
@@ -2954,21 +2978,30 @@ __global__ void __launch_bounds__(kTileRunThreads + 32, 1)
     for (int c = 0; c < 6; c++) M.tau[c * ne + e] = tau[c * C.e0 + q];
     M.pls[e] = tau[6 * C.e0 + q];
   }
-  if (!grid_barrier(bar, target += gridDim.x, P.st, &s_ok)) return;
-  // reaction history: block partials of each step added in block order
-  if (blockIdx.x == 0) {
-    for (int64_t it = t; it < nsteps; it += NT + 32) {
-      double tot = 0.0;
-      for (unsigned i = 0; i < gridDim.x; i++) {
-        const double v = part[it * gridDim.x + i];
-        if (__double_as_longlong(v) << 1 != 0) tot += v;
+  // reaction history, by the block that arrives last: a warp a step, lanes over
+  // the blocks, then a fixed tree. (One thread a step, adding 152 partials one
+  // after the other, was a third of a run of one step.)
+  if (!last_arrival(bar, target + gridDim.x, &s_ok)) return;
+  for (int64_t it = t >> 5; it < nsteps; it += (NT + 32) / 32) {
+    double tot = 0.0;
+    bool any = false;
+#pragma unroll 4
+    for (unsigned i = t & 31; i < gridDim.x; i += 32) {
+      const double v = __ldcg(&part[it * gridDim.x + i]);
+      if (__double_as_longlong(v) << 1 != 0) {
+        tot += v;
+        any = true;
       }
-      if (step0 + it < P.hist_cap) P.hist[step0 + it] = tot;
     }
-    if (lane == 0) {
-      P.st->step = step0 + nsteps;
-      P.st->time = time;
+    if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) tot += __shfl_down_sync(0xffffffffu, tot, o);
     }
+    if ((t & 31) == 0 && step0 + it < P.hist_cap) P.hist[step0 + it] = tot;
+  }
+  if (lane == 0) {
+    P.st->step = step0 + nsteps;
+    P.st->time = time;
   }
 }
 
@@ -3599,7 +3632,7 @@ cudaError_t mix_cluster_run(const StepParams &P, const MixState &M, float *vol, 
 
 namespace {
 using TileRunKernel = void (*)(StepParams, MixState, float *, double *, int64_t, unsigned *,
-                               TileRunShape);
+                               unsigned, TileRunShape);
 TileRunKernel tile_run_kernel(const StepParams &P) {
   if (P.thermal) return P.mat_general ? k_mix_tile_run<1, true> : k_mix_tile_run<0, true>;
   return P.mat_general ? k_mix_tile_run<1, false> : k_mix_tile_run<0, false>;
@@ -3668,9 +3701,8 @@ bool mix_tile_run_shape(const StepParams &P, TileRunShape &C) {
 }
 
 cudaError_t mix_tile_run(const StepParams &P, const MixState &M, float *vol, double *part,
-                         unsigned *bar, int64_t nsteps, const TileRunShape &C, cudaStream_t st) {
-  const cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(unsigned), st);
-  if (e != cudaSuccess) return e;
+                         unsigned *bar, unsigned &base, int64_t nsteps, const TileRunShape &C,
+                         cudaStream_t st) {
   const TileRunKernel k = tile_run_kernel(P);
   const int bytes = TileRunSmem(C).total;
   const cudaError_t a = allow_smem((const void *)k, kTileRunSmemMax);
@@ -3685,7 +3717,10 @@ cudaError_t mix_tile_run(const StepParams &P, const MixState &M, float *vol, dou
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, P, M, vol, part, nsteps, bar, C);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k, P, M, vol, part, nsteps, bar, base, C);
+  // two barriers a step and the last arrival; the counter wraps
+  if (e == cudaSuccess) base += (unsigned)(2 * nsteps + 1) * cfg.gridDim.x;
+  return e;
 }
 
 void mix_predict(const StepParams &P, const MixState &M, cudaStream_t st) {
