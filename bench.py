@@ -282,6 +282,7 @@ def run_ours(args):
     stream = torch.cuda.ExternalStream(dm.stream_handle(), device=device)
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     mode, cl_blocks, cl_bs = dm.step_mode()
+    kernels = dm.run_kernels(K)
     tile_stats = dm.tile_stats()
     barrier()
     torch.cuda.synchronize(device)
@@ -456,8 +457,8 @@ def run_ours(args):
                                 "the run), displacement readback into a pinned host buffer + "
                                 "reaction readback"},
             "gpu_launches": int(launches),
-            "step_mode": step_mode_label(mode, cl_blocks, cl_bs, K, graph_replays, launches,
-                                         tile_stats),
+            "step_mode": step_mode_label(mode, kernels, cl_blocks, cl_bs, K, graph_replays,
+                                         launches, tile_stats),
             "autotuned_launch": tuned,
             "launch_note": "items_per_thread 0 = persistent grid (SMs x resident blocks)",
             "roofline": roof,
@@ -471,12 +472,17 @@ def run_ours(args):
         dist.destroy_process_group()
 
 
-def step_mode_label(mode, cl_blocks, cl_bs, K, graph_replays, launches, tile_stats=None):
+def step_mode_label(mode, kernels, cl_blocks, cl_bs, K, graph_replays, launches,
+                    tile_stats=None):
     """What the timed wf_run(K) launched, as counted by the library."""
-    if mode == 2:
-        return {"mode": "one cluster launch per run", "cluster_blocks": cl_blocks,
-                "block_size": cl_bs, "kernel_launches": int(launches),
-                "note": "roofline phases are the per-phase kernels, timed apart"}
+    note = "roofline phases are the per-phase kernels, timed apart"
+    if kernels in ("cluster", "cluster_smem"):
+        shape = {"cluster_blocks": cl_blocks, "block_size": cl_bs} if mode == 2 else {}
+        return {"mode": "one cluster launch per run", **shape, "kernel_launches": int(launches),
+                "note": note}
+    if kernels == "tile_run":
+        return {"mode": "one cooperative launch over tiles per 256 steps",
+                "kernel_launches": int(launches), "note": note}
     full, rem = divmod(K, 32)
     kernels = ("geometry, nodal, tiled element+assembly, shared-node kernels" if mode == 3
                else "geometry, nodal, column-sweep kernels" if mode == 4
@@ -726,7 +732,7 @@ def run_adjoint(args):
                        "forward_over_forward": round(ms_ka / ms_fwd, 3),
                        "backward_fp64_over_forward": round(ms_kb / ms_fwd, 3),
                        "backward_fp32_over_forward": round(ms_kb32 / ms_fwd, 3),
-                       "stash_gb": round(N * (14 * case.n_node + 7 * E) * 8 / 1e9, 2)}},
+                       "stash_gb": round(N * (11 * case.n_node + 7 * E) * 8 / 1e9, 2)}},
         "element_steps_per_s_forward_fp64": round(E * N / (ms_fwd * 1e-3), 1),
         "loss": loss,
         "gradient_fd_check": fd,

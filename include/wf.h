@@ -434,18 +434,37 @@ WF_API wf_status wf_set_launch_config(wf_domain *d, int32_t phase, int32_t block
  * picks mode 2 for meshes of at most 3000 elements, or of at most 6500
  * hexahedra whose run fits the cluster's shared memory; else, for box meshes of
  * hexahedra whose tiles fit the SMs' shared memory (up to about 230,000; with
- * thermal coupling 185,000; no specimens, energy history or phase timing), whole spans of steps as one
- * cooperative launch, each block keeping its tile's stresses on the chip, with
- * two bounded barriers over the grid a step (mode 1's arithmetic and order of
- * sums; a barrier that runs out makes wf_sync return WF_ERR_TIMEOUT); else mode
- * 4 where the mesh is swept and its columns fill the GPU (at least 95 % of two
+ * thermal coupling 185,000; no specimens, energy history or phase timing), whole
+ * spans of steps as one cooperative launch, each block keeping its tile's
+ * stresses on the chip, with two bounded barriers over the grid a step (mode 1's
+ * arithmetic, the state bitwise; the reaction sum runs in another order; a
+ * barrier that runs out makes wf_sync return WF_ERR_TIMEOUT); else mode 4 where the mesh is swept and its columns fill the GPU (at least 95 % of two
  * per SM: a column is a sequence of layers), else mode 1.
- * wf_get_step_mode reports the mode the next wf_run uses (1 for the cooperative
- * launch and for a cluster run of more than 3000 elements) and, for mode 2, the
- * cluster's blocks and block size, for mode 3 the tiles and threads per tile,
- * for mode 4 the columns and threads per column, for mode 5 the blocks and
- * threads per block (0 otherwise). */
+ * wf_get_step_mode reports the mode whose arithmetic and order of sums over
+ * elements the next wf_run has (1 also for the cooperative launch and for a
+ * cluster run of more than 3000 elements; wf_get_run_kernels tells them apart)
+ * and, for mode 2, the cluster's blocks and block size, for mode 3 the tiles and
+ * threads per tile, for mode 4 the columns and threads per column, for mode 5 the
+ * blocks and threads per block (0 otherwise). */
 WF_API wf_status wf_set_step_mode(wf_domain *d, int32_t mode);
+/* No counterpart in the reference. Which kernels the next wf_run(d, nsteps)
+ * launches, of an initialised domain. */
+typedef enum {
+  WF_RUN_PHASES = 1,       /* the per-phase kernels (graphs or direct launches) */
+  WF_RUN_CLUSTER = 2,      /* the cluster run through L2 */
+  WF_RUN_TILED = 3,        /* the tiled kernels of mode 3 */
+  WF_RUN_SWEEP = 4,        /* the column sweep */
+  WF_RUN_FLOW = 5,         /* the dataflow step */
+  WF_RUN_CLUSTER_SMEM = 6, /* the cluster run with its state in shared memory */
+  WF_RUN_TILE_RUN = 7      /* the cooperative launch over tiles */
+} wf_run_kernels;
+WF_API wf_status wf_get_run_kernels(const wf_domain *d, int64_t nsteps, int32_t *kernels);
+/* No counterpart in the reference. What wf_init chose for the mixed kernels'
+ * gathers: the width of the node lists kept by position (0: the lists laid end
+ * to end, or computed), and whether the specimens' corners and lists are
+ * computed from their boxes (else from the arrays). Any output may be NULL. */
+WF_API wf_status wf_get_index_tables(const wf_domain *d, int32_t *list_width,
+                                     int32_t *specimen_boxes);
 /* No counterpart in the reference. Node rows per column of the column sweep
  * (4 or 8, default 8), before wf_init. wf_get_sweep: the columns along x and
  * y and the rows per column, or zeros and, in why (NUL-terminated, at most

@@ -28,6 +28,8 @@ STATUS = {0: "ok", 1: "invalid argument", 2: "call out of order", 3: "CUDA error
           7: "device wait timed out"}
 
 NODE_VEC = {"x": 0, "v": 1, "a": 2, "u": 3, "prev_a": 4, "fi": 5, "contforce": 7}
+RUN_KERNELS = {1: "phases", 2: "cluster", 3: "tiled", 4: "sweep", 5: "flow", 6: "cluster_smem",
+               7: "tile_run"}
 NODE_SCALAR = {"mass": 0, "voln": 1, "p_node": 2, "T": 3}
 ELEM_SCALAR = {"vol": 0, "vol0": 1, "detJ": 2, "p": 3, "pl_strain": 4, "sigma_y": 5, "rho": 6}
 ELEM_TENSOR = {"sigma": 0, "tau": 1, "eps": 2, "str_rate": 3, "rot_rate": 4}
@@ -137,6 +139,8 @@ _SIGS = {
     "wf_set_step_mode": [C.c_void_p, C.c_int32],
     "wf_get_step_mode": [C.c_void_p, C.POINTER(C.c_int32), C.POINTER(C.c_int32),
                          C.POINTER(C.c_int32)],
+    "wf_get_run_kernels": [C.c_void_p, C.c_int64, C.POINTER(C.c_int32)],
+    "wf_get_index_tables": [C.c_void_p, C.POINTER(C.c_int32), C.POINTER(C.c_int32)],
     "wf_set_box_indexing": [C.c_void_p, C.c_int32],
     "wf_set_sweep_rows": [C.c_void_p, C.c_int32],
     "wf_get_halo_node_width": [C.c_void_p, C.POINTER(C.c_int32)],
@@ -536,6 +540,18 @@ class Domain:
         m, b, t = C.c_int32(), C.c_int32(), C.c_int32()
         self._call("wf_get_step_mode", C.byref(m), C.byref(b), C.byref(t))
         return m.value, b.value, t.value
+
+    def run_kernels(self, n):
+        """Which kernels run(n) launches: a name of RUN_KERNELS."""
+        k = C.c_int32()
+        self._call("wf_get_run_kernels", int(n), C.byref(k))
+        return RUN_KERNELS[k.value]
+
+    def index_tables(self):
+        """(width of the node lists by position or 0, specimens indexed as boxes)."""
+        w, b = C.c_int32(), C.c_int32()
+        self._call("wf_get_index_tables", C.byref(w), C.byref(b))
+        return w.value, bool(b.value)
 
     def set_launch_config(self, phase, block, items_per_thread):
         """Launch shape of phase 0/1/2 (items_per_thread 0: persistent grid)."""

@@ -273,6 +273,7 @@ struct wf_domain {
   double *tr_part = nullptr;      // [kTileRunChunk][tiles] reaction partials
   unsigned *tr_bar = nullptr;     // the barrier's counter
   unsigned tr_base = 0;           // what the next launch finds in it
+  int32_t cols_width = 0;         // entries a node of the lists by position (P.cols)
   double *edge_min = nullptr;     // the shortest edge (wf_min_edge_length's device result)
   // batched ensemble
   int32_t nspec = 0;
@@ -1805,6 +1806,15 @@ bool tile_run_mode(const wf_domain *d) {
   return d->precision == WF_MIXED && d->step_mode == 0 && d->tile_run && !d->P.energy_on &&
          !d->phase_timing && !cluster_mode(d) && !tiled_mode(d) && !flow_mode(d) && !sweep_mode(d);
 }
+// The kernels of a run of nsteps steps (wf_run and wf_get_run_kernels).
+wf_run_kernels run_kernels(const wf_domain *d, int64_t nsteps) {
+  (void)nsteps;
+  if (cluster_mode(d)) return d->cl_smem ? WF_RUN_CLUSTER_SMEM : WF_RUN_CLUSTER;
+  if (tile_run_mode(d)) return WF_RUN_TILE_RUN;
+  if (tiled_mode(d)) return WF_RUN_TILED;
+  if (flow_mode(d)) return WF_RUN_FLOW;
+  return sweep_mode(d) ? WF_RUN_SWEEP : WF_RUN_PHASES;
+}
 }  // namespace
 
 WF_API wf_status wf_set_step_mode(wf_domain *d, int32_t mode) {
@@ -1829,6 +1839,22 @@ WF_API wf_status wf_get_step_mode(const wf_domain *d, int32_t *mode, int32_t *bl
   if (block_size)
     *block_size =
         c ? d->cl_bs : (t ? kTileElems : (f ? 256 : (w ? 32 * (d->W.cy + 1) : 0)));
+  return WF_OK;
+}
+
+WF_API wf_status wf_get_run_kernels(const wf_domain *d, int64_t nsteps, int32_t *kernels) {
+  if (!d || !kernels || nsteps < 0) return WF_ERR_ARG;
+  if (!d->initialized) return WF_ERR_STATE;
+  *kernels = run_kernels(d, nsteps);
+  return WF_OK;
+}
+
+WF_API wf_status wf_get_index_tables(const wf_domain *d, int32_t *list_width,
+                                     int32_t *specimen_boxes) {
+  if (!d) return WF_ERR_ARG;
+  if (!d->initialized) return WF_ERR_STATE;
+  if (list_width) *list_width = d->P.cols ? d->cols_width : 0;
+  if (specimen_boxes) *specimen_boxes = d->P.sbox ? 1 : 0;
   return WF_OK;
 }
 
@@ -2126,6 +2152,7 @@ WF_API wf_status wf_init(wf_domain *d) {
         list_cols(off, sl, nn, np, most, cols, d->stream);
         CUDA_TRY(cudaGetLastError());
         P.cols = cols;
+        d->cols_width = most;
       }
     }
   }
@@ -2906,11 +2933,13 @@ WF_API wf_status wf_run(wf_domain *d, int64_t nsteps) {
     return fail(d, WF_ERR_UNSUPPORTED,
                 "the cluster run needs mixed precision, a mesh of at most %lld elements, and no "
                 "specimens, energy history or phase timing", (long long)kClusterMaxElems);
-  if (cluster_mode(d)) {
+  const wf_run_kernels kern = run_kernels(d, nsteps);
+  if (kern == WF_RUN_CLUSTER || kern == WF_RUN_CLUSTER_SMEM) {
     // one launch per chunk of steps (kernels stay short)
+    const bool smem = kern == WF_RUN_CLUSTER_SMEM;
     while (left > 0) {
-      const int64_t chunk = std::min<int64_t>(left, d->cl_smem ? kClusterSmemChunk : kClusterChunk);
-      if (d->cl_smem)
+      const int64_t chunk = std::min<int64_t>(left, smem ? kClusterSmemChunk : kClusterChunk);
+      if (smem)
         CUDA_TRY(mix_cluster_smem_run(d->P, d->M, d->mvol, chunk, d->cl_blocks, d->cl_bs,
                                       d->cl_shape, d->stream));
       else
@@ -2920,7 +2949,7 @@ WF_API wf_status wf_run(wf_domain *d, int64_t nsteps) {
       left -= chunk;
     }
   }
-  if (tile_run_mode(d)) {
+  if (kern == WF_RUN_TILE_RUN) {
     while (left > 0) {
       const int64_t chunk = std::min<int64_t>(left, kTileRunChunk);
       CUDA_TRY(mix_tile_run(d->P, d->M, d->mvol, d->tr_part, d->tr_bar, d->tr_base, chunk,
@@ -2975,7 +3004,10 @@ WF_API wf_status wf_prepare_run(wf_domain *d, int64_t nsteps) {
     if (gs) return gs;
   }
   // these runs replay no graph
-  if (d->phase_timing || cluster_mode(d) || tile_run_mode(d)) return WF_OK;
+  const wf_run_kernels kern = run_kernels(d, nsteps);
+  if (d->phase_timing || kern == WF_RUN_CLUSTER || kern == WF_RUN_CLUSTER_SMEM ||
+      kern == WF_RUN_TILE_RUN)
+    return WF_OK;
   set_dt_constants(d->P, d->dt);
   cudaGraphExec_t g = nullptr;
   if (nsteps >= kGraphSteps) {
