@@ -433,8 +433,8 @@ WF_API wf_status wf_set_launch_config(wf_domain *d, int32_t phase, int32_t block
  * than the L2 reuse saves) and is only run when asked for. Mode 0 (default)
  * picks mode 2 for meshes of at most 3000 elements, or of at most 6500
  * hexahedra whose run fits the cluster's shared memory; else, for box meshes of
- * hexahedra whose tiles fit the SMs' shared memory (up to about 230,000; with
- * thermal coupling 185,000; no specimens, energy history or phase timing), whole
+ * hexahedra whose tiles are small enough (up to 180,000, boxes narrow along x up
+ * to 270,000; no specimens, energy history or phase timing), whole
  * spans of steps as one cooperative launch, each block keeping its tile's
  * stresses on the chip, with two bounded barriers over the grid a step (mode 1's
  * arithmetic, the state bitwise; the reaction sum runs in another order; a

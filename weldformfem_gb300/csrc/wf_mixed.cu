@@ -2621,8 +2621,8 @@ __global__ void __launch_bounds__(BS + 32, 1) k_mix_cluster_smem(StepParams P, M
 
 // ---------------------------------------------------------------------------
 // Tile run of box meshes: a whole run of steps in one cooperative launch, one
-// block per SM, for boxes between the cluster run's size and what fits in the
-// SMs' shared memory (about 230,000 hexahedra). There a step's four kernels
+// block per SM, for boxes between the cluster run's size and what a block's threads
+// go through in two or three passes (mix_tile_run_shape). There a step's four kernels
 // were launch, ramp-up and two or three dependent L2 round trips each: 20 to 25
 // us for a few microseconds of work. A block owns a tile of elements (and the
 // a share of the nodes), and a step is two phases with a barrier over the
@@ -3681,11 +3681,15 @@ bool mix_tile_run_shape(const StepParams &P, TileRunShape &C) {
       }
     }
   if (!found) return false;
-  // thermal elements in more than two passes are faster per phase (Johnson-Cook,
-  // tile run and per phase: 168,000 in two passes 32.7 and 34.4 us a step, 195,000
-  // in three 38.0 and 38.3, 226,000 47.5 and 44.4; without heat 226,000 take 27.7
-  // and 29.9)
-  if (P.thermal && C.e0 > 2 * kTileRunThreads) return false;
+  // Where the tile run ends: three passes of the working threads over the
+  // elements pay only where the tiles keep whole rows along x (a cut row starts
+  // within a sector at both ends), four and, with heat, three do not. us a step of
+  // the tile run and per phase, bilinear: two passes 162,540 19.3 and 22.7; three,
+  // whole rows 256,500 28.8 and 30.2, 246,120 24.9 and 28.7; three, cut rows
+  // 226,920 27.4 and 27.1, 229,824 29.9 and 27.3, 252,000 33.7 and 29.3; four
+  // 270,336 37.9 and 30.4. Johnson-Cook with heat: two passes 168,000 32.7 and
+  // 34.4, three 195,000 38.0 and 38.3, 226,000 47.5 and 44.4.
+  if (C.e0 > (P.thermal || C.ta > 1 ? 2 : 3) * kTileRunThreads) return false;
   const TileRunKernel k = tile_run_kernel(P);
   const int bytes = TileRunSmem(C).total;
   int dev = 0, coop = 0, per = 0;
