@@ -431,8 +431,9 @@ WF_API wf_status wf_set_launch_config(wf_domain *d, int32_t phase, int32_t block
  * expected) makes the next wf_sync return WF_ERR_TIMEOUT. On GB300 mode 5 is
  * slower than modes 4 and 1 (the blocks' waits and ticket traffic cost more
  * than the L2 reuse saves) and is only run when asked for. Mode 0 (default)
- * picks mode 2 for meshes of at most 3000 elements, or of at most 6500
- * hexahedra whose run fits the cluster's shared memory; else, for box meshes of
+ * picks mode 2 for meshes of at most 3000 elements, and for runs of 5 steps and
+ * more of at most 6500 hexahedra that fit the cluster's shared memory (8 and 4096
+ * nodes for a box mesh); else, for box meshes of
  * hexahedra whose tiles are small enough (up to 180,000, boxes narrow along x up
  * to 270,000; no specimens, energy history or phase timing), whole
  * spans of steps as one cooperative launch, each block keeping its tile's

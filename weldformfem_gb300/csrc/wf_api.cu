@@ -1732,11 +1732,21 @@ WF_API wf_status wf_set_launch_config(wf_domain *d, int32_t phase, int32_t block
 // automatic mode uses it.
 constexpr int64_t kClusterMaxElems = 65536;
 constexpr int64_t kClusterAutoElems = 3000;
-// With the state in shared memory the cluster run stays ahead further: 7.2
-// against 13.3 us a step at 4096 hexahedra, 8.6 against 13.4 at 5832 (8000 no
-// longer fit). Past kClusterAutoElems it is reported as the per-phase mode it
-// replaces, whose arithmetic it runs.
+// With the state in shared memory the cluster run stays ahead further. Against the
+// per-phase kernels: 7.1 and 12.6 us a step at 4096 hexahedra, 8.5 and 12.9 at 5832
+// (8000 no longer fit). Against the tile run of box meshes it is ahead while its
+// threads take an element and a node each: 5.65 and 7.1 us at 3375 hexahedra (4096
+// nodes on 4096 threads), 7.1 and 7.0 at 4096 (4913 nodes), 8.2 and 7.2 at 4913.
+// Past kClusterAutoElems it is reported as the per-phase mode it replaces, whose
+// arithmetic it runs.
 constexpr int64_t kClusterSmemElems = 6500;
+// Its set-up costs some 20 us a run, more than the other kernels', so runs of few
+// steps take those: below kClusterAutoElems the cluster run through L2 (2744
+// hexahedra, us a run of 1, 2, 3 steps: 27, 36, 49 through L2, 36, 40, 42 with the
+// state in shared memory), past it the tile run (3375: 27, 33, 40 and 4 more steps
+// at 7; here 31 and 5.65 a step) or the per-phase kernels (4096, 3, 4, 8 steps: 53,
+// 65, 115 and here 54, 66, 92).
+constexpr int64_t kClusterSmemSteps = 3, kClusterSmemStepsTile = 8, kClusterSmemStepsPast = 5;
 // Meshes of tetrahedra with this many nodes and more keep their node lists by
 // position as well in the mixed step (NodeSlots): it costs 0.13 ms of init on
 // 576,000 tetrahedra, and below a step's kernels wait for launches, not for loads.
@@ -1748,8 +1758,11 @@ namespace {
 bool cluster_mode(const wf_domain *d) {
   if (d->precision != WF_MIXED || d->nspec || d->P.energy_on || d->phase_timing || !d->cl_blocks)
     return false;
-  return d->step_mode == 2 ||
-         (d->step_mode == 0 && d->ne <= (d->cl_smem ? kClusterSmemElems : kClusterAutoElems));
+  if (d->step_mode == 2) return true;
+  if (d->step_mode != 0) return false;
+  if (d->ne <= kClusterAutoElems) return true;
+  if (!d->cl_smem || d->ne > kClusterSmemElems) return false;
+  return !d->tile_run || std::max(d->ne, d->nn) <= (int64_t)d->cl_blocks * d->cl_bs;
 }
 // Whether the automatic mode picks the tiled kernels for tiled meshes.
 constexpr bool kTiledAuto = false;
@@ -1804,16 +1817,27 @@ namespace {
 // (reported as mode 1, whose arithmetic it is).
 bool tile_run_mode(const wf_domain *d) {
   return d->precision == WF_MIXED && d->step_mode == 0 && d->tile_run && !d->P.energy_on &&
-         !d->phase_timing && !cluster_mode(d) && !tiled_mode(d) && !flow_mode(d) && !sweep_mode(d);
+         !d->phase_timing && !tiled_mode(d) && !flow_mode(d) && !sweep_mode(d);
 }
 // The kernels of a run of nsteps steps (wf_run and wf_get_run_kernels).
 wf_run_kernels run_kernels(const wf_domain *d, int64_t nsteps) {
-  (void)nsteps;
-  if (cluster_mode(d)) return d->cl_smem ? WF_RUN_CLUSTER_SMEM : WF_RUN_CLUSTER;
+  if (cluster_mode(d)) {
+    const bool past = d->step_mode == 0 && d->ne > kClusterAutoElems;
+    const int64_t least = !past ? kClusterSmemSteps
+                                : d->tile_run ? kClusterSmemStepsTile : kClusterSmemStepsPast;
+    if (d->cl_smem && nsteps >= least) return WF_RUN_CLUSTER_SMEM;
+    if (!past) return WF_RUN_CLUSTER;
+  }
   if (tile_run_mode(d)) return WF_RUN_TILE_RUN;
   if (tiled_mode(d)) return WF_RUN_TILED;
   if (flow_mode(d)) return WF_RUN_FLOW;
   return sweep_mode(d) ? WF_RUN_SWEEP : WF_RUN_PHASES;
+}
+// The reaction partials of the cluster run through L2, allocated by the first run
+// that needs them.
+cudaError_t cluster_partials(wf_domain *d, wf_run_kernels kern) {
+  if (kern != WF_RUN_CLUSTER || d->cl_part) return cudaSuccess;
+  return dalloc_raw(d, &d->cl_part, (size_t)kClusterChunk * d->cl_blocks);
 }
 }  // namespace
 
@@ -2633,6 +2657,7 @@ WF_API wf_status wf_init(wf_domain *d) {
       if (ts) return ts;
     }
     d->cl_blocks = d->cl_bs = 0;
+    d->cl_part = nullptr;
     d->cl_smem = false;
     if (d->ne <= kClusterMaxElems && !d->nspec) {
       // the largest cluster (16 blocks needs the non-portable size) that
@@ -2651,7 +2676,6 @@ WF_API wf_status wf_init(wf_domain *d) {
             d->cl_smem = mix_cluster_smem_fits(P, M, d->mvol, blocks, bs, most[0], most[1], most[2],
                                                d->cl_shape);
           }
-          if (!d->cl_smem) CUDA_TRY(dalloc(d, &d->cl_part, (size_t)kClusterChunk * blocks));
           break;
         }
       }
@@ -2934,6 +2958,7 @@ WF_API wf_status wf_run(wf_domain *d, int64_t nsteps) {
                 "the cluster run needs mixed precision, a mesh of at most %lld elements, and no "
                 "specimens, energy history or phase timing", (long long)kClusterMaxElems);
   const wf_run_kernels kern = run_kernels(d, nsteps);
+  CUDA_TRY(cluster_partials(d, kern));
   if (kern == WF_RUN_CLUSTER || kern == WF_RUN_CLUSTER_SMEM) {
     // one launch per chunk of steps (kernels stay short)
     const bool smem = kern == WF_RUN_CLUSTER_SMEM;
@@ -3005,6 +3030,7 @@ WF_API wf_status wf_prepare_run(wf_domain *d, int64_t nsteps) {
   }
   // these runs replay no graph
   const wf_run_kernels kern = run_kernels(d, nsteps);
+  CUDA_TRY(cluster_partials(d, kern));
   if (d->phase_timing || kern == WF_RUN_CLUSTER || kern == WF_RUN_CLUSTER_SMEM ||
       kern == WF_RUN_TILE_RUN)
     return WF_OK;
