@@ -414,7 +414,9 @@ constexpr int kClusterSmemChunk = 1024;
 struct ClusterShape {
   int32_t nn = 0, ne = 0, mc = 0, nc = 0, nt = 0, words = 0, chunk = 0;
 };
-// Whether it runs this domain (fills C from the blocks' largest counts).
+// Whether it might run this domain, from the mesh's size alone, and whether it
+// does (fills C from the blocks' largest counts).
+bool mix_cluster_smem_may_fit(const StepParams &P, int blocks, int bs);
 bool mix_cluster_smem_fits(const StepParams &P, const MixState &M, float *vol, int blocks, int bs,
                            int64_t max_list, int64_t max_copies, int64_t max_targets,
                            ClusterShape &C);

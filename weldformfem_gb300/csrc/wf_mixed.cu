@@ -3598,18 +3598,35 @@ int mix_cluster_fits(const StepParams &P, const MixState &M, float *vol, int blo
   return fits;
 }
 
-bool mix_cluster_smem_fits(const StepParams &P, const MixState &M, float *vol, int blocks, int bs,
-                           int64_t max_list, int64_t max_copies, int64_t max_targets,
-                           ClusterShape &C) {
-  if (P.npe != 8 || P.thermal || P.tri_on) return false;
+namespace {
+bool cluster_shape(const StepParams &P, int blocks, int bs, int64_t max_list, int64_t max_copies,
+                   int64_t max_targets, ClusterShape &C) {
   C.nn = (int)((P.nn + blocks - 1) / blocks);
   C.ne = (int)((P.ne + blocks - 1) / blocks);
+  // in 64 bits: a node of many elements would wrap SmemRun's byte counts
+  if (16 * max_list * C.nn > kClusterSmemMax || max_copies > kClusterSmemMax ||
+      max_targets > kClusterSmemMax || P.nn > 16 * kClusterSmemMax)
+    return false;
   C.mc = (int)max_list;
   C.nc = (int)max_copies;
   C.nt = (int)max_targets;
   C.words = (int)((P.nn + 31) / 32);
   C.chunk = kClusterSmemChunk;
-  if (SmemRun(C, bs).total > kClusterSmemMax) return false;
+  return SmemRun(C, bs).total <= kClusterSmemMax;
+}
+}  // namespace
+
+bool mix_cluster_smem_may_fit(const StepParams &P, int blocks, int bs) {
+  ClusterShape C;
+  // the longest list is at least the mean
+  return P.npe == 8 && !P.thermal && !P.tri_on &&
+         cluster_shape(P, blocks, bs, (8 * P.ne + P.nn - 1) / P.nn, 0, 0, C);
+}
+
+bool mix_cluster_smem_fits(const StepParams &P, const MixState &M, float *vol, int blocks, int bs,
+                           int64_t max_list, int64_t max_copies, int64_t max_targets,
+                           ClusterShape &C) {
+  if (!cluster_shape(P, blocks, bs, max_list, max_copies, max_targets, C)) return false;
   int fits = 0;
   const cudaError_t e =
       P.mat_general ? smem_dispatch<1>(P, M, vol, 0, blocks, bs, C, nullptr, true, &fits)
