@@ -2436,8 +2436,8 @@ WF_API wf_status wf_init(wf_domain *d) {
     }
     CUDA_TRY(dalloc(d, &S.sr, 6 * ne));
     CUDA_TRY(dalloc(d, &S.rr, 6 * ne));
-    CUDA_TRY(dalloc_raw(d, &S.adj, (size_t)ne * (d->npe == 8 ? 9 : 10)));
     CUDA_TRY(dalloc(d, &S.fe, (size_t)ne * d->npe * 3));
+    S.adj = S.fe;
     if (P.hg_on) CUDA_TRY(dalloc(d, &S.fhg, (size_t)ne * d->npe * 3));
   }
   CUDA_TRY(dalloc_raw(d, &d->rho0_dev, ne));
@@ -2452,7 +2452,9 @@ WF_API wf_status wf_init(wf_domain *d) {
     // initial volumes, densities, nodal volumes and masses (CalcElemInitialVol,
     // calcElemDensity, CalcNodalVol, CalcNodalMassFromVol); the mixed state
     // forms its own in FP32 (mix_init)
-    fp64_geometry(P, S, d->stream, true);
+    Fp64State pre = S;
+    pre.adj = nullptr;   // no element forces yet
+    fp64_geometry(P, pre, d->stream, true);
     CUDA_TRY(cudaMemcpyAsync(S.vol0, S.vol, sizeof(double) * ne, cudaMemcpyDeviceToDevice,
                              d->stream));
     fp64_density(P, S, d->rho0_dev, d->stream);
@@ -3481,8 +3483,10 @@ WF_API wf_status wf_get_elem_scalar(wf_domain *d, int32_t field, double *out) {
     default: return fail(d, WF_ERR_ARG, "unknown element scalar %d", field);
   }
   if (field == WF_ELEM_DETJ) {
-    // refresh detJ for the current coordinates
-    fp64_geometry(d->P, d->S, d->stream, true);
+    // refresh detJ for the current coordinates; the element forces stay
+    Fp64State now = S;
+    now.adj = nullptr;
+    fp64_geometry(d->P, now, d->stream, true);
     CUDA_TRY(cudaGetLastError());
   }
   return copy_plain(d, src, out, d->ne);

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_geometry(StepParams P, Fp
   }
   S.vol[e] = v;
   if (store_detj) S.detJ[e] = detJ;
-  if (!S.adj) return;   // the preamble of a mixed domain, or its detJ readback
+  if (!S.adj) return;   // the preamble, or a detJ readback
 #pragma unroll
   for (int k = 0; k < 3; k++)
 #pragma unroll
@@ -501,14 +501,14 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_tets(StepParams P, Fp64St
   double dH[3][NPE];
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    const double a0 = __ldg(&S.adj[(3 * k) * ne + e]), a1 = __ldg(&S.adj[(3 * k + 1) * ne + e]),
-                 a2 = __ldg(&S.adj[(3 * k + 2) * ne + e]);
+    const double a0 = S.adj[(3 * k) * ne + e], a1 = S.adj[(3 * k + 1) * ne + e],
+                 a2 = S.adj[(3 * k + 2) * ne + e];
     dH[k][0] = -a0 - a1 - a2;
     dH[k][1] = a0;
     dH[k][2] = a1;
     dH[k][3] = a2;
   }
-  const double detJ = __ldg(&S.adj[9 * ne + e]);
+  const double detJ = S.adj[9 * ne + e];
   const double vol = __ldg(&S.vol[e]);
   const int32_t mat_id = P.emat ? __ldg(&P.emat[e]) : 0;
   const MatDev m = P.mats[mat_id];
@@ -650,8 +650,8 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_tets_thermal(StepParams P
 #pragma unroll
   for (int k = 0; k < 3; k++)
 #pragma unroll
-    for (int mm = 0; mm < 3; mm++) A[k][mm] = __ldg(&S.adj[(3 * k + mm) * ne + e]);
-  const double detJ = __ldg(&S.adj[9 * ne + e]), vol = __ldg(&S.vol[e]);
+    for (int mm = 0; mm < 3; mm++) A[k][mm] = S.adj[(3 * k + mm) * ne + e];
+  const double detJ = S.adj[9 * ne + e], vol = __ldg(&S.vol[e]);
   const int32_t mat_id = P.emat ? __ldg(&P.emat[e]) : 0;
   const MatDev &m = P.mats[mat_id];
   const double f = 1.0 / detJ, fh = 0.5 * f;
@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_hexes(StepParams P, Fp64S
 #pragma unroll
   for (int k = 0; k < 3; k++)
 #pragma unroll
-    for (int mm = 0; mm < 3; mm++) A[k][mm] = __ldg(&S.adj[(3 * k + mm) * ne + e]);
+    for (int mm = 0; mm < 3; mm++) A[k][mm] = S.adj[(3 * k + mm) * ne + e];
   const double vol = __ldg(&S.vol[e]), D = vol * 64.0;
   const int32_t mat_id = P.emat ? __ldg(&P.emat[e]) : 0;
   const MatDev &m = P.mats[mat_id];

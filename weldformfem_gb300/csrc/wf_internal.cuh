@@ -214,7 +214,9 @@ struct Fp64State {
   double *tau, *sig, *eps, *sr, *rr;             // [6][ne]
   double *fe, *fhg;                              // [npe * 3][ne]
   // adjugate of the step's Jacobian [9][ne] (hexahedra: of 8 J), tetrahedra
-  // with detJ as a tenth row
+  // with detJ as a tenth row: from the geometry phase to the element phase, in
+  // the first rows of fe, which the element kernel's thread of the same element
+  // overwrites after reading them (so not through the read-only path)
   double *adj;
   // thermal coupling: nodal temperature, die heat per node (kept after the
   // contact ends), and the element-node temperature rates of the step in two
