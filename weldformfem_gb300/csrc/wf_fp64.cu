@@ -188,6 +188,11 @@ __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodal(StepParams P, Fp64S
     // hexahedra: the densities' sum times voln / c, an exact division for the
     // 1, 2, 4 or 8 elements of a box mesh's nodes
     if constexpr (NPE == 8) mass = c > 0 ? rs * voln * rc : 0.0;
+    // tetrahedra: an infinity has no remainder, and zero times it is not zero
+    if (NPE == 4 && !(fabs(voln) < 1e290)) {
+      mass = 0.0;
+      for (int32_t k = 0; k < c; k++) mass += __ldg(&S.rho[elem(k)]) * voln / c;
+    }
     S.mass[n] = mass;
   }
   S.jr[n] = s / s0;
