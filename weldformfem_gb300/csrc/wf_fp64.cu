@@ -112,31 +112,13 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_geometry(StepParams P, Fp
 // nodal: CalcNodalVol (Mechanical.C:1555-1572), CalcNodalMassFromVol
 // (:1576-1601) and the nodal volume ratio of calcElemPressure (:694-705).
 // init_mode 1 also forms the constant sum of initial volumes.
-// BOX: the node's elements computed from its indices (box meshes of a mixed
-// domain, whose preamble runs this kernel), in the lists' order.
-template <int NPE, bool BOX>
+template <int NPE>
 __global__ void __launch_bounds__(kNodeThreads) k_fp64_nodal(StepParams P, Fp64State S,
                                                         int init_mode) {
   int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= P.nn) return;
-  int32_t b = 0, c = 0;
-  int32_t bel[8];
-  if constexpr (BOX) {
-    int32_t el[8], cor[8];
-    box_node_list(P, n, el, cor);
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-      if (el[j] >= 0) bel[c++] = el[j];
-  } else {
-    b = __ldg(&P.off[n]);
-    c = __ldg(&P.off[n + 1]) - b;
-  }
-  auto elem = [&](int32_t k) -> int32_t {
-    if constexpr (BOX)
-      return bel[k];
-    else
-      return __ldg(&P.slot[b + k]) / NPE;
-  };
+  const int32_t b = __ldg(&P.off[n]), c = __ldg(&P.off[n + 1]) - b;
+  auto elem = [&](int32_t k) -> int32_t { return __ldg(&P.slot[b + k]) / NPE; };
   // sums in list order, eight entries at a time: a chunk's loads are in
   // flight together
   double s = 0.0, s0 = 0.0;
@@ -1346,12 +1328,10 @@ void fp64_geometry(const StepParams &P, const Fp64State &S, cudaStream_t st, boo
 
 void fp64_nodal(const StepParams &P, const Fp64State &S, cudaStream_t st, int init_mode) {
   const int t = spread(P.nn, kNodeThreads, P.sms);
-  if (P.npe == 8 && P.box)
-    k_fp64_nodal<8, true><<<grid_for(P.nn, t), t, 0, st>>>(P, S, init_mode);
-  else if (P.npe == 8)
-    k_fp64_nodal<8, false><<<grid_for(P.nn, t), t, 0, st>>>(P, S, init_mode);
+  if (P.npe == 8)
+    k_fp64_nodal<8><<<grid_for(P.nn, t), t, 0, st>>>(P, S, init_mode);
   else
-    k_fp64_nodal<4, false><<<grid_for(P.nn, t), t, 0, st>>>(P, S, init_mode);
+    k_fp64_nodal<4><<<grid_for(P.nn, t), t, 0, st>>>(P, S, init_mode);
 }
 
 void fp64_elements(const StepParams &P, const Fp64State &S, cudaStream_t st) {
