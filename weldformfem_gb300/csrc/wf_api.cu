@@ -2164,21 +2164,6 @@ WF_API wf_status wf_init(wf_domain *d) {
     d->init_stage = stage;
     CUDA_TRY(build_connectivity(d->mesh_el, ne, d->npe, nn, nullptr, off, sl,
                                 static_cast<int32_t *>(stage), d->stream));
-    // the lists by position for the mixed tetrahedra's gathers, at most twice the
-    // lists' entries and no list longer than 64
-    if (d->precision == WF_MIXED && d->npe == 4 && nn >= kColsMinNodes) {
-      int32_t *flag = nullptr, most = 0;
-      CUDA_TRY(dalloc_raw(d, &flag, 1));
-      CUDA_TRY(longest_list(off, nn, flag, d->stream, &most));
-      if (most <= 64 && (int64_t)most * nn <= 2 * (int64_t)ent) {
-        int32_t *cols = nullptr;
-        CUDA_TRY(dalloc_raw(d, &cols, (size_t)most * np));
-        list_cols(off, sl, nn, np, most, cols, d->stream);
-        CUDA_TRY(cudaGetLastError());
-        P.cols = cols;
-        d->cols_width = most;
-      }
-    }
   }
   // BC codes per node (value set << 3 | fixed dimensions), zero but at the
   // BC nodes: scattered on the device from the BC nodes' records
@@ -2652,6 +2637,25 @@ WF_API wf_status wf_init(wf_domain *d) {
         CUDA_TRY(dalloc(d, &d->W.partials, cols));
         d->sweep = true;
         set_parity(d, 0);
+      }
+    }
+    // the lists by position for the mixed tetrahedra's gathers, at most twice the
+    // lists' entries and no list longer than 64; after the arrays that the step
+    // cannot do without, and left out where they no longer fit
+    if (d->npe == 4 && nn >= kColsMinNodes) {
+      int32_t *flag = nullptr, most = 0, *cols = nullptr;
+      CUDA_TRY(dalloc_raw(d, &flag, 1));
+      CUDA_TRY(longest_list(P.off, nn, flag, d->stream, &most));
+      if (most <= 64 && (int64_t)most * nn <= 2 * (int64_t)ent) {
+        const cudaError_t e = dalloc_raw(d, &cols, (size_t)most * np);
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+        else CUDA_TRY(e);
+      }
+      if (cols) {
+        list_cols(P.off, P.slot, nn, np, most, cols, d->stream);
+        CUDA_TRY(cudaGetLastError());
+        P.cols = cols;
+        d->cols_width = most;
       }
     }
     if (d->autotune) {
