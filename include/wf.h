@@ -439,7 +439,10 @@ WF_API wf_status wf_set_launch_config(wf_domain *d, int32_t phase, int32_t block
  * spans of steps as one cooperative launch, each block keeping its tile's
  * stresses on the chip, with two bounded barriers over the grid a step (mode 1's
  * arithmetic, the state bitwise; the reaction sum runs in another order; a
- * barrier that runs out makes wf_sync return WF_ERR_TIMEOUT); else mode 4 where the mesh is swept and its columns fill the GPU (at least 95 % of two
+ * barrier that runs out makes wf_sync return WF_ERR_TIMEOUT; up to 7600
+ * hexahedra the launch leaves SMs to other domains, above it takes them all, so
+ * that domains stepped side by side take turns: a program with several such
+ * domains at once sets mode 1); else mode 4 where the mesh is swept and its columns fill the GPU (at least 95 % of two
  * per SM: a column is a sequence of layers), else mode 1.
  * wf_get_step_mode reports the mode whose arithmetic and order of sums over
  * elements the next wf_run has (1 also for the cooperative launch and for a

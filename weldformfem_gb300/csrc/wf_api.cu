@@ -1736,7 +1736,8 @@ constexpr int64_t kClusterAutoElems = 3000;
 // per-phase kernels: 7.1 and 12.6 us a step at 4096 hexahedra, 8.5 and 12.9 at 5832
 // (8000 no longer fit). Against the tile run of box meshes it is ahead while its
 // threads take an element and a node each: 5.65 and 7.1 us at 3375 hexahedra (4096
-// nodes on 4096 threads), 7.1 and 7.0 at 4096 (4913 nodes), 8.2 and 7.2 at 4913.
+// nodes on 4096 threads), 7.1 and 7.3 at 4096 (4913 nodes), 8.2 and 8.0 at 4913, 8.7
+// and 7.6 at 6156, 10.3 and 8.3 at 40 x 40 x 3.
 // Past kClusterAutoElems it is reported as the per-phase mode it replaces, whose
 // arithmetic it runs.
 constexpr int64_t kClusterSmemElems = 6500;

@@ -3664,11 +3664,21 @@ bool mix_tile_run_shape(const StepParams &P, TileRunShape &C) {
   // over the elements (800 each), the ring elements (170), the corner and own
   // nodes (60 and 350) and the staged nodes (40)
   const int n[3] = {P.bx, P.by, P.bz};
+  // A small box leaves SMs to other domains' runs, which share the GPU when their
+  // blocks fit beside each other (a block takes its SM). A quarter of the SMs costs
+  // such a run next to nothing to 160 elements a tile (with heat 108), half of them
+  // to 100: us a step of one domain and of four at once, 4096 hexahedra 7.2 and 27.8
+  // on all SMs, 7.3 and 7.7 on a quarter, 12.6 and 15.7 per phase; 8000 on all 7.6
+  // and 29.3, 12.9 and 16.5 per phase.
+  const int64_t ne = (int64_t)n[0] * n[1] * n[2];
+  const int sms = ne <= (P.thermal ? 108 : 160) * (P.sms / 4) ? P.sms / 4
+                  : ne <= 100 * (P.sms / 2)                   ? P.sms / 2
+                                                              : P.sms;
   double best = 0.0;
   bool found = false;
-  for (int a = 1; a <= P.sms && a <= n[0]; a++)
-    for (int b = 1; a * b <= P.sms && b <= n[1]; b++) {
-      const int c = std::min(P.sms / (a * b), n[2]);
+  for (int a = 1; a <= sms && a <= n[0]; a++)
+    for (int b = 1; a * b <= sms && b <= n[1]; b++) {
+      const int c = std::min(sms / (a * b), n[2]);
       const int64_t x = (n[0] + a - 1) / a, y = (n[1] + b - 1) / b, z = (n[2] + c - 1) / c;
       TileRunShape S;
       S.ta = a;
