@@ -2,8 +2,10 @@
 
 One nvcc invocation per translation unit, run in parallel, for sm_103a only;
 the library links the CUDA runtime statically and exports only the C ABI of
-include/wf.h. The FP64 kernels are compiled with --fmad=false so that they
-round exactly as the reference CPU code (built without FMA contraction).
+include/wf.h. The FP64 kernels are compiled with --fmad=false, so that those that
+run the reference's operations in its order (tetrahedra without heat) round
+exactly as the reference CPU code built without FMA contraction; the others
+write their FMA out.
 """
 from __future__ import annotations
 

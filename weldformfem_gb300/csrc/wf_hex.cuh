@@ -116,11 +116,13 @@ __device__ __forceinline__ double pow_two_thirds(double v) {
 // X[m][k] = sum of the corners' coordinates k weighted by the sign of
 // direction m (8 J), from differences along the edges (21 additions a
 // component; the velocity sums take 17). The pressure is the bulk modulus
-// times a change of volume of 1e-3 and less, and differences of sums of
-// absolute coordinates left the step's largest rounding error (against 64-bit
-// sums of coordinates relative to a corner, 1.05 M hexahedra, 20 steps:
-// displacement 2e-13 from edge differences, 8e-13 without, as the reference's
-// alternating sums).
+// times a change of volume of 1e-3 and less, so the rounding of these sums shows
+// in the state. Which form is closer depends on what it is held against: 1.05 M
+// hexahedra, 20 steps, displacement 2e-13 from edge differences and 8e-13 from the
+// reference's alternating sums against 64-bit sums of coordinates relative to a
+// corner, 2e-12 and 6e-13 against 64-bit alternating sums, which share the latter's
+// rounding. Against 80-bit arithmetic (8^3 and 16^3 cubes, 64 steps) the two are
+// alike, 7.3e-13 and 7.4e-13, 8.2e-13 and 8.9e-13.
 template <typename T>
 __device__ __forceinline__ void corner_sums(const T (&x2)[8][3], T (&X)[3][3]) {
 #pragma unroll

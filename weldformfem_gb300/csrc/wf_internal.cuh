@@ -524,7 +524,7 @@ int64_t connectivity_scratch_ints(int64_t nn);
 // kColsMinNodes): with the lists end to end (slot) the entries that a warp reads
 // together lie 96 bytes apart, a line each, and those reads were a third of its
 // gathers' lines. 576,000 tetrahedra: node update 17.2 -> 15.6 us, nodal phase
-// 10.2 -> 8.5, a step 38.0 -> 35.0 with the registers below. Hexahedra keep slot:
+// 10.2 -> 8.5, a step 36.6 -> 32.8 with the node kernel's registers. Hexahedra keep slot:
 // a node's eight entries are one 32-byte sector (the FP64 node kernels took 14 %
 // longer from cols).
 #ifdef __CUDACC__

@@ -2624,8 +2624,8 @@ __global__ void __launch_bounds__(BS + 32, 1) k_mix_cluster_smem(StepParams P, M
 // block per SM, for boxes between the cluster run's size and what a block's threads
 // go through in two or three passes (mix_tile_run_shape). There a step's four kernels
 // were launch, ramp-up and two or three dependent L2 round trips each: 20 to 25
-// us for a few microseconds of work. A block owns a tile of elements (and the
-// a share of the nodes), and a step is two phases with a barrier over the
+// us for a few microseconds of work. A block owns a tile of elements and a share
+// of the nodes, and a step is two phases with a barrier over the
 // grid (1.3 us) after each:
 //   A  the positions of the nodes around the tile, two layers out, into shared
 //      memory; the volumes of the elements around it, one layer out, the J
@@ -2643,7 +2643,10 @@ __global__ void __launch_bounds__(BS + 32, 1) k_mix_cluster_smem(StepParams P, M
 // plain loads see the other blocks' writes). A wait that runs out (never
 // expected: a cooperative launch has all its blocks resident) sets bit 1 of the
 // step status, which wf_sync reports, and every block leaves.
-constexpr int kTileRunThreads = 608;   // working threads: 96 registers each
+// Working threads: 96 registers each (640 threads on a block's 65,536), at which the
+// variants keep 16 to 24 bytes on the stack, of them up to 24 stored and 16 loaded as
+// spills.
+constexpr int kTileRunThreads = 608;
 constexpr int kGridSpin = 1 << 22;
 constexpr int kTileRunSmemMax = 225 * 1024;   // the launch's dynamic shared memory at most
 
