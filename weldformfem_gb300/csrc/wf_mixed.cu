@@ -90,6 +90,41 @@ struct F2 {
   __device__ __forceinline__ F2 operator-() const { return F2{-x, -y}; }
 };
 
+// f(V, k) for the components x, y and z: PAIR: (x, y) as a pair of type V2, then z;
+// else one by one. gather and scatter move a pair's or a scalar's components from
+// k on. Kernels that read corners through the connectivity have no registers for
+// the pairs: 729,000 renumbered hexahedra, elements 36.9 us in packed pairs, 35.8 in
+// pairs of scalars, 35.3 one by one; geometry (pairs of scalars) 18.3 and 16.5. The
+// tiled kernel takes pairs of scalars: 16.4 us packed, 15.0, one by one 15.8 at
+// 64,000.
+template <class V2, bool PAIR, class F>
+__device__ __forceinline__ void components(F f) {
+  if constexpr (PAIR) {
+    f(V2{}, 0);
+    f(0.f, 2);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 3; k++) f(0.f, k);
+  }
+}
+template <bool P, class G>
+__device__ __forceinline__ void gather(F2<P> &v, int k, G g) {
+  v = F2<P>{g(k), g(k + 1)};
+}
+template <class G>
+__device__ __forceinline__ void gather(float &v, int k, G g) {
+  v = g(k);
+}
+template <bool P, class S>
+__device__ __forceinline__ void scatter(F2<P> v, int k, S s) {
+  s(k, v.x);
+  s(k + 1, v.y);
+}
+template <class S>
+__device__ __forceinline__ void scatter(float v, int k, S s) {
+  s(k, v);
+}
+
 // a - b for nearby points: hi parts subtract exactly when within a factor 2.
 template <bool PACKED = true>
 __device__ __forceinline__ float pair_rel(float2 a, float2 b) {
@@ -174,7 +209,7 @@ __device__ __forceinline__ void rel_coords(const StepParams &P, const MixState &
   for (int a = 1; a < NPE; a++)
 #pragma unroll
     for (int k = 0; k < 3; k++)
-      r[a][k] = pair_rel<NPE == 8>(ldx<LD>(&M.xh[k * P.np + nid[a]]), o[k]);
+      r[a][k] = pair_rel<NPE == 8 && BOX != kBoxNone>(ldx<LD>(&M.xh[k * P.np + nid[a]]), o[k]);
 }
 
 template <typename V>
@@ -184,16 +219,17 @@ __device__ __forceinline__ void jacobian_sums(const V (&v)[8], V (&o)[3]) {
   o[2] = -v[0] - v[1] - v[2] - v[3] + v[4] + v[5] + v[6] + v[7];
 }
 
-template <int NPE>
+template <int NPE, bool PACKED = true>
 __device__ __forceinline__ void jacobian_f(const float (&x2)[NPE][3], float J[3][3]) {
   if constexpr (NPE == 8) {
 #pragma unroll
     for (int k = 0; k < 3; k += 2) {
       // (x, y) packed, then z
       if (k == 0) {
-        F2<> v[8], o[3];
+        using V2 = F2<PACKED>;
+        V2 v[8], o[3];
 #pragma unroll
-        for (int a = 0; a < 8; a++) v[a] = F2<>{x2[a][0], x2[a][1]};
+        for (int a = 0; a < 8; a++) v[a] = V2{x2[a][0], x2[a][1]};
         jacobian_sums(v, o);
 #pragma unroll
         for (int m = 0; m < 3; m++) {
@@ -266,7 +302,7 @@ __device__ __forceinline__ void geometry_one(const StepParams &P, const MixState
   int32_t nid[NPE];
   rel_coords<NPE, LD, BOX>(P, M, e, r, nid);
   float J[3][3];
-  jacobian_f<NPE>(r, J);
+  jacobian_f<NPE, BOX != kBoxNone>(r, J);
   vol[e] = det3f(J) * weightf<NPE>();
 }
 
@@ -285,8 +321,8 @@ __global__ void __launch_bounds__(BS) k_mix_geometry(StepParams P, MixState M, f
     rel_coords<NPE, kLdRo, BOX>(P, M, e, r0, n0);
     rel_coords<NPE, kLdRo, BOX>(P, M, e + stride, r1, n1);
     float J0[3][3], J1[3][3];
-    jacobian_f<NPE>(r0, J0);
-    jacobian_f<NPE>(r1, J1);
+    jacobian_f<NPE, BOX != kBoxNone>(r0, J0);
+    jacobian_f<NPE, BOX != kBoxNone>(r1, J1);
     vol[e] = det3f(J0) * weightf<NPE>();
     vol[e + stride] = det3f(J1) * weightf<NPE>();
   }
@@ -792,6 +828,7 @@ struct ThermalNodes {
 // them before every read of them is done) and only the J ratios through L2.
 template <int LD, int BOX = kBoxNone, int LDX = LD>
 struct GlobalNodes : ThermalNodes<8, LD> {
+  static constexpr bool packed = BOX != kBoxNone, paired = packed;
   using ThermalNodes<8, LD>::nid;
   const float2 *xh;
   const float *vp, *jr;
@@ -851,7 +888,7 @@ __device__ __forceinline__ void element_hex_core(const StepParams &P, const MixS
                                                  int64_t e, const Nodes &nd, float *stash,
                                                  int stride, long long step, Out &out,
                                                  const IO &io) {
-  using V2 = F2<LAW == 0>;
+  using V2 = F2<LAW == 0 && Nodes::packed>;
   float A[3][3], detJ;
   float J_avg = 0.f;
   {
@@ -865,31 +902,21 @@ __device__ __forceinline__ void element_hex_core(const StepParams &P, const MixS
 #pragma unroll
     for (int a = 1; a < 8; a++)
 #pragma unroll
-      for (int k = 0; k < 3; k++) r[a][k] = pair_rel(nd.x(a, k), o[k]);
+      for (int k = 0; k < 3; k++) r[a][k] = pair_rel<Nodes::packed>(nd.x(a, k), o[k]);
     if constexpr (EARLY_JR) {
 #pragma unroll
       for (int a = 0; a < 8; a++) J_avg += nd.j(a);
     }
     float J[3][3];
-    {
-      V2 v[8], o8[8];
+    components<V2, Nodes::paired>([&](auto v0, int k) {
+      decltype(v0) v[8], o8[8];
 #pragma unroll
-      for (int a = 0; a < 8; a++) v[a] = V2{r[a][0], r[a][1]};
+      for (int a = 0; a < 8; a++) gather(v[a], k, [&](int c) { return r[a][c]; });
       walsh8(v, o8);
 #pragma unroll
-      for (int mm = 0; mm < 3; mm++) {
-        J[mm][0] = 0.125f * o8[1 + mm].x;
-        J[mm][1] = 0.125f * o8[1 + mm].y;
-      }
-    }
-    {
-      float v[8], o8[8];
-#pragma unroll
-      for (int a = 0; a < 8; a++) v[a] = r[a][2];
-      walsh8(v, o8);
-#pragma unroll
-      for (int mm = 0; mm < 3; mm++) J[mm][2] = 0.125f * o8[1 + mm];
-    }
+      for (int mm = 0; mm < 3; mm++)
+        scatter(o8[1 + mm], k, [&](int c, float x) { J[mm][c] = 0.125f * x; });
+    });
     A[0][0] = (J[1][1] * J[2][2] - J[1][2] * J[2][1]);
     A[1][0] = -(J[1][0] * J[2][2] - J[1][2] * J[2][0]);
     A[2][0] = (J[1][0] * J[2][1] - J[1][1] * J[2][0]);
@@ -905,32 +932,16 @@ __device__ __forceinline__ void element_hex_core(const StepParams &P, const MixS
   const MatF &m = P.matf[P.emat ? __ldg(&P.emat[e]) : 0];
   // velocity Walsh sums: G[m][k] (derivative directions), hm[k][j] (hourglass)
   float G[3][3], hm[3][4];
-  {
-    V2 v[8], o[8];
+  components<V2, Nodes::paired>([&](auto v0, int k) {
+    decltype(v0) v[8], o[8];
 #pragma unroll
-    for (int a = 0; a < 8; a++) v[a] = V2{nd.v(a, 0), nd.v(a, 1)};
+    for (int a = 0; a < 8; a++) gather(v[a], k, [&](int c) { return nd.v(a, c); });
     walsh8(v, o);
 #pragma unroll
-    for (int mm = 0; mm < 3; mm++) {
-      G[mm][0] = o[1 + mm].x;
-      G[mm][1] = o[1 + mm].y;
-    }
+    for (int mm = 0; mm < 3; mm++) scatter(o[1 + mm], k, [&](int c, float x) { G[mm][c] = x; });
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      hm[0][j] = o[4 + j].x;
-      hm[1][j] = o[4 + j].y;
-    }
-  }
-  {
-    float v[8], o[8];
-#pragma unroll
-    for (int a = 0; a < 8; a++) v[a] = nd.v(a, 2);
-    walsh8(v, o);
-#pragma unroll
-    for (int mm = 0; mm < 3; mm++) G[mm][2] = o[1 + mm];
-#pragma unroll
-    for (int j = 0; j < 4; j++) hm[2][j] = o[4 + j];
-  }
+    for (int j = 0; j < 4; j++) scatter(o[4 + j], k, [&](int c, float x) { hm[c][j] = x; });
+  });
   // hourglass forces' coefficients ch h_j, kept in shared memory (one column
   // per thread) across the stress update to free registers
   {
@@ -971,31 +982,18 @@ __device__ __forceinline__ void element_hex_core(const StepParams &P, const MixS
   auto fs = [&](int mm, int k) {
     return A[0][mm] * S[0][k] + A[1][mm] * S[1][k] + A[2][mm] * S[2][k];
   };
-  {
-    V2 o[8], f[8];
-    o[0] = V2{0.f, 0.f};
+  components<V2, Nodes::paired>([&](auto v0, int k) {
+    decltype(v0) o[8], f[8];
+    gather(o[0], k, [](int) { return 0.f; });
 #pragma unroll
-    for (int mm = 0; mm < 3; mm++) o[1 + mm] = V2{fs(mm, 0), fs(mm, 1)};
+    for (int mm = 0; mm < 3; mm++) gather(o[1 + mm], k, [&](int c) { return fs(mm, c); });
 #pragma unroll
-    for (int j = 0; j < 4; j++) o[4 + j] = V2{stash[j * stride], stash[(4 + j) * stride]};
+    for (int j = 0; j < 4; j++)
+      gather(o[4 + j], k, [&](int c) { return stash[(c * 4 + j) * stride]; });
     walsh8_synth(o, f);
 #pragma unroll
-    for (int a = 0; a < 8; a++) {
-      out.put(a, 0, f[a].x);
-      out.put(a, 1, f[a].y);
-    }
-  }
-  {
-    float o[8], f[8];
-    o[0] = 0.f;
-#pragma unroll
-    for (int mm = 0; mm < 3; mm++) o[1 + mm] = fs(mm, 2);
-#pragma unroll
-    for (int j = 0; j < 4; j++) o[4 + j] = stash[(8 + j) * stride];
-    walsh8_synth(o, f);
-#pragma unroll
-    for (int a = 0; a < 8; a++) out.put(a, 2, f[a]);
-  }
+    for (int a = 0; a < 8; a++) scatter(f[a], k, [&](int c, float x) { out.put(a, c, x); });
+  });
   if constexpr (TH) {
     // conduction in the same Walsh form: grad T detJ = A (Walsh sums of T) / 8,
     // (K T)_a = k_T / detJ * synthesis of A^T grad T detJ (w = 8 cancels 1/8)
@@ -1458,6 +1456,7 @@ __global__ void __launch_bounds__(kNodeThreads, NPE == 4 ? 4 : WF_NODE_MIN_BLOCK
 
 // A tile's staged node values through tile-local indices.
 struct TileNodes {
+  static constexpr bool packed = false, paired = true;
   const float2 *sx;
   const float *svp, *sjr;
   int32_t loc[8];
@@ -1664,6 +1663,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // b + {0, 1, kSwNX + 1, kSwNX}[a & 3] of the lower (a < 4) or upper plane.
 template <int PL>
 struct SweepNodes {
+  static constexpr bool packed = true, paired = true;
   const float2 *x0, *x1;
   const float *v0, *v1, *j0, *j1;
   int b;
@@ -2239,6 +2239,7 @@ __device__ __forceinline__ int64_t owner_of(int64_t i, int64_t n, int64_t nb) {
 // An element's corners in the block's node copies: planes (x, y hi and lo),
 // (z hi and lo, v_x, v_y), (v_z, J ratio).
 struct CopyNodes {
+  static constexpr bool packed = true, paired = true;
   const float4 *q0, *q1;
   const float2 *q2;
   uint32_t c[8];
@@ -2738,6 +2739,7 @@ struct TileRunSmem {
 // An element's corners in the staged blocks of nodes (b1: its corner 0 among
 // the tile's corner nodes, b2: among the staged positions).
 struct TileRunNodes {
+  static constexpr bool packed = true, paired = true;
   const float2 *sx;
   const float *sv, *sj, *sm, *sT;
   int n1, n2, b1, b2, px1, pxy1, px2, pxy2;
