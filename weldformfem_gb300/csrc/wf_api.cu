@@ -2690,7 +2690,9 @@ WF_API wf_status wf_init(wf_domain *d) {
       }
     }
   }
-  d->tile_run = !fp64 && !d->nspec && !d->energy && mix_tile_run_shape(P, d->tr_shape);
+  // (meshes that always run as a cluster need none)
+  d->tile_run = !fp64 && !d->nspec && !d->energy &&
+                !(d->cl_blocks && d->ne <= kClusterAutoElems) && mix_tile_run_shape(P, d->tr_shape);
   if (d->tile_run) {
     const TileRunShape &C = d->tr_shape;
     CUDA_TRY(dalloc(d, &d->tr_part, (size_t)kTileRunChunk * C.ta * C.tb * C.tc));
