@@ -45,3 +45,20 @@ def test_specimen_reactions(prec):
         long = d.specimen_reaction(k)
         assert long.shape == (8340,)
         np.testing.assert_array_equal(long[:40], short[k])
+
+
+def test_halo_forces_of_a_small_layer():
+    """A layer of 100 hexahedra costs two readbacks at most, in each direction (the
+    caller's order is made on the device; with scratch from the pool and a launch per
+    array it was 1.5 times the copies alone)."""
+    d = wf.Domain(wf.WF_FP64)
+    W.apply(d, W.config(0, scale=(10, 10, 10)))
+    d.init()
+    d.run(3)
+    d.sync()
+    plain = median(d.reaction, 100)
+    d.step_begin()
+    buf = np.zeros(2 * 100 * 24)
+    for call in ("wf_get_halo_forces", "wf_set_halo_forces"):
+        t = median(lambda: d._call(call, 100, 200, buf), 100)
+        assert t <= 1.45 * plain, (call, t, plain)

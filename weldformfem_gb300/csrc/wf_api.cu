@@ -264,6 +264,8 @@ struct wf_domain {
   int flow_par = 0;
   int32_t flow_tile = 512, flow_lag = 4;
   int cl_blocks = 0, cl_bs = 0;
+  double *halo_buf = nullptr;     // FP64 halo forces in the caller's order
+  size_t halo_cap = 0;            // values it holds
   double *cl_part = nullptr;      // [kClusterChunk][cl_blocks] reaction partials
   bool cl_smem = false;           // the cluster run keeps its state in shared memory
   ClusterShape cl_shape;
@@ -413,6 +415,8 @@ void free_device(wf_domain *d) {
   if (d->out_stream) cudaStreamSynchronize(d->out_stream);
   for (void *p : d->allocs) cudaFreeAsync(p, d->stream);
   d->allocs.clear();
+  d->halo_buf = nullptr;
+  d->halo_cap = 0;
   d->st_pending = false;
   for (auto &sn : d->snap) {
     if (sn.dev) cudaFree(sn.dev);
@@ -3133,6 +3137,16 @@ WF_API wf_status wf_step_end(wf_domain *d) {
   return WF_OK;
 }
 
+namespace {
+// Device room for n values of the FP64 halo forces, kept with the domain.
+cudaError_t halo_buffer(wf_domain *d, size_t n) {
+  if (n <= d->halo_cap) return cudaSuccess;
+  const cudaError_t e = dalloc_raw(d, &d->halo_buf, n);
+  if (e == cudaSuccess) d->halo_cap = n;
+  return e;
+}
+}  // namespace
+
 WF_API wf_status wf_get_halo_forces(wf_domain *d, int64_t e0, int64_t e1, double *out) {
   wf_status s = need_halves(d);
   if (s) return s;
@@ -3159,15 +3173,11 @@ WF_API wf_status wf_get_halo_forces(wf_domain *d, int64_t e0, int64_t e1, double
   // strided rows transposed by the host 1.1 ms)
   if (k == 0) return WF_OK;
   const int parts = d->S.fhg ? 2 : 1;
-  double *buf = nullptr;
-  CUDA_TRY(pool_alloc(d, reinterpret_cast<void **>(&buf), sizeof(double) * parts * k));
-  rows_to_items(d->S.fe, d->ne, e0, e1 - e0, d->npe * 3, buf, d->stream);
-  if (parts == 2) rows_to_items(d->S.fhg, d->ne, e0, e1 - e0, d->npe * 3, buf + k, d->stream);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(out, buf, sizeof(double) * parts * k, cudaMemcpyDeviceToHost, d->stream);
-  cudaFreeAsync(buf, d->stream);
-  CUDA_TRY(e);
+  CUDA_TRY(halo_buffer(d, parts * k));
+  rows_to_items(d->S.fe, d->S.fhg, d->ne, e0, e1 - e0, d->npe * 3, d->halo_buf, d->stream);
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaMemcpyAsync(out, d->halo_buf, sizeof(double) * parts * k, cudaMemcpyDeviceToHost,
+                           d->stream));
   if (parts == 1) std::fill(out + k, out + 2 * k, 0.0);
   CUDA_TRY(cudaStreamSynchronize(d->stream));
   d->d2h_bytes += (int64_t)(sizeof(double) * 2 * k);
@@ -3192,18 +3202,12 @@ WF_API wf_status wf_set_halo_forces(wf_domain *d, int64_t e0, int64_t e1, const 
   }
   if (k == 0) return WF_OK;
   const int parts = d->S.fhg ? 2 : 1;
-  double *buf = nullptr;
-  CUDA_TRY(pool_alloc(d, reinterpret_cast<void **>(&buf), sizeof(double) * parts * k));
-  cudaError_t e =
-      cudaMemcpyAsync(buf, in, sizeof(double) * parts * k, cudaMemcpyHostToDevice, d->stream);
-  if (e == cudaSuccess) {
-    items_to_rows(buf, d->ne, e0, e1 - e0, d->npe * 3, d->S.fe, d->stream);
-    if (parts == 2) items_to_rows(buf + k, d->ne, e0, e1 - e0, d->npe * 3, d->S.fhg, d->stream);
-    e = cudaGetLastError();
-  }
-  cudaFreeAsync(buf, d->stream);
-  CUDA_TRY(e);
-  CUDA_TRY(cudaStreamSynchronize(d->stream));
+  CUDA_TRY(halo_buffer(d, parts * k));
+  CUDA_TRY(cudaMemcpyAsync(d->halo_buf, in, sizeof(double) * parts * k, cudaMemcpyHostToDevice,
+                           d->stream));
+  CUDA_TRY(cudaStreamSynchronize(d->stream));   // `in` is the caller's again
+  items_to_rows(d->halo_buf, d->ne, e0, e1 - e0, d->npe * 3, d->S.fe, d->S.fhg, d->stream);
+  CUDA_TRY(cudaGetLastError());
   d->h2d_bytes += (int64_t)(sizeof(double) * 2 * k);
   return WF_OK;
 }

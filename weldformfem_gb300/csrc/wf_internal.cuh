@@ -589,11 +589,12 @@ cudaError_t check_spec_boxes(const int32_t *el_soa, int64_t ne, const uint16_t *
 void coords_soa(const double *x_aos, int64_t nn, int64_t np, double *out, cudaStream_t st);
 // SoA [3][np] -> AoS [nn][3]
 void coords_aos(const double *soa, int64_t nn, int64_t np, double *out, cudaStream_t st);
-// [row][stride] columns at .. at + m -> items [m][rows], and back
-void rows_to_items(const double *src, int64_t stride, int64_t at, int64_t m, int rows, double *items,
-                   cudaStream_t st);
-void items_to_rows(const double *items, int64_t stride, int64_t at, int64_t m, int rows, double *dst,
-                   cudaStream_t st);
+// [row][stride] columns at .. at + m of one or two (second not null) arrays -> items
+// [m][rows], the second's after the first's, and back
+void rows_to_items(const double *first, const double *second, int64_t stride, int64_t at, int64_t m,
+                   int rows, double *items, cudaStream_t st);
+void items_to_rows(const double *items, int64_t stride, int64_t at, int64_t m, int rows,
+                   double *first, double *second, cudaStream_t st);
 void fill_values(double *p, double v, int64_t n, cudaStream_t st);
 // sigma_y = sy0 of each element's material
 void initial_yield(const StepParams &P, double *sy, cudaStream_t st);

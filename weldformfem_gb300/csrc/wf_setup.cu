@@ -710,28 +710,31 @@ namespace {
 // Neighbouring threads take neighbouring values of an item: the item side is
 // coalesced, the row side reads a sector per row of four columns, all used.
 template <bool TO_ITEMS>
-__global__ void k_rows_items(double *rows_of, int64_t stride, int64_t at, int64_t n, int rows,
-                             double *items) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double *r = rows_of + (i % rows) * stride + at + i / rows;
-  if (TO_ITEMS) items[i] = *r;
-  else *r = items[i];
+__global__ void k_rows_items(double *first, double *second, int64_t stride, int64_t at, int64_t n,
+                             int rows, double *items) {
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= (second ? 2 * n : n)) return;
+  const int64_t i = j < n ? j : j - n;
+  double *r = (j < n ? first : second) + (i % rows) * stride + at + i / rows;
+  if (TO_ITEMS) items[j] = *r;
+  else *r = items[j];
 }
 }  // namespace
 
-void rows_to_items(const double *src, int64_t stride, int64_t at, int64_t m, int rows, double *items,
-                   cudaStream_t st) {
-  if (m > 0)
-    k_rows_items<true><<<grid_for(m * rows), kThreads, 0, st>>>(const_cast<double *>(src), stride, at,
-                                                                m * rows, rows, items);
+void rows_to_items(const double *first, const double *second, int64_t stride, int64_t at, int64_t m,
+                   int rows, double *items, cudaStream_t st) {
+  const int64_t n = m * rows;
+  if (n > 0)
+    k_rows_items<true><<<grid_for(second ? 2 * n : n), kThreads, 0, st>>>(
+        const_cast<double *>(first), const_cast<double *>(second), stride, at, n, rows, items);
 }
 
-void items_to_rows(const double *items, int64_t stride, int64_t at, int64_t m, int rows, double *dst,
-                   cudaStream_t st) {
-  if (m > 0)
-    k_rows_items<false><<<grid_for(m * rows), kThreads, 0, st>>>(dst, stride, at, m * rows, rows,
-                                                                 const_cast<double *>(items));
+void items_to_rows(const double *items, int64_t stride, int64_t at, int64_t m, int rows,
+                   double *first, double *second, cudaStream_t st) {
+  const int64_t n = m * rows;
+  if (n > 0)
+    k_rows_items<false><<<grid_for(second ? 2 * n : n), kThreads, 0, st>>>(
+        first, second, stride, at, n, rows, const_cast<double *>(items));
 }
 
 void fill_values(double *p, double v, int64_t n, cudaStream_t st) {
