@@ -62,3 +62,15 @@ def test_halo_forces_of_a_small_layer():
     for call in ("wf_get_halo_forces", "wf_set_halo_forces"):
         t = median(lambda: d._call(call, 100, 200, buf), 100)
         assert t <= 1.45 * plain, (call, t, plain)
+
+
+@pytest.mark.parametrize("prec", [wf.WF_FP64, wf.WF_MIXED])
+def test_detj_of_tetrahedra(prec):
+    """detJ is formed at the call: 1.36 times a plain field of 576,000 tetrahedra (1.58
+    when the geometry kernel formed the step's adjugates for it as well), bar 1.47."""
+    d = wf.Domain(prec)
+    W.apply(d, W.config(1))
+    d.init()
+    d.run(2)
+    vol = median(lambda: d.elem_scalar("vol"), 80)
+    assert median(lambda: d.elem_scalar("detJ"), 80) <= 1.47 * vol

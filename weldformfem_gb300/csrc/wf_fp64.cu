@@ -93,7 +93,6 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_geometry(StepParams P, Fp
     v = detJ * 8.0;
   } else {
     jacobian(x2, J);
-    adjugate(J, A);
     detJ = det3(J);
     v = 0.0;
     v += detJ * weight<NPE>() * 1.0;
@@ -101,6 +100,7 @@ __global__ void __launch_bounds__(kElemThreads) k_fp64_geometry(StepParams P, Fp
   S.vol[e] = v;
   if (store_detj) S.detJ[e] = detJ;
   if (!S.adj) return;   // the preamble, or a detJ readback
+  if constexpr (NPE == 4) adjugate(J, A);
 #pragma unroll
   for (int k = 0; k < 3; k++)
 #pragma unroll
