@@ -23,8 +23,8 @@ def median(f, n=60):
 
 @pytest.mark.parametrize("prec", [wf.WF_FP64, wf.WF_MIXED])
 def test_specimen_reactions(prec):
-    """A short history's reaction costs about what a domain's does (1.0; 1.4 when
-    every call gathered the specimen's column on the device); long and short ones
+    """A short history's reaction costs about what a domain's does (0.92; 1.24 to 1.36
+    when every call gathered the specimen's column on the device); long and short ones
     are the same values."""
     b = W.ensemble(n_spec=8, nmin=4, nmax=6)
     d = wf.Domain(prec)
@@ -48,9 +48,9 @@ def test_specimen_reactions(prec):
 
 
 def test_halo_forces_of_a_small_layer():
-    """A layer of 100 hexahedra costs two readbacks at most, in each direction (the
-    caller's order is made on the device; with scratch from the pool and a launch per
-    array it was 1.5 times the copies alone)."""
+    """A layer of 100 hexahedra costs what a reaction readback does, 0.85 to 0.95 of it
+    in each direction (the caller's order is made on the device; with scratch from the
+    pool and a launch per array it was 1.47 to 1.60)."""
     d = wf.Domain(wf.WF_FP64)
     W.apply(d, W.config(0, scale=(10, 10, 10)))
     d.init()
@@ -66,8 +66,9 @@ def test_halo_forces_of_a_small_layer():
 
 @pytest.mark.parametrize("prec", [wf.WF_FP64, wf.WF_MIXED])
 def test_detj_of_tetrahedra(prec):
-    """detJ is formed at the call: 1.36 times a plain field of 576,000 tetrahedra (1.58
-    when the geometry kernel formed the step's adjugates for it as well), bar 1.47."""
+    """detJ is formed at the call: 1.33 to 1.35 times a plain field of 576,000 tetrahedra
+    (1.55 to 1.59 when the geometry kernel formed the step's adjugates for it as
+    well), bar 1.47."""
     d = wf.Domain(prec)
     W.apply(d, W.config(1))
     d.init()

@@ -3677,8 +3677,9 @@ bool mix_tile_run_shape(const StepParams &P, TileRunShape &C) {
   // blocks fit beside each other (a block takes its SM). A quarter of the SMs costs
   // such a run next to nothing to 160 elements a tile (with heat 108), half of them
   // to 100: us a step of one domain and of four at once, 4096 hexahedra 7.2 and 27.8
-  // on all SMs, 7.3 and 7.7 on a quarter, 12.6 and 15.7 per phase; 8000 on all 7.6
-  // and 29.3, 12.9 and 16.5 per phase.
+  // on all SMs, 7.3 and 7.7 on a quarter, 12.6 and 15.7 per phase; 3553 with heat
+  // (Johnson-Cook) alone 10.5 on all, 10.7 on a quarter; 8000 on all 7.6 and 29.3,
+  // 12.9 and 16.5 per phase.
   const int64_t ne = (int64_t)n[0] * n[1] * n[2];
   const int sms = ne <= (P.thermal ? 108 : 160) * (P.sms / 4) ? P.sms / 4
                   : ne <= 100 * (P.sms / 2)                   ? P.sms / 2
@@ -3720,10 +3721,10 @@ bool mix_tile_run_shape(const StepParams &P, TileRunShape &C) {
   // Where the tile run ends: three passes of the working threads over the
   // elements pay only where the tiles keep whole rows along x (a cut row starts
   // within a sector at both ends), four and, with heat, three do not. us a step of
-  // the tile run and per phase, bilinear: two passes 162,540 19.3 and 22.7; three,
-  // whole rows 256,500 28.8 and 30.2, 246,120 24.9 and 28.7; three, cut rows
-  // 226,920 27.4 and 27.1, 229,824 29.9 and 27.3, 252,000 33.7 and 29.3; four
-  // 270,336 37.9 and 30.4. Johnson-Cook with heat: two passes 168,000 32.7 and
+  // the tile run and per phase, bilinear: two passes 162,540 19.2 and 22.7; three,
+  // whole rows 256,500 28.7 and 29.0, 246,120 24.8 and 27.7; three, cut rows
+  // 226,920 27.4 and 27.1, 229,824 29.9 and 27.0, 252,000 33.7 and 27.9; four
+  // 270,336 37.9 and 28.9. Johnson-Cook with heat: two passes 168,000 32.7 and
   // 34.4, three 195,000 38.0 and 38.3, 226,000 47.5 and 44.4.
   if (C.e0 > (P.thermal || C.ta > 1 ? 2 : 3) * kTileRunThreads) return false;
   const TileRunKernel k = tile_run_kernel(P);
